@@ -96,6 +96,59 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
 		: "memory");
 }
 
+// Packed FP32 (sm_100 and later): two independent lanes' values in one aligned register
+// pair, each half rounded as the scalar instruction rounds it.  fma/add/mul.f32x2 do the
+// FMA pipe's work of two scalar instructions in one issue slot, which is what limits the
+// pair loops.  Kept as 64-bit integers so that the halves stay in register pairs.
+typedef unsigned long long u64;
+
+__device__ __forceinline__ u64 pack2(float a, float b)
+{
+	u64 r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+	return r;
+}
+
+__device__ __forceinline__ void unpack2(u64 v, float& a, float& b)
+{
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c)
+{
+	u64 r;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+	return r;
+}
+
+__device__ __forceinline__ u64 mul2(u64 a, u64 b)
+{
+	u64 r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+
+__device__ __forceinline__ u64 add2(u64 a, u64 b)
+{
+	u64 r;
+	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+
+// A row's position by four 32-bit loads.  Values that two rows' packed pairs are made of
+// must not come from one 128-bit load: the compiler then keeps the loaded quad and forms
+// the pairs again by register moves at every step of the pair loop (4 moves per pair
+// measured, 1.38 against 1.17 ms per stage 1 at 65536 bodies).
+__device__ __forceinline__ float4 load_row(const float4* p)
+{
+	float4 r;
+	asm volatile("ld.global.f32 %0, [%1];" : "=f"(r.x) : "l"(p));
+	asm volatile("ld.global.f32 %0, [%1+4];" : "=f"(r.y) : "l"(p));
+	asm volatile("ld.global.f32 %0, [%1+8];" : "=f"(r.z) : "l"(p));
+	asm volatile("ld.global.f32 %0, [%1+12];" : "=f"(r.w) : "l"(p));
+	return r;
+}
+
 // Compensated accumulation (Knuth's TwoSum, "The Art of Computer Programming" vol. 2,
 // 4.2.2): hi + lo is the running sum; the rounding error of hi + x is kept exactly and
 // added to lo.  Six FP32 additions; no FP64 (which runs at ~1/75 of the FP32 rate on
@@ -145,9 +198,7 @@ __device__ __forceinline__ float near_threshold(float max_abs_coord)
 	return max_abs_coord * max_abs_coord * inv_k2;
 }
 
-// Running minimum of the r2 values of a thread's B rows for the near test, one
-// three-input min per two rows (min.f32 with three operands, sm_100 and later): call
-// with k = 0 .. B-1 in order; `prev` holds the previous row's r2 between calls.
+// Three-input minimum (min.f32 with three operands, sm_100 and later).
 __device__ __forceinline__ float min3f(float a, float b, float c)
 {
 	float r;
@@ -155,6 +206,9 @@ __device__ __forceinline__ float min3f(float a, float b, float c)
 	return r;
 }
 
+// Running minimum of the r2 values of a thread's B rows for the near test, one
+// three-input min per two rows: call with k = 0 .. B-1 in order; `prev` holds the previous
+// row's r2 between calls.
 template <int B>
 __device__ __forceinline__ void near_min_step(int k, float r2, float& m, float& prev)
 {
@@ -185,9 +239,7 @@ __device__ __forceinline__ void near_delta(float dx, float dy, float dz, float r
 }
 
 // One j-tile against a thread's B rows, every ordered pair, rows only: the inner loop
-// of the all-pairs kernel (stage1_f32.cu); the rows' low parts are rowlo[k * T + tid].
-// (The unique-pair kernel keeps its own copy of this loop with a test per step: with
-// this function inlined there its main loop compiled measurably slower on GB300.)  NEAR adds the near
+// of the all-pairs kernel (stage1_f32.cu); the rows' low parts are rowlo[k * T + tid].  NEAR adds the near
 // test (one three-input min per two rows and a compare; with SELF -- tiles that hold the
 // thread block's own rows -- a test per pair that also excludes r2 = eps2, so that self
 // pairs do not count) whose result is a bit per step, and after every 32 steps a cold

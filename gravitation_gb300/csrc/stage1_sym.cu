@@ -25,6 +25,21 @@
 // Row sums are FP32 per tile, folded into compensated (TwoSum) FP32 hi+lo sums, as in
 // stage1_f32.cu, and go out as FP32 (hi, lo) pairs; column sums are FP32 per tile and go
 // out as FP32 (the first 3R floats of the slot), which stage 2 adds by TwoSum in FP32.
+//
+// What bounds it, and the packed loop.  With scalar FP32 instructions the loop issued 18
+// (near-corrected 22) instructions per pair for 16 of the FMA pipe and ran at 25-26 cycles
+// per pair and warp: issue slots and register-port conflicts, FMA pipe 67 % busy.  Two rows
+// of a thread now share every FMA-pipe instruction (f32x2: one issue slot for the pipe work
+// of two; a thread's rows come in packed pairs), the j-tile is expanded in shared memory to
+// (x, x) pairs so that no register move builds them, and the chunk is stored twice in a row
+// so that the rotated read needs no index arithmetic: 11 (12) instructions and 21.8 (24.4)
+// cycles per pair, FMA pipe 79 % (66 %) busy.  What is left is the pipe itself (16 cycles),
+// the SFU's reciprocal square root (it costs the scheduler ~2 more) and, in the near mode,
+// the three-input minima, whose register reads compete with the packed operands'.
+// Stage 1 at 65536 bodies, best tile, scalar loop -> this one: fp32u 1.335 -> 1.166 ms,
+// fp32cu 2.07 -> 1.58 ms, fp32un 1.40 -> 1.34 ms; at 16384 bodies 98 -> 88, 129 -> 118,
+// 106 -> 100 us.  One barrier per j-tile: a warp that is done with tile t expands its share
+// of tile t + 1 and meets the others once; the column sums of tile t leave after that.
 #include "grav_device.cuh"
 
 namespace grav {
@@ -34,40 +49,160 @@ namespace grav {
 //   SYM_DS    (GRAV_MODE_FP32CU): FP32 hi and lo parts of the FP64 positions,
 //             d = (hi_j - hi_i) + (lo_j - lo_i), exact to FP32 relative precision however
 //             far from the origin the bodies are (+6 FADD per pair).
-//   SYM_NEAR  (GRAV_MODE_FP32UN): the SYM_PLAIN loop plus one compare per pair against
-//             the near radius (grav_device.cuh, near_threshold); a step of the loop where
-//             any lane of the warp met a near pair re-evaluates those pairs from the
-//             double-single separation and adds the difference (near_delta).  Near pairs
+//   SYM_NEAR  (GRAV_MODE_FP32UN): the SYM_PLAIN loop plus a running minimum of r2 over the
+//             thread's rows, compared with the near radius once per step (grav_device.cuh,
+//             near_threshold) into a bit mask; after a chunk of 32 steps those that met a
+//             near pair in some lane of the warp re-evaluate the near pairs from the
+//             double-single separation and add the difference (near_delta).  Near pairs
 //             are rare (~3e-5 of the pairs of the N = 65536 uniform cube), so this path is
-//             cold; it is warp-uniform, so it costs no divergence.
+//             cold; it is warp-uniform, so it costs no divergence.  (With a vote and the
+//             cold path in every step the loop could not be unrolled; with the mask it is,
+//             1.41 -> 1.34 ms.)
 enum { SYM_PLAIN = 0, SYM_DS = 1, SYM_NEAR = 2 };
 
-template <int B, int W, int JT, int UNROLL = 4, int KIND = SYM_PLAIN>
-__global__ void __launch_bounds__(32 * W) stage1_sym_kernel(const grav_batch b)
+// Dynamic shared memory of one CTA, in this order (16-byte units throughout).
+template <int B, int W, int JT, int KIND>
+struct SymSmem {
+	static constexpr int T = 32 * W, NP = KIND == SYM_PLAIN ? 1 : 2;
+	static constexpr int EXA = KIND == SYM_DS ? 4 : 2;            // expanded rows per chunk
+	static constexpr int EX_TILE = (JT / 32) * EXA * 64;         // ulonglong2 per expanded tile
+	static constexpr int RAW = 0;                                 // [2][NP][JT] float4
+	static constexpr int EX = RAW + 2 * NP * JT * 16;             // [2][JT / 32][EXA][64] ulonglong2
+	static constexpr int CSUM = EX + 2 * EX_TILE * 16;            // [3][B][T] float2
+	static constexpr int COL = CSUM + 3 * B * T * 8;              // [2][W][3][JT] float
+	static constexpr int ROWLO = COL + 2 * W * 3 * JT * 4;        // [B][T] float4 (SYM_NEAR)
+	static constexpr int BYTES = ROWLO + (KIND == SYM_NEAR ? B * T * 16 : 0);
+};
+
+// Column sums of the j-tile `jt` (block J > I) -> column slot of (I, J), the warps added in
+// order.  They are FP32 sums, so they go out as FP32 (first half of the slot; stage 2 adds
+// them by TwoSum in FP32): half the bytes of an FP64 slot.  s: the segment of block I.
+template <int W, int T, int JT, int R>
+__device__ __forceinline__ void flush_columns(const grav_batch& b, int s, int blkI, int blkJ,
+	int64_t jt, const float* __restrict__ col, int tid)
 {
+	const grav_seg_desc SJ = b.seg[s + (blkJ - blkI)];
+	const int64_t slot = SJ.slot_base + SJ.nslots - (blkJ - blkI);
+	float* __restrict__ out = reinterpret_cast<float*>(b.part + slot * 3 * R) +
+		(jt * JT - static_cast<int64_t>(blkJ) * R);
+	for (int i = tid; i < JT; i += T) {
+#pragma unroll
+		for (int c = 0; c < 3; ++c) {
+			float sum = col[c * JT + i];
+#pragma unroll
+			for (int w = 1; w < W; ++w) sum += col[(w * 3 + c) * JT + i];
+			out[c * R + i] = sum;
+		}
+	}
+}
+
+// Fold a packed pair of row partials into the rows' compensated sums (entries sums[0] and
+// sums[T]).
+__device__ __forceinline__ void fold_pair(float2* sums, int T, u64 f)
+{
+	float f0, f1;
+	unpack2(f, f0, f1);
+	float2 a = sums[0], c = sums[T];
+	two_sum_acc(a.x, a.y, f0);
+	two_sum_acc(c.x, c.y, f1);
+	sums[0] = a;
+	sums[T] = c;
+}
+
+// The near correction of one column body (pj, low part lj) against a thread's rows: pairs
+// closer than the near radius again, from the double-single separation, the difference
+// added to the rows' sums f and (COLS) the rows' column terms, Gm_i e, to q.  Warp-uniform:
+// every lane calls it with its own body and the votes keep the lanes together.
+template <int H, int T, bool COLS>
+__device__ __forceinline__ void near_rows(const float4& pj, const float4& lj, float eps2, float thr,
+	const u64 (&nx)[H], const u64 (&ny)[H], const u64 (&nz)[H], const u64 (&g2)[H],
+	const float4* __restrict__ rowlo, u64 (&fx)[H], u64 (&fy)[H], u64 (&fz)[H], float& qx,
+	float& qy, float& qz)
+{
+	const u64 px = pack2(pj.x, pj.x), py = pack2(pj.y, pj.y), pz = pack2(pj.z, pj.z);
+	const u64 pw = pack2(pj.w, pj.w), eps22 = pack2(eps2, eps2);
+#pragma unroll
+	for (int h = 0; h < H; ++h) {
+		const u64 dx = add2(px, nx[h]), dy = add2(py, ny[h]), dz = add2(pz, nz[h]);
+		float ra, rb;
+		unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
+		const bool na = (ra < thr) & (ra > eps2), nb = (rb < thr) & (rb > eps2);
+		if (__any_sync(0xffffffffu, na | nb)) {
+			float x0, x1, y0, y1, z0, z1, ex0, ey0, ez0, ex1, ey1, ez1;
+			unpack2(dx, x0, x1);
+			unpack2(dy, y0, y1);
+			unpack2(dz, z0, z1);
+			near_delta(x0, y0, z0, ra, lj, rowlo[(2 * h) * T], eps2, na, ex0, ey0, ez0);
+			near_delta(x1, y1, z1, rb, lj, rowlo[(2 * h + 1) * T], eps2, nb, ex1, ey1, ez1);
+			fx[h] = fma2(pack2(ex0, ex1), pw, fx[h]);
+			fy[h] = fma2(pack2(ey0, ey1), pw, fy[h]);
+			fz[h] = fma2(pack2(ez0, ez1), pw, fz[h]);
+			if (COLS) {
+				float ga, gb;
+				unpack2(g2[h], ga, gb);
+				qx = fmaf(ex1, gb, fmaf(ex0, ga, qx));
+				qy = fmaf(ey1, gb, fmaf(ey0, ga, qy));
+				qz = fmaf(ez1, gb, fmaf(ez0, ga, qz));
+			}
+		}
+	}
+}
+
+// Expand a j-tile for the packed loops: every coordinate twice in a 64-bit pair, (x, x | y, y)
+// and (z, z | Gm, Gm), and the 32 bodies of a chunk twice in a row, so that lane l reads
+// body (l + s) mod 32 at constant offset s.
+template <int T, int JT, bool DS>
+__device__ __forceinline__ void expand_tile(ulonglong2* __restrict__ ex,
+	const float4* __restrict__ hi, const float4* __restrict__ lo, int tid)
+{
+	constexpr int EXA = DS ? 4 : 2;
+	for (int i = tid; i < JT; i += T) {
+		ulonglong2* __restrict__ q = ex + (i >> 5) * (EXA * 64) + (i & 31);
+		const float4 p = hi[i];
+		const ulonglong2 xy = make_ulonglong2(pack2(p.x, p.x), pack2(p.y, p.y));
+		const ulonglong2 zw = make_ulonglong2(pack2(p.z, p.z), pack2(p.w, p.w));
+		q[0] = q[32] = xy;
+		q[64] = q[96] = zw;
+		if (DS) {
+			const float4 l = lo[i];
+			const ulonglong2 lxy = make_ulonglong2(pack2(l.x, l.x), pack2(l.y, l.y));
+			const ulonglong2 lz = make_ulonglong2(pack2(l.z, l.z), 0ull);
+			q[128] = q[160] = lxy;
+			q[192] = q[224] = lz;
+		}
+	}
+}
+
+// B rows per thread, W warps, j-tiles of JT bodies; MINB CTAs per SM (the register limit);
+// COLPAIR: the even and odd rows' column sums rotate apart (two shuffles per component, for
+// DS and NEAR: 1.56 against 1.60 and 1.34 against 1.37 ms) or added up in each step (one
+// shuffle and two additions, for PLAIN: 1.17 against 1.19 ms).
+template <int B, int W, int JT, int KIND, int UNROLL, int MINB, bool COLPAIR>
+__global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_batch b)
+{
+	using L = SymSmem<B, W, JT, KIND>;
 	constexpr int T = 32 * W;
 	constexpr int R = T * B;            // rows per block (= itile)
+	constexpr int H = B / 2;            // packed pairs of rows per thread
 	constexpr int TPB = R / JT;         // j-tiles per block
 	constexpr int NCH = JT / 32;        // 32-body chunks per j-tile
 	constexpr uint32_t TILE_BYTES = JT * sizeof(float4);
-	constexpr int NP = KIND == SYM_PLAIN ? 1 : 2;   // position arrays copied per j-tile
+	constexpr int NP = L::NP;                       // position arrays copied per j-tile
 	constexpr bool DS = KIND == SYM_DS;             // double-single separations everywhere
 	constexpr bool NEAR = KIND == SYM_NEAR;         // double-single for near pairs only
-	static_assert(R % JT == 0 && JT % 32 == 0, "tile shapes");
-	extern __shared__ __align__(128) float4 sym_tiles[];   // [2 buffers][NP][JT]
+	static_assert(B % 2 == 0 && R % JT == 0 && JT % 32 == 0 && (NCH & (NCH - 1)) == 0, "tile shapes");
+	extern __shared__ __align__(128) unsigned char sym_smem[];
+	float4* const raw = reinterpret_cast<float4*>(sym_smem + L::RAW);
+	ulonglong2* const ex = reinterpret_cast<ulonglong2*>(sym_smem + L::EX);
+	// compensated row sums (hi, lo) of this thread's rows, touched once per j-tile
+	float2* const csum = reinterpret_cast<float2*>(sym_smem + L::CSUM) + threadIdx.x;  // [c][k]: (c * B + k) * T
 	// column sums of a j-tile, one row per warp: every warp writes each chunk of the tile
 	// once, and the flush adds the warps in a fixed order (no shared-memory atomics, whose
 	// order would depend on warp timing)
-	__shared__ float colacc[W][3][JT];
+	float* const colacc = reinterpret_cast<float*>(sym_smem + L::COL);
+	// low parts of this thread's rows (NEAR), read back on the cold path only
+	float4* const rowlo = reinterpret_cast<float4*>(sym_smem + L::ROWLO) + threadIdx.x;  // [k]: k * T
 	__shared__ __align__(8) uint64_t bar[2];
-	// low parts of this thread's rows (NEAR): read only on the cold correction path, by
-	// the thread that wrote them ([k][tid]: conflict-free 16-byte accesses)
-	__shared__ float4 rowlo[NEAR ? B : 1][NEAR ? T : 1];
-	// NEAR with 8 rows per thread keeps the compensated row sums (hi, lo) in shared memory
-	// instead of 48 registers, touched once per j-tile: the cold correction path's
-	// registers would otherwise cost a resident CTA per SM
-	constexpr bool SS = NEAR && B >= 8;
-	__shared__ float2 csum[SS ? 3 : 1][SS ? B : 1][SS ? T : 1];
 
 	const int tid = threadIdx.x;
 	const int lane = tid & 31;
@@ -88,11 +223,10 @@ __global__ void __launch_bounds__(32 * W) stage1_sym_kernel(const grav_batch b)
 
 	const float4* __restrict__ pos = static_cast<const float4*>(b.pos);
 	const float eps2 = b.eps2;
+	const u64 eps22 = pack2(eps2, eps2);
 
-	// Segment of unit ub by bisection, and no programmatic-launch instructions: this
-	// kernel runs for 1e5-1e6 cycles per CTA, where a few microseconds of prologue do
-	// not matter, and with the warp-parallel search or griddepcontrol in it the
-	// compiled main loop measured 1-4 % slower on GB300 (N = 65536, tile 8/128/256).
+	// Segment of unit ub by bisection, and no programmatic-launch instructions: a CTA runs
+	// for 1e5-1e6 cycles, where a few microseconds of prologue do not matter.
 	int s;
 	{
 		int lo = 0, hi = b.n_seg - 1;
@@ -104,8 +238,8 @@ __global__ void __launch_bounds__(32 * W) stage1_sym_kernel(const grav_batch b)
 		s = lo;
 	}
 
-	uint32_t gt = 0;
-	bool timed_out = false;
+	uint32_t gt = 0;   // tiles of this CTA before this piece (tile g: buffer g & 1, phase g >> 1)
+	int in_flight = 0;  // copies in flight when a wait expired, the first one that of tile gt
 	while (ub < ue && s < b.n_seg) {
 		const grav_seg_desc S = b.seg[s];
 		if (S.n_units == 0 || S.unit_begin + S.n_units <= ub) {
@@ -117,71 +251,82 @@ __global__ void __launch_bounds__(32 * W) stage1_sym_kernel(const grav_batch b)
 		const int64_t t0 = ub - S.unit_begin;                              // local unit
 		const int64_t t1 = min(ue - S.unit_begin, (int64_t)S.n_units);
 		const int nt = static_cast<int>(t1 - t0);
-		const int64_t jt_first = static_cast<int64_t>(blkI) * TPB;       // global j-tile of unit 0
+		const int64_t jt_first = static_cast<int64_t>(blkI) * TPB + t0;  // global j-tile of unit t0
 		const float4* __restrict__ jsrc = pos + Uu.pad_off;
 		const float4* __restrict__ jsrclo = pos + b.n_pad_total + Uu.pad_off;
-
-		if (tid == 0) {
-			const int bs = gt & 1;
+		const auto copy_tile = [&](int t) {   // tile t of this piece -> buffer (gt + t) & 1
+			const int bs = (gt + t) & 1;
 			mbar_arrive_expect_tx(&bar[bs], NP * TILE_BYTES);
-			bulk_g2s(sym_tiles + bs * NP * JT, jsrc + (jt_first + t0) * JT, TILE_BYTES, &bar[bs]);
+			bulk_g2s(raw + bs * NP * JT, jsrc + (jt_first + t) * JT, TILE_BYTES, &bar[bs]);
 			if (NP == 2)
-				bulk_g2s(sym_tiles + (bs * NP + 1) * JT, jsrclo + (jt_first + t0) * JT, TILE_BYTES,
-					&bar[bs]);
+				bulk_g2s(raw + (bs * NP + 1) * JT, jsrclo + (jt_first + t) * JT, TILE_BYTES, &bar[bs]);
+		};
+		// wait for tile t and expand this thread's share of it; false when the wait expired
+		const auto expand = [&](int t) {
+			const int bs = (gt + t) & 1;
+			if (!mbar_wait_bounded(&bar[bs], ((gt + t) >> 1) & 1)) return false;
+			expand_tile<T, JT, DS>(ex + bs * L::EX_TILE, raw + bs * NP * JT, raw + (bs * NP + 1) * JT, tid);
+			return true;
+		};
+		if (tid == 0) {
+			copy_tile(0);
+			if (nt > 1) copy_tile(1);
 		}
 
-		// rows of this warp: w*32*B + k*32 + lane
+		// rows of this warp: w*32*B + k*32 + lane, packed (2h, 2h + 1), coordinates negated so
+		// that a separation is one packed add
 		const int64_t ibase = Uu.pad_off + S.il0 + warp * 32 * B + lane;
-		float xi[B], yi[B], zi[B], gi[B], fx[B], fy[B], fz[B];
-		float xl[B], yl[B], zl[B];                       // low parts (DS)
-		float hx[B], hy[B], hz[B], lx[B], ly[B], lz[B];  // compensated row sums
+		u64 nx[H], ny[H], nz[H], g2[H], fx[H], fy[H], fz[H];
+		u64 nxl[H], nyl[H], nzl[H];                      // low parts (DS)
 		float xmax = 0.f;                                // NEAR: largest |coordinate| of the rows
 #pragma unroll
-		for (int k = 0; k < B; ++k) {
-			const float4 p = pos[ibase + k * 32];
-			xi[k] = p.x;
-			yi[k] = p.y;
-			zi[k] = p.z;
-			gi[k] = p.w;
+		for (int h = 0; h < H; ++h) {
+			const float4 p = load_row(pos + ibase + (2 * h) * 32);
+			const float4 q = load_row(pos + ibase + (2 * h + 1) * 32);
+			nx[h] = pack2(-p.x, -q.x);
+			ny[h] = pack2(-p.y, -q.y);
+			nz[h] = pack2(-p.z, -q.z);
+			g2[h] = pack2(p.w, q.w);
+			nxl[h] = nyl[h] = nzl[h] = 0ull;
 			if (DS) {
-				const float4 q = pos[b.n_pad_total + ibase + k * 32];
-				xl[k] = q.x;
-				yl[k] = q.y;
-				zl[k] = q.z;
-			} else {
-				xl[k] = yl[k] = zl[k] = 0.f;
+				const float4 pl = load_row(pos + b.n_pad_total + ibase + (2 * h) * 32);
+				const float4 ql = load_row(pos + b.n_pad_total + ibase + (2 * h + 1) * 32);
+				nxl[h] = pack2(-pl.x, -ql.x);
+				nyl[h] = pack2(-pl.y, -ql.y);
+				nzl[h] = pack2(-pl.z, -ql.z);
 			}
 			if (NEAR) {
-				rowlo[NEAR ? k : 0][NEAR ? tid : 0] = pos[b.n_pad_total + ibase + k * 32];
-				xmax = fmaxf(xmax, near_scale(p.x, p.y, p.z));
+				rowlo[(2 * h) * T] = pos[b.n_pad_total + ibase + (2 * h) * 32];
+				rowlo[(2 * h + 1) * T] = pos[b.n_pad_total + ibase + (2 * h + 1) * 32];
+				xmax = fmaxf(xmax, fmaxf(near_scale(p.x, p.y, p.z), near_scale(q.x, q.y, q.z)));
 			}
-			fx[k] = fy[k] = fz[k] = 0.f;
-			hx[k] = hy[k] = hz[k] = lx[k] = ly[k] = lz[k] = 0.f;
-			if (SS) {
-#pragma unroll
-				for (int cpt = 0; cpt < 3; ++cpt) csum[SS ? cpt : 0][SS ? k : 0][SS ? tid : 0] = make_float2(0.f, 0.f);
-			}
+			fx[h] = fy[h] = fz[h] = 0ull;
 		}
+#pragma unroll
+		for (int e = 0; e < 3 * B; ++e) csum[e * T] = make_float2(0.f, 0.f);
 		const float thr = near_threshold(xmax);
 
-		for (int t = 0; t < nt; ++t, ++gt) {
-			const int bs = gt & 1;
-			const bool ok = mbar_wait_bounded(&bar[bs], (gt >> 1) & 1);
+		bool ok = expand(0);
+		int blk_done = 0;   // block J of the previous tile when it left column sums, else 0
+		for (int t = 0; t < nt; ++t) {
+			// every warp has finished tile t - 1, its share of tile t is expanded, and its
+			// column sums of tile t - 1 are in colacc
 			if (__syncthreads_or(!ok)) {
-				timed_out = true;
+				in_flight = t == 0 && nt > 1 ? 2 : 1;
+				gt += t;
 				break;
 			}
-			const int64_t jt = jt_first + t0 + t;  // global j-tile index in the universe
-			if (tid == 0 && t + 1 < nt) {
-				const int bn = (gt + 1) & 1;
-				mbar_arrive_expect_tx(&bar[bn], NP * TILE_BYTES);
-				bulk_g2s(sym_tiles + bn * NP * JT, jsrc + (jt + 1) * JT, TILE_BYTES, &bar[bn]);
-				if (NP == 2)
-					bulk_g2s(sym_tiles + (bn * NP + 1) * JT, jsrclo + (jt + 1) * JT, TILE_BYTES,
-						&bar[bn]);
+			const int bs = (gt + t) & 1;
+			if (t > 0) {
+				if (tid == 0 && t + 1 < nt) copy_tile(t + 1);   // over tile t - 1
+				if (blk_done)
+					flush_columns<W, T, JT, R>(b, s, blkI, blk_done, jt_first + t - 1,
+						colacc + (bs ^ 1) * W * 3 * JT, tid);
 			}
-			const float4* __restrict__ sj = sym_tiles + bs * NP * JT;
-			const float4* __restrict__ sjl = sj + JT;  // low parts (NP == 2)
+			const int64_t jt = jt_first + t;   // j-tile index in the universe
+			const float4* __restrict__ sj = raw + bs * NP * JT;
+			const float4* __restrict__ sjl = sj + JT;   // low parts (NP == 2)
+			const ulonglong2* __restrict__ et = ex + bs * L::EX_TILE;
 			const int blkJ = static_cast<int>(jt / TPB);
 			if (blkJ == blkI) {
 				// diagonal block: every ordered pair of the block once, rows only.  In NEAR
@@ -190,220 +335,228 @@ __global__ void __launch_bounds__(32 * W) stage1_sym_kernel(const grav_batch b)
 				// do not send the warp down the correction path
 				const int jl0 = static_cast<int>(jt - static_cast<int64_t>(blkI) * TPB) * JT;
 				const bool own = jl0 < (warp + 1) * 32 * B && jl0 + JT > warp * 32 * B;
-#pragma unroll 4
-				for (int j = 0; j < JT; ++j) {
-					const float4 pj = sj[j];
-					float4 lj = make_float4(0.f, 0.f, 0.f, 0.f);
-					if (DS) lj = sjl[j];
-					bool near = false;
-#pragma unroll
-					for (int k = 0; k < B; ++k) {
-						float dx = pj.x - xi[k], dy = pj.y - yi[k], dz = pj.z - zi[k];
+#pragma unroll 1
+				for (int ch = 0; ch < NCH; ++ch) {
+					const ulonglong2* __restrict__ se = et + ch * (L::EXA * 64);
+					uint32_t nmask = 0;
+#pragma unroll 2
+					for (int j = 0; j < 32; ++j) {
+						const ulonglong2 pxy = se[j], pzw = se[64 + j];
+						ulonglong2 lxy = make_ulonglong2(0ull, 0ull), lz = lxy;
 						if (DS) {
-							dx = dx + (lj.x - xl[k]);
-							dy = dy + (lj.y - yl[k]);
-							dz = dz + (lj.z - zl[k]);
+							lxy = se[128 + j];
+							lz = se[192 + j];
 						}
-						const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
-						if (NEAR) near |= own ? (r2 < thr) & (r2 > eps2) : (r2 < thr);
-						const float inv = rsqrt_sfu(r2);
-						float w = pj.w * inv;
-						w = w * (inv * inv);
-						fx[k] = fmaf(dx, w, fx[k]);
-						fy[k] = fmaf(dy, w, fy[k]);
-						fz[k] = fmaf(dz, w, fz[k]);
-					}
-					if (NEAR && __any_sync(0xffffffffu, near)) {
-						lj = sjl[j];
+						bool near = false;
 #pragma unroll
-						for (int k = 0; k < B; ++k) {
-							const float dx = pj.x - xi[k], dy = pj.y - yi[k], dz = pj.z - zi[k];
-							const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
-							const bool nk = (r2 < thr) & (r2 > eps2);
-							if (__any_sync(0xffffffffu, nk)) {
-								float ex, ey, ez;
-								near_delta(dx, dy, dz, r2, lj, rowlo[NEAR ? k : 0][NEAR ? tid : 0],
-									eps2, nk, ex, ey, ez);
-								fx[k] = fmaf(ex, pj.w, fx[k]);
-								fy[k] = fmaf(ey, pj.w, fy[k]);
-								fz[k] = fmaf(ez, pj.w, fz[k]);
+						for (int h = 0; h < H; ++h) {
+							u64 dx = add2(pxy.x, nx[h]), dy = add2(pxy.y, ny[h]), dz = add2(pzw.x, nz[h]);
+							if (DS) {
+								dx = add2(dx, add2(lxy.x, nxl[h]));
+								dy = add2(dy, add2(lxy.y, nyl[h]));
+								dz = add2(dz, add2(lz.x, nzl[h]));
 							}
+							float ra, rb;
+							unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
+							if (NEAR)
+								near |= own ? ((ra < thr) & (ra > eps2)) | ((rb < thr) & (rb > eps2))
+								            : (ra < thr) | (rb < thr);
+							const u64 inv = pack2(rsqrt_sfu(ra), rsqrt_sfu(rb));
+							const u64 w = mul2(mul2(pzw.y, inv), mul2(inv, inv));
+							fx[h] = fma2(dx, w, fx[h]);
+							fy[h] = fma2(dy, w, fy[h]);
+							fz[h] = fma2(dz, w, fz[h]);
+						}
+						if (NEAR && near) nmask |= 1u << j;
+					}
+					if (NEAR) {
+						uint32_t todo = __reduce_or_sync(0xffffffffu, nmask);
+						while (todo) {
+							const int j = __ffs(todo) - 1;
+							todo &= todo - 1;
+							float qx = 0.f, qy = 0.f, qz = 0.f;
+							near_rows<H, T, false>(sj[ch * 32 + j], sjl[ch * 32 + j], eps2, thr, nx, ny, nz,
+								g2, rowlo, fx, fy, fz, qx, qy, qz);
 						}
 					}
 				}
+				blk_done = 0;
 			} else {
 				// unique pairs with block J > I: rotate the chunk's column sums
+				float* __restrict__ cw = colacc + (bs * W + warp) * 3 * JT;
 #pragma unroll 1
 				for (int cc = 0; cc < NCH; ++cc) {
 					const int ch = (cc + warp) & (NCH - 1);
-					const float4* __restrict__ sc = sj + ch * 32;
-					const float4* __restrict__ scl = sjl + ch * 32;
-					float cx = 0.f, cy = 0.f, cz = 0.f;
+					const ulonglong2* __restrict__ se = et + ch * (L::EXA * 64) + lane;
+					u64 cx = 0ull, cy = 0ull, cz = 0ull;     // even and odd rows' column sums
+					float sx = 0.f, sy = 0.f, sz = 0.f;
+					uint32_t nmask = 0;   // NEAR: bit 31 - st of a step st that met a near pair
 #pragma unroll UNROLL
 					for (int st = 0; st < 32; ++st) {
-						const float4 pj = sc[(lane + st) & 31];
-						float4 lj = make_float4(0.f, 0.f, 0.f, 0.f);
-						if (DS) lj = scl[(lane + st) & 31];
-						float rmin = 0.f, rprev = 0.f;   // NEAR: smallest r2 of this step
+						const ulonglong2 pxy = se[st], pzw = se[64 + st];
+						ulonglong2 lxy = make_ulonglong2(0ull, 0ull), lz = lxy;
+						if (DS) {
+							lxy = se[128 + st];
+							lz = se[192 + st];
+						}
+						float rmin = 0.f;   // NEAR: smallest r2 of this step
+						if (!COLPAIR) cx = cy = cz = 0ull;
 #pragma unroll
-						for (int k = 0; k < B; ++k) {
-							float dx = pj.x - xi[k], dy = pj.y - yi[k], dz = pj.z - zi[k];
+						for (int h = 0; h < H; ++h) {
+							u64 dx = add2(pxy.x, nx[h]), dy = add2(pxy.y, ny[h]), dz = add2(pzw.x, nz[h]);
 							if (DS) {
-								dx = dx + (lj.x - xl[k]);
-								dy = dy + (lj.y - yl[k]);
-								dz = dz + (lj.z - zl[k]);
+								dx = add2(dx, add2(lxy.x, nxl[h]));
+								dy = add2(dy, add2(lxy.y, nyl[h]));
+								dz = add2(dz, add2(lz.x, nzl[h]));
 							}
-							const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
-							if (NEAR) near_min_step<B>(k, r2, rmin, rprev);
-							const float inv = rsqrt_sfu(r2);
-							const float inv3 = inv * (inv * inv);
-							const float wj = pj.w * inv3;
-							const float wi = gi[k] * inv3;
-							fx[k] = fmaf(dx, wj, fx[k]);
-							fy[k] = fmaf(dy, wj, fy[k]);
-							fz[k] = fmaf(dz, wj, fz[k]);
-							cx = fmaf(-dx, wi, cx);
-							cy = fmaf(-dy, wi, cy);
-							cz = fmaf(-dz, wi, cz);
-						}
-						if (NEAR && __any_sync(0xffffffffu, rmin < thr)) {
-							// cold path: the pairs of this step closer than the near radius
-							// again, from the double-single separation (row and column)
-							lj = scl[(lane + st) & 31];
-#pragma unroll
-							for (int k = 0; k < B; ++k) {
-								const float dx = pj.x - xi[k], dy = pj.y - yi[k], dz = pj.z - zi[k];
-								const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
-								const bool nk = (r2 < thr) & (r2 > eps2);
-								if (__any_sync(0xffffffffu, nk)) {
-									float ex, ey, ez;
-									near_delta(dx, dy, dz, r2, lj,
-										rowlo[NEAR ? k : 0][NEAR ? tid : 0], eps2, nk, ex, ey, ez);
-									fx[k] = fmaf(ex, pj.w, fx[k]);
-									fy[k] = fmaf(ey, pj.w, fy[k]);
-									fz[k] = fmaf(ez, pj.w, fz[k]);
-									cx = fmaf(-ex, gi[k], cx);
-									cy = fmaf(-ey, gi[k], cy);
-									cz = fmaf(-ez, gi[k], cz);
-								}
+							float ra, rb;
+							unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
+							if (NEAR) rmin = h == 0 ? fminf(ra, rb) : min3f(rmin, ra, rb);
+							const u64 inv = pack2(rsqrt_sfu(ra), rsqrt_sfu(rb));
+							const u64 inv3 = mul2(inv, mul2(inv, inv));
+							const u64 wj = mul2(pzw.y, inv3);
+							const u64 wi = mul2(g2[h], inv3);
+							fx[h] = fma2(dx, wj, fx[h]);
+							fy[h] = fma2(dy, wj, fy[h]);
+							fz[h] = fma2(dz, wj, fz[h]);
+							if (!COLPAIR && h == 0) {
+								cx = mul2(dx, wi);
+								cy = mul2(dy, wi);
+								cz = mul2(dz, wi);
+							} else {
+								cx = fma2(dx, wi, cx);
+								cy = fma2(dy, wi, cy);
+								cz = fma2(dz, wi, cz);
 							}
 						}
+						// both are >= 0, so they compare as integers; the sign goes into the mask
+						if (NEAR)
+							nmask = __funnelshift_l(__float_as_uint(rmin) - __float_as_uint(thr), nmask, 1);
 						const int src = (lane + 1) & 31;
-						cx = __shfl_sync(0xffffffffu, cx, src);
-						cy = __shfl_sync(0xffffffffu, cy, src);
-						cz = __shfl_sync(0xffffffffu, cz, src);
+						float a0, a1;
+						if (COLPAIR) {
+							unpack2(cx, a0, a1);
+							cx = pack2(__shfl_sync(0xffffffffu, a0, src), __shfl_sync(0xffffffffu, a1, src));
+							unpack2(cy, a0, a1);
+							cy = pack2(__shfl_sync(0xffffffffu, a0, src), __shfl_sync(0xffffffffu, a1, src));
+							unpack2(cz, a0, a1);
+							cz = pack2(__shfl_sync(0xffffffffu, a0, src), __shfl_sync(0xffffffffu, a1, src));
+						} else {
+							unpack2(cx, a0, a1);
+							sx = __shfl_sync(0xffffffffu, sx + (a0 + a1), src);
+							unpack2(cy, a0, a1);
+							sy = __shfl_sync(0xffffffffu, sy + (a0 + a1), src);
+							unpack2(cz, a0, a1);
+							sz = __shfl_sync(0xffffffffu, sz + (a0 + a1), src);
+						}
 					}
-					colacc[warp][0][ch * 32 + lane] = cx;
-					colacc[warp][1][ch * 32 + lane] = cy;
-					colacc[warp][2][ch * 32 + lane] = cz;
-				}
-				__syncthreads();
-				// column sums of this tile -> column slot of (I, J), the warps added in order.
-				// They are FP32 sums, so they go out as FP32 (first half of the slot; stage
-				// 2 adds them by TwoSum in FP32): half the bytes of an FP64 slot
-				const int sJ = s + (blkJ - blkI);
-				const grav_seg_desc SJ = b.seg[sJ];
-				const int64_t slot = SJ.slot_base + SJ.nslots - (blkJ - blkI);
-				float* __restrict__ out = reinterpret_cast<float*>(b.part + slot * 3 * R) +
-					(jt * JT - static_cast<int64_t>(blkJ) * R);
-				for (int i = tid; i < JT; i += T) {
-					float sx = colacc[0][0][i], sy = colacc[0][1][i], sz = colacc[0][2][i];
-#pragma unroll
-					for (int w = 1; w < W; ++w) {
-						sx += colacc[w][0][i];
-						sy += colacc[w][1][i];
-						sz += colacc[w][2][i];
+					if (COLPAIR) {
+						float a0, a1;
+						unpack2(cx, a0, a1);
+						sx = a0 + a1;
+						unpack2(cy, a0, a1);
+						sy = a0 + a1;
+						unpack2(cz, a0, a1);
+						sz = a0 + a1;
 					}
-					out[i] = sx;
-					out[R + i] = sy;
-					out[2 * R + i] = sz;
+					if (NEAR) {
+						// cold path: the steps that met pairs closer than the near radius again,
+						// from the double-single separation; their column terms belong to the
+						// body the lane met then, whose sum lane (lane + st) mod 32 now holds
+						uint32_t todo = __reduce_or_sync(0xffffffffu, nmask);
+						while (todo) {
+							const int st = __clz(todo);
+							todo &= ~(0x80000000u >> st);
+							const int jb = ch * 32 + ((lane + st) & 31);
+							float qx = 0.f, qy = 0.f, qz = 0.f;
+							near_rows<H, T, true>(sj[jb], sjl[jb], eps2, thr, nx, ny, nz, g2, rowlo, fx, fy,
+								fz, qx, qy, qz);
+							const int from = (lane - st) & 31;
+							sx += __shfl_sync(0xffffffffu, qx, from);
+							sy += __shfl_sync(0xffffffffu, qy, from);
+							sz += __shfl_sync(0xffffffffu, qz, from);
+						}
+					}
+					cw[ch * 32 + lane] = -sx;
+					cw[JT + ch * 32 + lane] = -sy;
+					cw[2 * JT + ch * 32 + lane] = -sz;
 				}
+				blk_done = blkJ;
 			}
+			// fold the tile's row partials into the compensated sums
 #pragma unroll
-			for (int k = 0; k < B; ++k) {
-				if (SS) {
-					float2* cs = &csum[0][SS ? k : 0][SS ? tid : 0];
-					constexpr int CS = SS ? B * T : 0;   // stride between components
-					float2 h0 = cs[0], h1 = cs[CS], h2 = cs[2 * CS];
-					two_sum_acc(h0.x, h0.y, fx[k]);
-					two_sum_acc(h1.x, h1.y, fy[k]);
-					two_sum_acc(h2.x, h2.y, fz[k]);
-					cs[0] = h0;
-					cs[CS] = h1;
-					cs[2 * CS] = h2;
-				} else {
-					two_sum_acc(hx[k], lx[k], fx[k]);
-					two_sum_acc(hy[k], ly[k], fy[k]);
-					two_sum_acc(hz[k], lz[k], fz[k]);
-				}
-				fx[k] = fy[k] = fz[k] = 0.f;
+			for (int h = 0; h < H; ++h) {
+				fold_pair(csum + (0 * B + 2 * h) * T, T, fx[h]);
+				fold_pair(csum + (1 * B + 2 * h) * T, T, fy[h]);
+				fold_pair(csum + (2 * B + 2 * h) * T, T, fz[h]);
+				fx[h] = fy[h] = fz[h] = 0ull;
 			}
+			ok = t + 1 < nt ? expand(t + 1) : true;
 		}
-		if (timed_out) break;
+		if (in_flight) break;
+		__syncthreads();   // colacc of the last tile is complete; the buffers are free again
+		if (blk_done)
+			flush_columns<W, T, JT, R>(b, s, blkI, blk_done, jt_first + nt - 1,
+				colacc + ((gt + nt - 1) & 1) * W * 3 * JT, tid);
+		gt += nt;
 
 		// row sums of this CTA's piece as FP32 (hi, lo) pairs, one 8-byte slot entry each
 		const int64_t slot = S.slot_base + (c - S.cta_first);
-		float2* __restrict__ out = reinterpret_cast<float2*>(b.part + slot * 3 * R);
-		const int r0 = warp * 32 * B + lane;
+		float2* __restrict__ out = reinterpret_cast<float2*>(b.part + slot * 3 * R) + warp * 32 * B + lane;
 #pragma unroll
-		for (int k = 0; k < B; ++k) {
-			if (SS) {
-				out[r0 + k * 32] = csum[0][SS ? k : 0][SS ? tid : 0];
-				out[R + r0 + k * 32] = csum[SS ? 1 : 0][SS ? k : 0][SS ? tid : 0];
-				out[2 * R + r0 + k * 32] = csum[SS ? 2 : 0][SS ? k : 0][SS ? tid : 0];
-			} else {
-				out[r0 + k * 32] = make_float2(hx[k], lx[k]);
-				out[R + r0 + k * 32] = make_float2(hy[k], ly[k]);
-				out[2 * R + r0 + k * 32] = make_float2(hz[k], lz[k]);
-			}
-		}
+		for (int cpt = 0; cpt < 3; ++cpt)
+#pragma unroll
+			for (int k = 0; k < B; ++k) out[cpt * R + k * 32] = csum[(cpt * B + k) * T];
 		ub = S.unit_begin + t1;
 		++s;
 	}
 
-	if (timed_out && tid == 0) {
+	if (in_flight && tid == 0) {
 		set_error(b.err, GRAV_DEV_TIMEOUT);
-		mbar_wait_bounded(&bar[gt & 1], (gt >> 1) & 1);
+		// give each copy in flight one more bounded wait, so that none lands in shared memory
+		// after this CTA exits
+		for (uint32_t g = gt; g < gt + in_flight; ++g) mbar_wait_bounded(&bar[g & 1], (g >> 1) & 1);
 	}
 }
 
 // launched the ordinary way (not as a programmatic dependent): see the kernel's prologue
-#define GRAV_SYM_ENTRY(B, W, J) \
-	{GRAV_MODE_FP32U, B, 32 * W, J, \
-		reinterpret_cast<const void*>(&stage1_sym_kernel<B, W, J, 4, SYM_PLAIN>), 2 * J * 16, false}
-#define GRAV_SYMC_ENTRY(B, W, J) \
-	{GRAV_MODE_FP32CU, B, 32 * W, J, \
-		reinterpret_cast<const void*>(&stage1_sym_kernel<B, W, J, 4, SYM_DS>), 2 * 2 * J * 16, false}
-// the near kernel's step loop is not unrolled: with its vote and cold path in every step
-// the unrolled form held 167 registers against 147 and ran 1.4 % slower (N = 65536,
-// tile 8/128/256: stage 1 1.458 against 1.438 ms; unrolled by 2 1.456, by 8 it spilled)
-#define GRAV_SYMN_ENTRY(B, W, J) \
-	{GRAV_MODE_FP32UN, B, 32 * W, J, \
-		reinterpret_cast<const void*>(&stage1_sym_kernel<B, W, J, 1, SYM_NEAR>), 2 * 2 * J * 16, false}
+#define GRAV_SYM_KERNEL(MODE, KIND, B, W, J, UN, MINB, CP) \
+	{MODE, B, 32 * W, J, \
+		reinterpret_cast<const void*>(&stage1_sym_kernel<B, W, J, KIND, UN, MINB, CP>), \
+		SymSmem<B, W, J, KIND>::BYTES, false}
+#define GRAV_SYM_ENTRY(B, W, J, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32U, SYM_PLAIN, B, W, J, 4, MINB, false)
+#define GRAV_SYMC_ENTRY(B, W, J, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32CU, SYM_DS, B, W, J, 4, MINB, true)
+#define GRAV_SYMN_ENTRY(B, W, J, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32UN, SYM_NEAR, B, W, J, 4, MINB, true)
 
+// The step loop is unrolled by 4 (by 2 fp32un 1.38, by 8 1.34, by 4 1.34 ms; by 16 and more it
+// spills).  MINB is the occupancy at which the loop keeps its registers: 8 rows per thread
+// want ~165 (fp32cu ~200); at 128 registers it measured 5-9 % slower.
 static const Stage1Kernel k_table_sym[] = {
-	GRAV_SYM_ENTRY(4, 4, 128),
-	GRAV_SYM_ENTRY(4, 8, 256),
-	GRAV_SYM_ENTRY(8, 4, 256),
-	GRAV_SYM_ENTRY(4, 4, 256),
-	GRAV_SYM_ENTRY(2, 8, 256),
-	GRAV_SYM_ENTRY(8, 8, 256),
-	GRAV_SYM_ENTRY(8, 4, 128),
-	GRAV_SYM_ENTRY(8, 4, 64),
-	GRAV_SYM_ENTRY(4, 2, 64),
-	GRAV_SYMC_ENTRY(4, 4, 128),
-	GRAV_SYMC_ENTRY(8, 4, 256),
-	GRAV_SYMC_ENTRY(4, 4, 256),
-	GRAV_SYMC_ENTRY(4, 8, 256),
-	GRAV_SYMN_ENTRY(4, 4, 128),
-	GRAV_SYMN_ENTRY(8, 4, 256),
-	GRAV_SYMN_ENTRY(8, 4, 128),
-	GRAV_SYMN_ENTRY(8, 4, 64),
-	GRAV_SYMN_ENTRY(4, 4, 256),
-	GRAV_SYMN_ENTRY(4, 8, 256),
-	GRAV_SYMN_ENTRY(4, 2, 64),
-	GRAV_SYMN_ENTRY(8, 2, 64),
-	GRAV_SYMN_ENTRY(8, 2, 128),
+	GRAV_SYM_ENTRY(4, 4, 128, 4),
+	GRAV_SYM_ENTRY(4, 8, 256, 2),
+	GRAV_SYM_ENTRY(8, 4, 256, 2),
+	GRAV_SYM_ENTRY(4, 4, 256, 3),
+	GRAV_SYM_ENTRY(2, 8, 256, 2),
+	GRAV_SYM_ENTRY(8, 8, 256, 1),
+	GRAV_SYM_ENTRY(8, 4, 128, 3),
+	GRAV_SYM_ENTRY(8, 4, 64, 3),
+	GRAV_SYM_ENTRY(4, 2, 64, 8),
+	GRAV_SYMC_ENTRY(4, 4, 128, 3),
+	GRAV_SYMC_ENTRY(8, 4, 256, 1),
+	GRAV_SYMC_ENTRY(4, 4, 256, 2),
+	GRAV_SYMC_ENTRY(4, 8, 256, 1),
+	GRAV_SYMC_ENTRY(8, 4, 128, 2),
+	GRAV_SYMC_ENTRY(4, 2, 64, 6),
+	GRAV_SYMC_ENTRY(8, 2, 64, 5),
+	GRAV_SYMN_ENTRY(4, 4, 128, 3),
+	GRAV_SYMN_ENTRY(8, 4, 256, 2),
+	GRAV_SYMN_ENTRY(8, 4, 128, 3),
+	GRAV_SYMN_ENTRY(8, 4, 64, 3),
+	GRAV_SYMN_ENTRY(4, 4, 256, 2),
+	GRAV_SYMN_ENTRY(4, 8, 256, 1),
+	GRAV_SYMN_ENTRY(4, 2, 64, 7),
+	GRAV_SYMN_ENTRY(8, 2, 64, 5),
+	GRAV_SYMN_ENTRY(8, 2, 128, 4),
 };
 
 int stage1_table_sym(const Stage1Kernel** out)

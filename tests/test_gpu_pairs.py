@@ -1,0 +1,74 @@
+"""GPU tests of the packed unique-pair kernels (stage1_sym.cu) at the edges of their tiles:
+every compiled shape of every unique-pair mode with one body below, at and above one row
+block, with several blocks and a ragged end, and with pairs of bodies 1e-3 apart at
+|x| ~ 1000 planted inside a block and across blocks (the near correction's row and column
+terms).
+
+Tolerance, per body: |a - a_ref| <= 1e-5 sum_j |a_ij|, a_ij the pair terms in FP64.  A pair
+term carries the rounding of the FP32 operations that form it (about ten, each 2^-24, and
+the reciprocal square root's 2^-22 three times: below 1.5e-6) and, in fp32un, up to 4.5e-6
+from the rounding of positions beyond the near radius; the FP32 partial sums of at most 256
+terms add less than 2e-6 (random rounding signs).
+"""
+
+import numpy as np
+import pytest
+
+import oracle
+from gravitation_gb300 import _lib
+from gravitation_gb300.engine import Engine, tile_list
+from gravitation_gb300.scenarios import G_DEFAULT, uniform_cube
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+
+
+def planted_cube(n, rows, seed):
+    """A uniform cube with close pairs: within the first block and from the first to the
+    last body's block."""
+    r, v, m = uniform_cube(n, seed=seed)
+    rng = np.random.default_rng(seed + 1)
+    for k in range(6):
+        for i, j in ((7 + 40 * k, 23 + 40 * k), (11 + 40 * k, n - 3 - 5 * k)):
+            if max(i, j) < n and i < min(rows, n) and j > i:
+                r[i] = np.sign(r[i]) * 990.0 + rng.uniform(-5, 5, 3)
+                r[j] = r[i] + rng.uniform(-1e-3, 1e-3, 3)
+    return r, v, m
+
+
+def magnitudes(r, gm):
+    """sum_j Gm_j / |r_j - r_i|^2 per body."""
+    out = np.zeros(len(gm))
+    for i in range(0, len(gm), 256):
+        d2 = ((r[None, :, :] - r[i:i + 256, None, :]) ** 2).sum(-1)
+        with np.errstate(divide='ignore'):
+            out[i:i + 256] = np.where(d2 > 0, gm[None, :] / d2, 0.0).sum(1)
+    return out
+
+
+@pytest.mark.parametrize('mode', ['fp32u', 'fp32cu', 'fp32un'])
+@pytest.mark.parametrize('case', ['below', 'block', 'above', 'ragged'])
+def test_pair_tiles_at_block_edges(gpu, mode, case):
+    done = {}
+    for t in tile_list(mode):
+        rows = t.bpt * t.threads
+        n = {'below': rows - 1, 'block': rows, 'above': rows + 1,
+             'ragged': 2 * rows + t.jtile + 33}[case]
+        if n not in done:
+            r, v, m = planted_cube(n, rows, seed=900 + n)
+            gm = G_DEFAULT * m
+            rr, gg = r, gm
+            if mode == 'fp32u':   # plain FP32 separations: on the positions it reads
+                rr = r.astype(np.float32).astype(np.float64)
+                gg = gm.astype(np.float32).astype(np.float64)
+            done[n] = (r, v, gm, oracle.accel_fp64(rr, gg, 1.0, coincident=True),
+                       magnitudes(rr, gg))
+        r, v, gm, ref, scale = done[n]
+        for grid in (0, 5):
+            eng = Engine([n], 1e3, mode=mode, tile=_lib.Tile(t.bpt, t.threads, t.jtile, grid))
+            eng.set_state(r, v, gm)
+            a = eng.forces().cpu().numpy()
+            eng.raise_on_device_error()
+            err = np.linalg.norm(a - ref, axis=1) / scale
+            assert err.max() < TOL, (mode, t, grid, n, err.max())
