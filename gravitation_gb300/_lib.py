@@ -12,7 +12,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, 'libgravgb300.so')
 
 # ---- constants (mirror of the header) -------------------------------------------
-GRAV_ABI_VERSION = 5
+GRAV_ABI_VERSION = 6
 GRAV_OK = 0
 GRAV_E_ARG = -1
 GRAV_E_TILE = -2
@@ -134,6 +134,10 @@ _DECLS = {
                                             ctypes.c_int32, _P(ctypes.c_int32)]),
     'grav_step_fused': (ctypes.c_int, [_P(Batch), ctypes.c_int, ctypes.c_int32, ctypes.c_int32,
                                        ctypes.c_void_p, ctypes.c_void_p]),
+    'grav_steps_supported': (ctypes.c_int, [ctypes.c_int, ctypes.c_int32, ctypes.c_int32]),
+    'grav_steps_scratch_bytes': (ctypes.c_int64, [ctypes.c_int32]),
+    'grav_steps': (ctypes.c_int, [_P(Batch), ctypes.c_int, ctypes.c_int32, ctypes.c_int64,
+                                  ctypes.c_void_p, ctypes.c_void_p]),
     'grav_fp32_peak_probe': (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32,
                                             ctypes.c_void_p]),
     'grav_energy': (ctypes.c_int, [_P(Batch), ctypes.c_void_p, ctypes.c_void_p]),

@@ -213,21 +213,11 @@ class Rollout:
         return [(s, min(s + self.every, self.steps)) for s in starts]
 
     def _fwd_launch(self, s0, s1, stream):
-        """Forward steps s0 .. s1-1; with store_a each writes its accelerations to acc[k]
-        (the batch's a_out is pointed there for that launch and restored after)."""
-        f = self.fwd
-        if not self.store_a:
-            f.step(s1 - s0, stream=stream)
-            return
-        flags = _lib.GRAV_S2_INTEGRATE | _lib.GRAV_S2_WRITE_A
-        h = f._h(stream)
-        keep = f.batch.a_out
-        try:
-            for k in range(s0, s1):
-                f.batch.a_out = self.acc[k].data_ptr()
-                check(f.lib.grav_step(f._bref, flags, h))
-        finally:
-            f.batch.a_out = keep
+        """Forward steps s0 .. s1-1; with store_a each writes its accelerations to acc[k]."""
+        if self.store_a:
+            self.fwd.steps_to(self.acc[s0:s1], stream=stream)
+        else:
+            self.fwd.step(s1 - s0, stream=stream)
 
     def _graph(self, cache, key, device, enqueue):
         g = cache.get(key)

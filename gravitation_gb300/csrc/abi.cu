@@ -461,6 +461,46 @@ int grav_step_fused(const grav_batch* b, int flags, int32_t threads, int32_t row
 	return ok();
 }
 
+int grav_steps_supported(int mode, int32_t n, int32_t sm_count)
+{
+	return grav::steps_supported(mode, n, sm_count) ? 1 : 0;
+}
+
+int64_t grav_steps_scratch_bytes(int32_t n)
+{
+	if (n < 0) return fail(GRAV_E_ARG, "n < 0");
+	return grav::steps_scratch(n);
+}
+
+int grav_steps(const grav_batch* b, int flags, int32_t steps, int64_t a_stride, void* scratch,
+	void* stream)
+{
+	int rc = check_batch(b);
+	if (rc) return rc;
+	if (b->n_univ != 1) return fail(GRAV_E_ARG, "grav_steps takes one universe (n_univ = %d)", b->n_univ);
+	if (steps < 0) return fail(GRAV_E_ARG, "steps < 0");
+	if (!scratch) return fail(GRAV_E_ARG, "scratch is NULL");
+	if (!b->err) return fail(GRAV_E_ARG, "NULL err pointer");
+	if (flags & ~(GRAV_S2_INTEGRATE | GRAV_S2_WRITE_A))
+		return fail(GRAV_E_ARG, "grav_steps takes GRAV_S2_INTEGRATE and GRAV_S2_WRITE_A only");
+	if (!(flags & GRAV_S2_INTEGRATE) && steps > 1)
+		return fail(GRAV_E_ARG, "more than one step without GRAV_S2_INTEGRATE");
+	if ((flags & GRAV_S2_WRITE_A) && !b->a_out) return fail(GRAV_E_ARG, "GRAV_S2_WRITE_A without a_out");
+	if ((flags & GRAV_S2_INTEGRATE) && !b->v) return fail(GRAV_E_ARG, "NULL v pointer");
+	if (a_stride < 0) return fail(GRAV_E_ARG, "a_stride < 0");
+	if (b->n_bodies == 0 || steps == 0) return ok();
+	int dev = 0, sms = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+	if (e != cudaSuccess) return cuda_fail(e, "SM count query");
+	if (b->n_bodies > INT32_MAX || !grav::steps_supported(b->mode, static_cast<int>(b->n_bodies), sms))
+		return fail(GRAV_E_SIZE, "grav_steps does not take %lld bodies in mode %d",
+			(long long)b->n_bodies, b->mode);
+	e = grav::launch_steps(*b, flags, steps, a_stride, scratch, sms, static_cast<cudaStream_t>(stream));
+	if (e != cudaSuccess) return cuda_fail(e, "multi-step launch");
+	return ok();
+}
+
 int grav_host_device_pointer(const void* host, void** dev)
 {
 	if (!host || !dev) return fail(GRAV_E_ARG, "NULL host or dev pointer");

@@ -30,6 +30,12 @@ cudaError_t launch_fused(const grav_batch& b, int flags, int threads, int rows, 
 	cudaStream_t stream);
 int fused_occupancy(int mode, int64_t n, int threads, int rows, int* ctas_per_sm);
 
+// K steps of one universe in one launch (steps.cu).
+bool steps_supported(int mode, int n, int sms);
+int64_t steps_scratch(int n);
+cudaError_t launch_steps(const grav_batch& b, int flags, int steps, int64_t a_stride, void* scratch,
+	int sms, cudaStream_t stream);
+
 // Kernel tables, one per translation unit (stage1_f32.cu, stage1_f64.cu).
 int stage1_table_f32(const Stage1Kernel** out);
 int stage1_table_f64(const Stage1Kernel** out);

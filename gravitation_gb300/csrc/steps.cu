@@ -1,0 +1,697 @@
+// steps.cu -- K full steps (stage 1 + stage 2) of one universe in one launch
+// (grav_steps).
+//
+// Up to about ten thousand bodies a step is a few microseconds of arithmetic, and two
+// dependent launches per step (the persistent stage-1 grid, then stage 2 over its slots)
+// spend most of it on launch, drain and memory latency: 8.8 us per step at 64 bodies, 9.2 us
+// at 1000, 17.7 us at 4096 (fp32n, graph-replayed).  Here one grid of at most one CTA per SM
+// stays for all K steps: 2.1, 4.1 and 14.4 us per step of 20.  Each CTA keeps the FP64 state
+// of its R rows in registers and every body's FP32 position in shared memory; per step it
+// completes its rows' accelerations over all columns, integrates the rows and exchanges the
+// new positions with the other CTAs.  At 1000 bodies a step is ~0.9 us of pair work, ~0.8 us
+// of FP64 update (a chain of eleven FP64 instructions of 67 cycles each) and ~2 us of
+// exchange and waiting for the slowest CTA; from ~4000 bodies the pair loop is most of it.
+//
+// Exchange.  There is no grid barrier between steps.  A row's new position is published as
+// a 128-bit word (x, y, z, tag) by one relaxed 128-bit store and read by one relaxed
+// 128-bit load, which the memory model keeps whole; the tag is a step number that no
+// earlier step (or launch) used, so a reader that polls until the tag matches has the
+// position itself and needs no separate flag, fence or second round trip.  Two buffers
+// alternate: a CTA overwrites step k's positions when it publishes step k + 2, which it
+// does only after it has read every CTA's position of step k + 1, and a CTA publishes that
+// only after it is done with step k's.  One CTA alone exchanges through its own shared
+// memory.  The CTAs wait on one another, so they are co-scheduled: up to 16 as one
+// thread-block cluster (launched as a programmatic dependent), more as a cooperative
+// launch.  Every wait is bounded (GRAV_WAIT_NS); when one expires the CTA records
+// GRAV_DEV_TIMEOUT and leaves without writing the state.
+//
+// Pair loop.  A CTA's rows come in groups of 4 and the columns in blocks of 64; a unit is one
+// group against one block and the CTA's units are dealt evenly to its warps in order, so a
+// few rows keep every warp busy.  Lane 16 q + c of a warp takes rows 2 q and 2 q + 1 of the
+// group and the column pairs c and c + 16 of the block: the two columns of a pair are one
+// packed FP32 pair (x0, x1), read from shared memory in that layout, the rows duplicated
+// pairs.  12 packed FMA-pipe instructions and two reciprocal square roots per row and pair
+// (24 + 4 cycles), one 128-bit shared load; with one row per lane and two loads the loads'
+// return path was as long as the arithmetic.  Partials are FP32 over 16 blocks (32
+// terms per lane and column parity) and added into a second FP32 level; the warps' pieces of a row are added by
+// TwoSum (48 bits) in warp order: nothing depends on scheduling.
+#include "grav_device.cuh"
+
+namespace grav {
+
+enum { STEPS_DS = 0, STEPS_NEAR = 1 };
+constexpr int ST_T = 512;            // threads per CTA
+constexpr int ST_W = ST_T / 32;
+constexpr int ST_RG = 4;             // rows per group
+constexpr int ST_CB = 64;            // columns per block
+constexpr int ST_CHUNK = 16;          // blocks per first-level FP32 sum
+constexpr int ST_RPW = 10;           // rows whose state one warp holds (3 lanes each)
+constexpr int ST_MAX_ROWS = ST_RPW * ST_W;
+constexpr int ST_SMEM_MAX = 227 * 1024;
+constexpr unsigned ST_CLUSTER_MAX = 16;
+constexpr unsigned ST_CLUSTER_PORTABLE = 8;
+
+// Head of the scratch buffer; the two position buffers (hi, then lo, `rows` 16-byte words
+// each) follow at ST_HEAD_BYTES.
+struct StepsHead {
+	uint32_t epoch;     // tags used so far
+	int32_t departed;   // CTAs done with the launch
+};
+constexpr int ST_HEAD_BYTES = 128;
+
+typedef unsigned __int128 u128;
+
+__device__ __forceinline__ u128 load_word(const void* p)
+{
+	u128 v;
+	asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(v) : "l"(p) : "memory");
+	return v;
+}
+
+__device__ __forceinline__ void store_word(void* p, float x, float y, float z, uint32_t tag)
+{
+	const u64 lo = static_cast<u64>(__float_as_uint(y)) << 32 | __float_as_uint(x);
+	const u64 hi = static_cast<u64>(tag) << 32 | __float_as_uint(z);
+	const u128 v = static_cast<u128>(hi) << 64 | lo;
+	asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(v) : "memory");
+}
+
+__device__ __forceinline__ uint32_t word_tag(u128 v) { return static_cast<uint32_t>(v >> 96); }
+
+__device__ __forceinline__ float4 word_position(u128 v)
+{
+	return make_float4(__uint_as_float(static_cast<uint32_t>(v)),
+		__uint_as_float(static_cast<uint32_t>(v >> 32)),
+		__uint_as_float(static_cast<uint32_t>(v >> 64)), 0.f);
+}
+
+// Poll one published position until its tag is `tag`; false when the bounded wait expired.
+__device__ __forceinline__ bool wait_word(const void* p, uint32_t tag, u128& v)
+{
+	if (word_tag(v) == tag) return true;
+	const uint64_t t0 = global_ns();
+	for (;;) {
+		for (int k = 0; k < 64; ++k) {
+			v = load_word(p);
+			if (word_tag(v) == tag) return true;
+		}
+		if (global_ns() - t0 > GRAV_WAIT_NS) return false;
+	}
+}
+
+__device__ __forceinline__ void steps_cluster_arrive()
+{
+	asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void steps_cluster_wait()
+{
+	asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ unsigned steps_cluster_ctas()
+{
+	unsigned v;
+	asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(v));
+	return v;
+}
+
+// Shared memory of one CTA for n bodies and R rows per CTA (byte offsets, 16-byte units).
+struct StepsSmem {
+	int cols;     // [blocks][2][32] ulonglong2: (x0, x1 | y0, y1), (z0, z1 | Gm0, Gm1)
+	int colslo;   // the same for the low parts (DS, and NEAR where they fit: lo_here)
+	int rown;     // [rows][2] ulonglong2: (-x, -x | -y, -y), (-z, -z | near radius^2)
+	int rownlo;   // the same for the low parts (DS, NEAR)
+	int red;      // [groups + warps][ST_RG][3] float: the pieces' sums
+	int bytes;
+	bool lo_here;
+	__host__ __device__ StepsSmem(int kind, int n, int rows)
+	{
+		const int nb = (n + ST_CB - 1) / ST_CB;
+		const int ng = (rows + ST_RG - 1) / ST_RG;
+		const int r4 = ng * ST_RG;
+		const int tail = r4 * 64 + (ng + ST_W) * ST_RG * 3 * 4;
+		lo_here = kind == STEPS_DS || nb * 2048 + tail <= ST_SMEM_MAX;
+		cols = 0;
+		colslo = cols + nb * 1024;
+		rown = colslo + (lo_here ? nb * 1024 : 0);
+		rownlo = rown + r4 * 32;
+		red = rownlo + r4 * 32;
+		bytes = (red + (ng + ST_W) * ST_RG * 3 * 4 + 15) / 16 * 16;
+	}
+};
+
+// A row's duplicated, negated coordinates and, for its high parts, the near radius squared.
+__device__ __forceinline__ void set_row(ulonglong2* p, float x, float y, float z, float thr)
+{
+	p[0] = make_ulonglong2(pack2(-x, -x), pack2(-y, -y));
+	p[1] = make_ulonglong2(pack2(-z, -z), pack2(thr, 0.f));
+}
+
+// Two columns (2p, 2p + 1) of an expanded array; w given only where it is first written.
+__device__ __forceinline__ void set_pair(ulonglong2* cols, int p, const float4& a, const float4& c)
+{
+	ulonglong2* q = cols + (p >> 5) * 64 + (p & 31);
+	q[0] = make_ulonglong2(pack2(a.x, c.x), pack2(a.y, c.y));
+	*reinterpret_cast<u64*>(q + 32) = pack2(a.z, c.z);
+}
+
+// One coordinate set of column j (one CTA: its rows are all the columns).
+__device__ __forceinline__ void set_column(ulonglong2* cols, int j, float x, float y, float z)
+{
+	float* q = reinterpret_cast<float*>(cols + (j >> 6) * 64 + ((j >> 1) & 31)) + (j & 1);
+	q[0] = x;
+	q[2] = y;
+	q[32 * 4] = z;
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, const int flags,
+	const int K, const int64_t a_stride, const int R, unsigned char* __restrict__ scratch)
+{
+	constexpr bool DS = KIND == STEPS_DS;
+	constexpr bool NEAR = KIND == STEPS_NEAR;
+	extern __shared__ __align__(16) unsigned char steps_smem[];
+	const int tid = threadIdx.x;
+	const int lane = tid & 31;
+	const int warp = tid >> 5;
+	const int n = static_cast<int>(b.n_bodies);
+	const int G = gridDim.x;
+	const bool multi = G > 1;
+	const bool clustered = multi && steps_cluster_ctas() == static_cast<unsigned>(G);
+	const int row0 = blockIdx.x * R;
+	const int rows_here = max(0, min(R, n - row0));
+	const int NB = (n + ST_CB - 1) / ST_CB;
+	const int NG = (rows_here + ST_RG - 1) / ST_RG;
+	const float eps2 = b.eps2;
+	const u64 eps22 = pack2(eps2, eps2);
+	const bool integrate = (flags & GRAV_S2_INTEGRATE) != 0;
+
+	const StepsSmem L(KIND, n, R);
+	ulonglong2* const cols = reinterpret_cast<ulonglong2*>(steps_smem + L.cols);
+	ulonglong2* const colslo = reinterpret_cast<ulonglong2*>(steps_smem + L.colslo);
+	ulonglong2* const rown = reinterpret_cast<ulonglong2*>(steps_smem + L.rown);
+	ulonglong2* const rownlo = reinterpret_cast<ulonglong2*>(steps_smem + L.rownlo);
+	float* const red = reinterpret_cast<float*>(steps_smem + L.red);
+	const bool lo_here = L.lo_here;
+
+	StepsHead* const head = reinterpret_cast<StepsHead*>(scratch);
+	const int64_t words = static_cast<int64_t>(NB) * ST_CB;   // per array and buffer
+	float4* const xbuf = reinterpret_cast<float4*>(scratch + ST_HEAD_BYTES);  // [2][hi, lo][words]
+	const double Tu = b.univ[0].T;
+
+	// this warp's units [u0, u1) of the CTA's NG x NB
+	const int U = NG * NB;
+	const int Wn = max(1, min(ST_W, U));
+	const int u0 = warp < Wn ? warp * U / Wn : U, u1 = warp < Wn ? (warp + 1) * U / Wn : U;
+	const int g_first = u0 / NB;
+	const int cb_first = u0 - g_first * NB;
+	const int c16 = lane & 15;             // column lane; rows 2 (lane / 16) and the next one
+
+	// three lanes per row, ten rows per warp: lane 3 i + c owns component c of its row's r and
+	// v for the whole launch (FP64 instructions cost this GPU ~20 cycles per warp and SM
+	// whatever their active lanes, so the rows' components share them)
+	const int rl = warp * ST_RPW + lane / 3, rc = lane % 3;
+	const bool mine = lane < 3 * ST_RPW && rl < rows_here;
+	const bool warp_rows = warp * ST_RPW < rows_here;
+	const int grow = rl / ST_RG;   // this lane's row group; the warps that hold its pieces
+	int w_lo = 0, w_hi = -1;
+	if (mine) {
+		w_lo = ((grow * NB + 1) * Wn + U - 1) / U - 1;
+		w_hi = ((grow + 1) * NB * Wn + U - 1) / U - 1;
+	}
+
+	// everything below belongs to the kernels before this one
+	grid_dep_wait();
+	const uint32_t tag0 = multi ? head->epoch + 1 : 0;   // tag of the positions step 0 makes
+	double* const rd = b.r;
+	double* const vd = b.v;
+	const int64_t e = 4 * static_cast<int64_t>(row0 + rl) + rc;
+	double rr = 0.0, vv = 0.0;
+	const float4* __restrict__ pos = static_cast<const float4*>(b.pos);
+	const float4* __restrict__ poslo = pos + b.n_pad_total;
+	if (mine && integrate) {
+		rr = rd[e];
+		vv = vd[e];
+	}
+
+	// positions of every body; padding columns sit far away with Gm = 0: no contribution, and
+	// never near (the origin might be)
+	for (int p = tid; p < NB * 32; p += ST_T) {
+		const float4 far = make_float4(1e18f, 1e18f, 1e18f, 0.f), z = make_float4(0.f, 0.f, 0.f, 0.f);
+		const int j = 2 * p;
+		const float4 a = j < n ? pos[j] : far, c = j + 1 < n ? pos[j + 1] : far;
+		set_pair(cols, p, a, c);
+		(cols + (p >> 5) * 64 + (p & 31) + 32)->y = pack2(a.w, c.w);
+		if (lo_here) set_pair(colslo, p, j < n ? poslo[j] : z, j + 1 < n ? poslo[j + 1] : z);
+	}
+	// own rows, the last group padded with its last row (results unused)
+	for (int i = tid; i < NG * ST_RG; i += ST_T) {
+		const int64_t row = row0 + min(i, rows_here - 1);
+		const float4 p = pos[row];
+		set_row(rown + 2 * i, p.x, p.y, p.z, near_threshold(near_scale(p.x, p.y, p.z)));
+		const float4 q = poslo[row];
+		set_row(rownlo + 2 * i, q.x, q.y, q.z, 0.f);
+	}
+
+	const bool deferred = integrate && multi && !clustered && K == 1;
+	bool ok = true;
+	for (int k = 0; k < K; ++k) {
+		if (__syncthreads_or(!ok)) {
+			ok = false;
+			break;
+		}
+		// ---- the rows' accelerations: this warp's pieces ----
+		int u = u0, g = g_first, cb = cb_first;
+		while (u < u1) {
+			int left = min(NB - cb, u1 - u);   // blocks of this piece
+			u += left;
+			const ulonglong2* __restrict__ rp = rown + 2 * (g * ST_RG + (lane >> 4) * 2);
+			const ulonglong2* __restrict__ rlp = rownlo + 2 * (g * ST_RG + (lane >> 4) * 2);
+			u64 nx[2], ny[2], nz[2], lx[2], ly[2], lz[2];   // the rows; DS: their low parts
+			u64 sx[2], sy[2], sz[2];                        // second-level sums
+			// NEAR: r2 as an integer less eps2 + 1 is below `near_below` for near pairs; self
+			// pairs and coincident bodies (r2 = eps2) wrap to the largest integers
+			const uint32_t eps_bits = __float_as_uint(eps2) + 1u;
+			uint32_t near_below[2];
+			float thr[2];
+#pragma unroll
+			for (int r = 0; r < 2; ++r) {
+				const ulonglong2 xy = rp[2 * r], zt = rp[2 * r + 1];
+				nx[r] = xy.x;
+				ny[r] = xy.y;
+				nz[r] = zt.x;
+				if (DS) {
+					const ulonglong2 lxy = rlp[2 * r], lzz = rlp[2 * r + 1];
+					lx[r] = lxy.x;
+					ly[r] = lxy.y;
+					lz[r] = lzz.x;
+				}
+				if (NEAR) {
+					float unused;
+					unpack2(zt.y, thr[r], unused);
+					const uint32_t t = __float_as_uint(thr[r]);
+					near_below[r] = t > eps_bits ? t - eps_bits : 0u;
+				}
+				sx[r] = sy[r] = sz[r] = 0ull;
+			}
+			do {
+				const int m = min(ST_CHUNK, left);
+				const ulonglong2* __restrict__ cp = cols + cb * 64 + c16;
+				const ulonglong2* __restrict__ cl = colslo + cb * 64 + c16;
+				u64 fx[2], fy[2], fz[2];
+				uint32_t nmask = 0;   // NEAR: bit q of a block q that holds a near pair
+#pragma unroll
+				for (int r = 0; r < 2; ++r) fx[r] = fy[r] = fz[r] = 0ull;
+#pragma unroll 2
+				for (int q = 0; q < m; ++q, cp += 64, cl += 64) {
+					uint32_t rmin[2] = {0xffffffffu, 0xffffffffu};
+#pragma unroll
+					for (int i = 0; i < 2; ++i) {
+						const ulonglong2 cxy = cp[16 * i], czw = cp[16 * i + 32];
+						ulonglong2 dxy = make_ulonglong2(0ull, 0ull), dzz = dxy;
+						if (DS) {
+							dxy = cl[16 * i];
+							dzz = cl[16 * i + 32];
+						}
+#pragma unroll
+						for (int r = 0; r < 2; ++r) {
+							u64 dx = add2(cxy.x, nx[r]), dy = add2(cxy.y, ny[r]), dz = add2(czw.x, nz[r]);
+							if (DS) {
+								dx = add2(dx, add2(dxy.x, lx[r]));
+								dy = add2(dy, add2(dxy.y, ly[r]));
+								dz = add2(dz, add2(dzz.x, lz[r]));
+							}
+							float ra, rb;
+							unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
+							if (NEAR)
+								rmin[r] = min(__float_as_uint(ra) - eps_bits,
+									min(__float_as_uint(rb) - eps_bits, rmin[r]));
+							const u64 inv = pack2(rsqrt_sfu(ra), rsqrt_sfu(rb));
+							const u64 w = mul2(mul2(czw.y, inv), mul2(inv, inv));
+							fx[r] = fma2(dx, w, fx[r]);
+							fy[r] = fma2(dy, w, fy[r]);
+							fz[r] = fma2(dz, w, fz[r]);
+						}
+					}
+					if (NEAR && (rmin[0] < near_below[0] || rmin[1] < near_below[1])) nmask |= 1u << q;
+				}
+				if (NEAR) {
+					// cold path: the blocks that met a pair within the near radius, pair by pair
+					uint32_t todo = __reduce_or_sync(0xffffffffu, nmask);
+					while (todo) {
+						const int q = __ffs(todo) - 1;
+						todo &= todo - 1;
+#pragma unroll 1
+						for (int i = 0; i < 2; ++i) {
+							const int at = (cb + q) * 64 + 16 * i + c16;
+							const ulonglong2 cxy = cols[at], czw = cols[at + 32];
+							float4 l0, l1;
+							bool have = false;
+#pragma unroll
+							for (int r = 0; r < 2; ++r) {
+								const u64 dx = add2(cxy.x, nx[r]), dy = add2(cxy.y, ny[r]), dz = add2(czw.x, nz[r]);
+								float ra, rb;
+								unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
+								const bool na = (ra < thr[r]) & (ra > eps2), nb = (rb < thr[r]) & (rb > eps2);
+								if (!(na | nb)) continue;
+								if (!have) {   // the two columns' low parts
+									const int j = (cb + q) * ST_CB + 2 * (16 * i + c16), j1 = min(j + 1, n - 1);
+									have = true;
+									if (lo_here) {
+										const ulonglong2 dxy = colslo[at], dzz = colslo[at + 32];
+										unpack2(dxy.x, l0.x, l1.x);
+										unpack2(dxy.y, l0.y, l1.y);
+										unpack2(dzz.x, l0.z, l1.z);
+									} else if (k == 0) {
+										l0 = poslo[j];
+										l1 = poslo[j1];
+									} else {
+										const float4* glo = xbuf + (((k - 1) & 1) * 2 + 1) * words;
+										const uint32_t tag = tag0 + static_cast<uint32_t>(k) - 1;
+										u128 w0 = load_word(glo + j), w1 = load_word(glo + j1);
+										ok = wait_word(glo + j, tag, w0) && wait_word(glo + j1, tag, w1) && ok;
+										l0 = word_position(w0);
+										l1 = word_position(w1);
+									}
+								}
+								const ulonglong2 lxy = rlp[2 * r], lzz = rlp[2 * r + 1];
+								float4 li;
+								float x0, x1, y0, y1, z0, z1, ex0, ey0, ez0, ex1, ey1, ez1;
+								unpack2(lxy.x, li.x, x0);
+								unpack2(lxy.y, li.y, x0);
+								unpack2(lzz.x, li.z, x0);
+								li = make_float4(-li.x, -li.y, -li.z, 0.f);
+								unpack2(dx, x0, x1);
+								unpack2(dy, y0, y1);
+								unpack2(dz, z0, z1);
+								near_delta(x0, y0, z0, ra, l0, li, eps2, na, ex0, ey0, ez0);
+								near_delta(x1, y1, z1, rb, l1, li, eps2, nb, ex1, ey1, ez1);
+								fx[r] = fma2(pack2(ex0, ex1), czw.y, fx[r]);
+								fy[r] = fma2(pack2(ey0, ey1), czw.y, fy[r]);
+								fz[r] = fma2(pack2(ez0, ez1), czw.y, fz[r]);
+							}
+						}
+						__syncwarp();
+					}
+				}
+#pragma unroll
+				for (int r = 0; r < 2; ++r) {
+					sx[r] = add2(sx[r], fx[r]);
+					sy[r] = add2(sy[r], fy[r]);
+					sz[r] = add2(sz[r], fz[r]);
+				}
+				left -= m;
+				cb += m;
+			} while (left > 0);
+			// the rows' sums over their 16 lanes: after the first round lanes 8 q .. 8 q + 7 hold
+			// row q's three components
+			float v[2][3], t;
+#pragma unroll
+			for (int r = 0; r < 2; ++r) {
+				unpack2(sx[r], v[r][0], t);
+				v[r][0] += t;
+				unpack2(sy[r], v[r][1], t);
+				v[r][1] += t;
+				unpack2(sz[r], v[r][2], t);
+				v[r][2] += t;
+			}
+			const bool second = lane & 8;
+#pragma unroll
+			for (int i = 0; i < 3; ++i) {
+				const float give = second ? v[0][i] : v[1][i], keep = second ? v[1][i] : v[0][i];
+				v[0][i] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+			}
+#pragma unroll
+			for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+				for (int i = 0; i < 3; ++i) v[0][i] += __shfl_xor_sync(0xffffffffu, v[0][i], o);
+			// pieces in (warp, group) order take distinct slots warp + group
+			const int c8 = lane & 7;
+			if (c8 < 3)
+				red[(g + warp) * (ST_RG * 3) + (lane >> 3) * 3 + c8] =
+					c8 == 0 ? v[0][0] : (c8 == 1 ? v[0][1] : v[0][2]);
+			++g;
+			cb = 0;
+		}
+		const bool last = k + 1 == K;
+		if (last) {
+			if (__syncthreads_or(!ok)) {
+				ok = false;
+				break;
+			}
+		} else {
+			__syncthreads();
+		}
+
+		// a single-step launch writes the positions it read: in a cluster once every CTA is
+		// done with them, else the last CTA out copies them over (with more steps, each CTA has
+		// by now read every other CTA's later ones)
+		const bool settle = integrate && clustered && K == 1;
+		if (settle) steps_cluster_arrive();
+
+		// ---- stage 2 of this lane's row component ----
+		if (warp_rows) {
+			double a = 0.0;
+			if (mine) {
+				float h = 0.f, l = 0.f;
+				for (int w = w_lo; w <= w_hi; ++w)
+					two_sum_acc(h, l, red[(grow + w) * (ST_RG * 3) + (rl % ST_RG) * 3 + rc]);
+				a = static_cast<double>(h) + static_cast<double>(l);
+			}
+			if (integrate) {
+				// the base class's update with separately rounded products and sums
+				// (_base_.py:58-62, np2.py:110-115), as stage2.cu applies it
+				vv = __dadd_rn(__dmul_rn(a, Tu), vv);
+				rr = __dadd_rn(__dmul_rn(vv, Tu), rr);
+				const float hx = __double2float_rn(rr);
+				const float hy = __shfl_down_sync(0xffffffffu, hx, 1);
+				const float hz = __shfl_down_sync(0xffffffffu, hx, 2);
+				const bool lead = mine && rc == 0;
+				const bool publish = lead && multi && (!last || deferred);
+				if (publish) store_word(xbuf + (k & 1) * 2 * words + row0 + rl, hx, hy, hz, tag0 + k);
+				const float lx = __double2float_rn(__dsub_rn(rr, static_cast<double>(hx)));
+				const float ly = __shfl_down_sync(0xffffffffu, lx, 1);
+				const float lz = __shfl_down_sync(0xffffffffu, lx, 2);
+				if (publish)
+					store_word(xbuf + ((k & 1) * 2 + 1) * words + row0 + rl, lx, ly, lz, tag0 + k);
+				if (last) {
+					// ---- the launch's results: state and stage-1 positions ----
+					if (settle) steps_cluster_wait();
+					if (mine) {
+						rd[e] = rr;
+						vd[e] = vv;
+						if (!deferred) {
+							float* const q = reinterpret_cast<float*>(b.pos) + e;
+							*q = hx;
+							q[4 * b.n_pad_total] = lx;
+						}
+					}
+				} else if (lead) {
+					// own rows for the next step; the last row also stands in for the padding rows
+					const float thr = near_threshold(near_scale(hx, hy, hz));
+					const int i1 = rl == rows_here - 1 ? NG * ST_RG : rl + 1;
+					for (int i = rl; i < i1; ++i) {
+						set_row(rown + 2 * i, hx, hy, hz, thr);
+						set_row(rownlo + 2 * i, lx, ly, lz, 0.f);
+					}
+					if (!multi) {
+						set_column(cols, rl, hx, hy, hz);
+						if (lo_here) set_column(colslo, rl, lx, ly, lz);
+					}
+				}
+			}
+			if (mine && (flags & GRAV_S2_WRITE_A) && (last || a_stride)) {
+				double* const ao = b.a_out + k * a_stride + e;
+				__stcs(ao, a);
+				if (rc == 2) __stcs(ao + 1, 0.0);
+			}
+		} else if (settle) {
+			steps_cluster_wait();
+		}
+
+		// ---- every body's new position ----
+		if (multi && !last) {
+			const float4* __restrict__ src = xbuf + (k & 1) * 2 * words;
+			const uint32_t want = tag0 + k;
+			constexpr int IN_FLIGHT = 2;
+			for (int p0 = tid; 2 * p0 < n; p0 += IN_FLIGHT * ST_T) {
+				u128 w0[IN_FLIGHT], w1[IN_FLIGHT], l0[IN_FLIGHT], l1[IN_FLIGHT];
+#pragma unroll
+				for (int i = 0; i < IN_FLIGHT; ++i) {
+					const int j = 2 * (p0 + i * ST_T);
+					if (j >= n) continue;
+					const int j1 = min(j + 1, n - 1);
+					w0[i] = load_word(src + j);
+					w1[i] = load_word(src + j1);
+					if (lo_here) {
+						l0[i] = load_word(src + words + j);
+						l1[i] = load_word(src + words + j1);
+					}
+				}
+#pragma unroll
+				for (int i = 0; i < IN_FLIGHT; ++i) {
+					const int p = p0 + i * ST_T, j = 2 * p;
+					if (j >= n) continue;
+					const int j1 = min(j + 1, n - 1);
+					ok = ok && wait_word(src + j, want, w0[i]) && wait_word(src + j1, want, w1[i]);
+					float4 c = word_position(w1[i]);
+					if (j + 1 >= n) c = make_float4(1e18f, 1e18f, 1e18f, 0.f);
+					set_pair(cols, p, word_position(w0[i]), c);
+					if (lo_here) {
+						ok = ok && wait_word(src + words + j, want, l0[i]) &&
+							wait_word(src + words + j1, want, l1[i]);
+						float4 cl = word_position(l1[i]);
+						if (j + 1 >= n) cl = make_float4(0.f, 0.f, 0.f, 0.f);
+						set_pair(colslo, p, word_position(l0[i]), cl);
+					}
+				}
+			}
+		}
+	}
+
+	if (!ok) set_error(b.err, GRAV_DEV_TIMEOUT);
+	// the last CTA out hands the tags on for the next launch and, after a deferred single step,
+	// moves the new positions into the stage-1 array that every CTA has now read
+	if (multi) {
+		__shared__ int last_out;
+		__threadfence();
+		__syncthreads();
+		if (tid == 0) {
+			last_out = atomicAdd(&head->departed, 1) == G - 1;
+			__threadfence();
+		}
+		__syncthreads();
+		if (last_out) {
+			if (deferred) {
+				float* const q = reinterpret_cast<float*>(b.pos);
+				constexpr int IN_FLIGHT = 4;
+				for (int j0 = tid; j0 < n; j0 += IN_FLIGHT * ST_T) {
+					u128 h[IN_FLIGHT], l[IN_FLIGHT];
+#pragma unroll
+					for (int i = 0; i < IN_FLIGHT; ++i) {
+						const int j = min(j0 + i * ST_T, n - 1);
+						h[i] = load_word(xbuf + j);
+						l[i] = load_word(xbuf + words + j);
+					}
+#pragma unroll
+					for (int i = 0; i < IN_FLIGHT; ++i) {
+						const int j = j0 + i * ST_T;
+						if (j >= n) continue;
+						const float4 p = word_position(h[i]);
+						*reinterpret_cast<float2*>(q + 4 * j) = make_float2(p.x, p.y);
+						q[4 * j + 2] = p.z;
+						reinterpret_cast<float4*>(q)[b.n_pad_total + j] = word_position(l[i]);
+					}
+				}
+			}
+			if (tid == 0) {
+				head->departed = 0;
+				head->epoch = tag0 - 1 + static_cast<uint32_t>(K);
+			}
+		}
+	}
+	grid_dep_launch();
+}
+
+namespace {
+
+int steps_kind(int mode)
+{
+	switch (mode) {
+	case GRAV_MODE_FP32C: case GRAV_MODE_FP32CU: return STEPS_DS;
+	case GRAV_MODE_FP32N: case GRAV_MODE_FP32UN: return STEPS_NEAR;
+	default: return -1;
+	}
+}
+
+const void* steps_fn(int kind)
+{
+	return kind == STEPS_DS ? reinterpret_cast<const void*>(&steps_kernel<STEPS_DS>)
+	                        : reinterpret_cast<const void*>(&steps_kernel<STEPS_NEAR>);
+}
+
+}  // namespace
+
+// Rows per CTA: up to 64 bodies one CTA; up to 512 at most 16 CTAs (one cluster); above, one
+// CTA per SM, whole groups of 4 rows.
+int steps_rows(int n, int sms)
+{
+	if (n <= 64) return 64;
+	const int ctas = n <= 512 ? static_cast<int>(ST_CLUSTER_MAX) : sms;
+	return (n + ST_RG * ctas - 1) / (ST_RG * ctas) * ST_RG;
+}
+
+// Whether grav_steps can take n bodies of `mode` on a GPU of `sms` SMs: the positions and a
+// CTA's rows fit its shared memory, and a CTA's rows its threads.
+bool steps_supported(int mode, int n, int sms)
+{
+	const int kind = steps_kind(mode);
+	if (kind < 0 || n < 1 || sms < 1 || n > ST_MAX_ROWS * sms) return false;
+	const int R = steps_rows(n, sms);
+	return R <= ST_MAX_ROWS && StepsSmem(kind, n, R).bytes <= ST_SMEM_MAX;
+}
+
+int64_t steps_scratch(int n)
+{
+	const int64_t words = (static_cast<int64_t>(n) + ST_CB - 1) / ST_CB * ST_CB;
+	return ST_HEAD_BYTES + 4 * words * 16;
+}
+
+cudaError_t launch_steps(const grav_batch& b, int flags, int steps, int64_t a_stride, void* scratch,
+	int sms, cudaStream_t stream)
+{
+	const int n = static_cast<int>(b.n_bodies);
+	const int kind = steps_kind(b.mode);
+	const void* fn = steps_fn(kind);
+	int R = steps_rows(n, sms);
+	const int smem = StepsSmem(kind, n, R).bytes;
+	cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+	if (e != cudaSuccess) return e;
+	const unsigned grid = static_cast<unsigned>((n + R - 1) / R);
+	grav_batch copy = b;
+	int f = flags, K = steps;
+	unsigned char* s = static_cast<unsigned char*>(scratch);
+	void* args[] = {&copy, &f, &K, &a_stride, &R, &s};
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(grid);
+	cfg.blockDim = dim3(ST_T);
+	cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+	cfg.stream = stream;
+	cudaLaunchAttribute attr[2];
+	cfg.attrs = attr;
+	cfg.numAttrs = 0;
+	const bool integrate = grid > 1 && (flags & GRAV_S2_INTEGRATE);
+	const bool waits = integrate && steps > 1;
+	bool cluster = integrate && grid <= ST_CLUSTER_MAX;
+	if (cluster) {
+		attr[0].id = cudaLaunchAttributeClusterDimension;
+		attr[0].val.clusterDim.x = grid;
+		attr[0].val.clusterDim.y = 1;
+		attr[0].val.clusterDim.z = 1;
+		cfg.numAttrs = 1;
+		if (grid > ST_CLUSTER_PORTABLE) {
+			int fits = 0;
+			e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+			if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fits, fn, &cfg);
+			if (e != cudaSuccess) {
+				cudaGetLastError();  // a refused query is not sticky: fall back
+				fits = 0;
+			}
+			cluster = fits > 0;
+			if (!cluster) cfg.numAttrs = 0;
+		}
+	}
+	if (waits && !cluster) {
+		attr[0].id = cudaLaunchAttributeCooperative;
+		attr[0].val.cooperative = 1;
+		cfg.numAttrs = 1;
+	} else {
+		attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+		attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+		++cfg.numAttrs;
+	}
+	return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
+}  // namespace grav

@@ -216,6 +216,29 @@ def default_fused(mode, sizes, dev_info=None):
     return None
 
 
+# Largest universe whose queued steps (and accelerations alone) run as one launch
+# (grav_steps), and up to which a single queued step does.  Measured on GB300, us per step of
+# 20 queued / accelerations alone / one step, in brackets the two-launch step:
+#   fp32n   64: 2.1 / 3.0 / 3.5 [8.6]   1000: 4.2 / 6.1 / 7.6 [9.2]   2048: 6.9 / 8.8 / 10 [10]
+#           4096: 13.9 / 17.2 / 20 [17.7]   8192: 41 / 43 / 48 [57]   12000: 82 / 83 / 90 [105]
+#   fp32c   1000: 3.7 / 5.5 / 7.1 [11.1]   4096: 15.0 / 17 / 20 [19.3]   6000: 27 / 29 / 34 [37]
+# The unique-pair modes' own kernels pass it between 6144 and 8192 bodies (fp32un 27 us
+# against 31 at 6144, 41 against 37 at 8192).  The plain modes, whose error is the rounding
+# of the positions, keep their own kernels and their sums bit for bit.  After a single step
+# the last CTA moves the positions over, which from ~2500 bodies on costs what the second
+# launch does.
+STEPS_MAX_N = {'fp32n': 12288, 'fp32c': 6144, 'fp32un': 6144, 'fp32cu': 6144}
+STEPS_SINGLE_MAX_N = 2048
+
+
+def default_steps(mode, sizes, dev_info):
+    """True when the queued steps of this workload run as one launch (grav_steps): one
+    universe within the measured size rule that the kernel takes on this GPU."""
+    if len(sizes) != 1 or not 0 < sizes[0] <= STEPS_MAX_N.get(mode, 0):
+        return False
+    return bool(_lib.load().grav_steps_supported(_lib.MODES[mode], sizes[0], dev_info.sm_count))
+
+
 class Engine:
     """Packed batch of universes on one GB300 with FP64 state.
 
@@ -228,7 +251,7 @@ class Engine:
       tile  : _lib.Tile, or None to use the autotuner's choice / the default shape
       fused : single-launch step (grav_step_fused) for one small universe: (threads,
               rows) per CTA, False for the two-launch step, None to decide by size
-              (default_fused)
+              (default_fused, and default_steps: all queued steps in one launch)
     """
 
     def __init__(self, sizes, T, mode='fp32', tile=None, device=None, tuner=None, fused=None):
@@ -244,10 +267,13 @@ class Engine:
             self.mode_name = {v: k for k, v in _lib.MODES.items()}[self.mode]
         self.sizes = [int(x) for x in sizes]
         self.T = list(T) if np.ndim(T) else [float(T)] * len(self.sizes)
+        # queued steps in one launch, unless the caller picks the kernels himself
+        self.chained = (fused is None and tile is None
+                        and default_steps(self.mode_name, self.sizes, self.dev_info))
         if fused is None:
             fused = default_fused(self.mode_name, self.sizes, self.dev_info)
         if tile is None:
-            if tuner is not None and not fused:
+            if tuner is not None and not fused and not self.chained:
                 tile = tuner.choose(self.mode_name, self.sizes, self.dev_info, T=self.T)
             else:
                 tile = default_tile(self.mode_name, self.sizes, self.dev_info.index)
@@ -310,6 +336,11 @@ class Engine:
             self.fused = (threads, rows)
             # grid-barrier counters of grav_step_fused (zero between calls)
             self.sync = torch.zeros(2, dtype=torch.int32, device=dev)
+        self.scratch = None
+        if self.chained:
+            # exchange buffers of grav_steps (zeroed once, then its own)
+            nbytes = int(self.lib.grav_steps_scratch_bytes(self.sizes[0]))
+            self.scratch = torch.zeros(nbytes, dtype=torch.uint8, device=dev)
 
     # ---- state ----------------------------------------------------------------------
     def set_state(self, r, v, gm, stream=None):
@@ -394,10 +425,13 @@ class Engine:
         check(self.lib.grav_stage2(self._bref, int(flags), self._h(stream)))
 
     def step(self, steps=1, stream=None, write_a=False):
-        """`steps` full steps (stage 1 + stage 2, or the single-launch step) queued on the
-        stream."""
+        """`steps` full steps (stage 1 + stage 2, the single-launch step, or all of them in
+        one launch) queued on the stream."""
         flags = _lib.GRAV_S2_INTEGRATE | (_lib.GRAV_S2_WRITE_A if write_a else 0)
         h = self._h(stream)
+        if self.chained and (int(steps) > 1 or self.sizes[0] <= STEPS_SINGLE_MAX_N):
+            self._steps(flags, int(steps), 0, h)
+            return
         if self.fused:
             threads, rows = self.fused
             sync = ctypes.c_void_p(self.sync.data_ptr())
@@ -407,9 +441,30 @@ class Engine:
         for _ in range(int(steps)):
             check(self.lib.grav_step(self._bref, flags, h))
 
+    def _steps(self, flags, steps, a_stride, h):
+        check(self.lib.grav_steps(self._bref, flags, steps, a_stride,
+                                  ctypes.c_void_p(self.scratch.data_ptr()), h))
+
+    def steps_to(self, a, stream=None):
+        """len(a) full steps, step k's accelerations written to a[k] (float64
+        [steps, n_bodies, 4], device)."""
+        flags = _lib.GRAV_S2_INTEGRATE | _lib.GRAV_S2_WRITE_A
+        h = self._h(stream)
+        keep = self.batch.a_out
+        try:
+            if self.chained:
+                self.batch.a_out = a.data_ptr()
+                self._steps(flags, len(a), a.stride(0), h)
+                return
+            for k in range(len(a)):
+                self.batch.a_out = a[k].data_ptr()
+                check(self.lib.grav_step(self._bref, flags, h))
+        finally:
+            self.batch.a_out = keep
+
     def capture_graph(self, steps=1):
-        """CUDA graph of `steps` full steps (the steady-state step: stage 1 + stage 2,
-        2 launches per step); returns a torch.cuda.CUDAGraph whose replay() runs them.
+        """CUDA graph of `steps` full steps (one launch, or stage 1 + stage 2: 2 launches
+        per step); returns a torch.cuda.CUDAGraph whose replay() runs them.
         The launches are recorded on a side stream that torch puts into capture mode."""
         side = torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream(self.device))
@@ -421,6 +476,9 @@ class Engine:
 
     def forces(self, stream=None):
         """Stage 1 only; returns the accelerations (float64 [n_bodies, 3], device)."""
+        if self.chained:
+            self._steps(_lib.GRAV_S2_WRITE_A, 1, 0, self._h(stream))
+            return self.a[:self.info.n_bodies, :3]
         self.stage1(stream)
         self.stage2(_lib.GRAV_S2_WRITE_A, stream)
         return self.a[:self.info.n_bodies, :3]

@@ -188,7 +188,9 @@ class GB300Stages:
         device = meta.get('device')
 
         def make_engine(m):
-            return Engine([n], float(self._T), mode=m, tile=tile, device=device, tuner=tuner)
+            # the unfused stages take the two-launch kernels
+            return Engine([n], float(self._T), mode=m, tile=tile, device=device, tuner=tuner,
+                          fused=None if self._gb_fuse else False)
         self._gb = make_engine(mode)
         dev = self._gb.device
         # pinned FP64 host mirror (x, y, z, G*m) / (vx, vy, vz, 0) / (ax, ay, az, 0)
@@ -275,9 +277,13 @@ class GB300Stages:
             with torch.cuda.stream(s):
                 g.r.copy_(self._gb_hr, non_blocking=True)
             g.prepare(stream=s)
-            g.stage1(stream=s)
-            s.wait_stream(side)
-            g.stage2(_lib.GRAV_S2_INTEGRATE, stream=s)
+            if g.chained or g.fused:
+                s.wait_stream(side)
+                g.step(1, stream=s)
+            else:
+                g.stage1(stream=s)
+                s.wait_stream(side)
+                g.stage2(_lib.GRAV_S2_INTEGRATE, stream=s)
         else:
             g.step(1, stream=s)
         self._gb_enqueue_download(state=self._gb_sync in ('full', 'pull'))

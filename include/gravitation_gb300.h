@@ -32,7 +32,7 @@
 extern "C" {
 #endif
 
-#define GRAV_ABI_VERSION 5
+#define GRAV_ABI_VERSION 6
 
 /* status codes */
 #define GRAV_OK 0
@@ -258,6 +258,34 @@ int grav_fused_occupancy(int mode, int32_t n, int32_t threads, int32_t rows,
  */
 int grav_step_fused(const grav_batch* b, int flags, int32_t threads, int32_t rows,
 	int32_t* sync, void* stream);
+
+/* ---- many steps of one universe in one launch ------------------------------------ */
+
+/* 1 if grav_steps takes one universe of n bodies in `mode` (the FP32 modes that keep the low
+ * parts of the positions, laid out by grav_plan or grav_plan_pairs) on a GPU of sm_count
+ * SMs, else 0: every CTA holds all positions in shared memory (up to ~12.9k bodies, ~6.5k
+ * with double-single separations for every pair). */
+int grav_steps_supported(int mode, int32_t n, int32_t sm_count);
+
+/* Bytes of device scratch grav_steps needs for n bodies: zeroed once by the caller, then
+ * left alone between calls (it numbers the exchanged positions). */
+int64_t grav_steps_scratch_bytes(int32_t n);
+
+/*
+ * `steps` full steps (GRAV_S2_INTEGRATE) of a batch holding one universe in one launch, or
+ * its accelerations alone (GRAV_S2_WRITE_A without GRAV_S2_INTEGRATE, steps = 1).  The pair
+ * arithmetic, near correction and FP64 update are those of grav_stage1 + grav_stage2 (the
+ * unique-pair modes visit ordered pairs here), summed in another order: results agree to
+ * FP32 rounding of the partial sums.  With GRAV_S2_WRITE_A step k writes its accelerations
+ * to a_out + k * a_stride (doubles); a_stride = 0 keeps the last step's only.  r, v and the
+ * stage-1 positions are read at the start and written at the end of the launch.  At most one
+ * CTA per SM; CTAs that wait on one another are one thread-block cluster or a cooperative
+ * launch, and every wait is bounded: after 2 s it sets GRAV_DEV_TIMEOUT in b->err and the
+ * state is left as it was.  b->part is not used.  Replaces the loop of a caller over
+ * universe_base.step's stage 1 and stage 2 calls (_base_.py:143-144).
+ */
+int grav_steps(const grav_batch* b, int flags, int32_t steps, int64_t a_stride, void* scratch,
+	void* stream);
 
 /* ---- diagnostics -------------------------------------------------------------------- */
 

@@ -396,3 +396,39 @@ def test_single_launch_rule_names_compiled_kernels(L):
         assert default_fused(mode, [100, 100]) is None
     for mode in ('fp32u', 'fp32un', 'fp32cu', 'fp64'):
         assert default_fused(mode, [100]) is None
+
+
+def test_steps_rejects_bad_calls_on_host(L):
+    """grav_steps validates on the host, and the engine's rule names sizes it takes."""
+    from gravitation_gb300.engine import STEPS_MAX_N, STEPS_SINGLE_MAX_N
+    for mode, n_max in STEPS_MAX_N.items():
+        m = _lib.MODES[mode]
+        for n in (1, 64, 65, 512, 513, 1000, STEPS_SINGLE_MAX_N, n_max):
+            assert L.grav_steps_supported(m, n, 152) == 1, (mode, n)
+        assert L.grav_steps_supported(m, 0, 152) == 0
+        assert L.grav_steps_supported(m, 1 << 20, 152) == 0
+        assert L.grav_steps_supported(m, 100, 0) == 0
+    for m in (_lib.GRAV_MODE_FP64, _lib.GRAV_MODE_FP32, _lib.GRAV_MODE_FP32U):
+        assert L.grav_steps_supported(m, 100, 152) == 0
+    assert L.grav_steps_supported(99, 100, 152) == 0
+    assert L.grav_steps_scratch_bytes(1000) >= 4 * 16 * 1000
+    assert L.grav_steps_scratch_bytes(-1) < 0
+    scratch = ctypes.c_void_p(16)   # never dereferenced: validation fails first
+    assert L.grav_steps(None, 1, 1, 0, scratch, None) == _lib.GRAV_E_ARG
+    b = _lib.Batch()
+    b.mode = _lib.GRAV_MODE_FP32N
+    b.tile = _lib.Tile(1, 128, 128, 1)
+    b.n_seg, b.n_pad_total, b.n_bodies, b.n_univ = 1, 128, 100, 1
+    b.univ = b.seg = b.pos = b.r = b.v = b.err = 16
+    b.eps2 = 1e-25
+    bb = ctypes.byref(b)
+    assert L.grav_steps(bb, 1, 1, 0, None, None) == _lib.GRAV_E_ARG           # no scratch
+    assert L.grav_steps(bb, 1, -1, 0, scratch, None) == _lib.GRAV_E_ARG       # steps < 0
+    assert L.grav_steps(bb, _lib.GRAV_S2_PREPARE, 1, 0, scratch, None) == _lib.GRAV_E_ARG
+    assert L.grav_steps(bb, _lib.GRAV_S2_WRITE_A, 1, 0, scratch, None) == _lib.GRAV_E_ARG
+    assert L.grav_steps(bb, 1, 2, -4, scratch, None) == _lib.GRAV_E_ARG       # a_stride < 0
+    b.a_out = 16
+    assert L.grav_steps(bb, _lib.GRAV_S2_WRITE_A, 2, 0, scratch, None) == _lib.GRAV_E_ARG
+    assert L.grav_steps(bb, 1, 0, 0, scratch, None) == _lib.GRAV_OK           # no steps
+    b.n_univ = 2
+    assert L.grav_steps(bb, 1, 1, 0, scratch, None) == _lib.GRAV_E_ARG

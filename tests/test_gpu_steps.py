@@ -1,0 +1,132 @@
+"""GPU tests of many steps of one universe in one launch (grav_steps, steps.cu): one CTA (up
+to 64 bodies), one cluster (up to 512) and one CTA per SM, at the edges of its row groups,
+column blocks and grids.
+
+  - the accelerations of every step against the FP64 oracle on that step's own state,
+    per body |a - a_ref| <= 1e-5 sum_j |a_ij| (a pair term carries ~1.5e-6 of FP32 rounding
+    and, near-corrected, up to 4.5e-6 from positions beyond the near radius; FP32 partial sums
+    of at most 32 terms add less than 1e-6), with pairs 1e-3 apart at |x| ~ 1000 planted;
+  - each FP64 update bit for bit from those accelerations (_base_.py:58-62), the stage-1
+    positions bit for bit what grav_prepare makes of the final state;
+  - K steps in one launch, in several launches, one by one and from a graph: the same bits.
+"""
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from gravitation_gb300.engine import Engine, STEPS_SINGLE_MAX_N
+from gravitation_gb300.scenarios import G_DEFAULT, uniform_cube
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+SIZES = [1, 2, 4, 5, 63, 64, 65, 67, 128, 511, 512, 513, 641, 1000, 1217, 2560]
+MODES = ['fp32n', 'fp32c']
+
+
+def planted(n, seed):
+    r, v, m = uniform_cube(n, seed=seed)
+    rng = np.random.default_rng(seed + 1)
+    for i, j in ((3, 9), (17, n - 2), (n // 3, n // 2)):
+        if 0 <= i < j < n:
+            r[i] = np.sign(r[i]) * 990.0 + rng.uniform(-5, 5, 3)
+            r[j] = r[i] + rng.uniform(-1e-3, 1e-3, 3)
+    return r, v, m
+
+
+def magnitudes(r, gm):
+    out = np.zeros(len(gm))
+    for i in range(0, len(gm), 256):
+        d2 = ((r[None, :, :] - r[i:i + 256, None, :]) ** 2).sum(-1)
+        with np.errstate(divide='ignore'):
+            out[i:i + 256] = np.where(d2 > 0, gm[None, :] / d2, 0.0).sum(1)
+    return out
+
+
+def check_steps(mode, n, steps, T=1.0):
+    r, v, m = planted(n, 40 + n)
+    gm = G_DEFAULT * m
+    eng = Engine([n], T, mode=mode)
+    assert eng.chained
+    eng.set_state(r, v, gm)
+    acc = torch.full((steps, n, 4), 7.0, dtype=torch.float64, device=eng.device)
+    eng.steps_to(acc)
+    torch.cuda.synchronize()
+    eng.raise_on_device_error()
+    acc = acc.cpu().numpy()
+    assert np.all(acc[:, :, 3] == 0.0)
+    for k in range(steps):
+        a = acc[k, :, :3]
+        ref = oracle.accel_fp64(r, gm, 1.0, coincident=True)
+        err = np.linalg.norm(a - ref, axis=1)
+        scale = magnitudes(r, gm)
+        assert np.all(err <= TOL * scale), (mode, n, k, np.max(err / np.maximum(scale, 1e-300)))
+        r, v = oracle.stage2_fp64(r, v, a, T)
+    assert np.array_equal(eng.r[:n, :3].cpu().numpy(), r)
+    assert np.array_equal(eng.v[:n, :3].cpu().numpy(), v)
+    assert np.array_equal(eng.r[:n, 3].cpu().numpy(), gm)
+    pos = eng.pos.clone()
+    eng.prepare()
+    torch.cuda.synchronize()
+    assert torch.equal(pos, eng.pos)
+
+
+@pytest.mark.parametrize('mode', MODES)
+@pytest.mark.parametrize('n', SIZES)
+def test_steps_against_oracle(gpu, mode, n):
+    check_steps(mode, n, 3)
+
+
+@pytest.mark.parametrize('mode,n', [('fp32n', 8200), ('fp32n', 6000), ('fp32n', 7500),
+                                    ('fp32n', 12288), ('fp32c', 6144), ('fp32un', 5000),
+                                    ('fp32cu', 4999)])
+def test_steps_large(gpu, mode, n):
+    """Near the largest sizes: with and without the low parts in shared memory."""
+    check_steps(mode, n, 2)
+
+
+@pytest.mark.parametrize('mode', MODES)
+@pytest.mark.parametrize('n', [1, 64, 100, 512, 515, 2000])
+def test_steps_split_and_replayed(gpu, mode, n):
+    assert n <= STEPS_SINGLE_MAX_N
+    r, v, m = planted(n, 8)
+    gm = G_DEFAULT * m
+    engines = [Engine([n], 1e3, mode=mode) for _ in range(5)]
+    for e in engines:
+        e.set_state(r, v, gm)
+    engines[0].step(6)
+    engines[1].step(2)
+    engines[1].step(4)
+    for _ in range(6):
+        engines[2].step(1)
+    g = engines[3].capture_graph(3)
+    g.replay()
+    g.replay()
+    engines[4].step(1)
+    engines[4].forces()
+    engines[4].step(5, write_a=True)
+    torch.cuda.synchronize()
+    for e in engines:
+        e.raise_on_device_error()
+        assert torch.equal(engines[0].r, e.r) and torch.equal(engines[0].v, e.v)
+        assert torch.equal(engines[0].pos, e.pos)
+
+
+@pytest.mark.parametrize('mode', MODES)
+@pytest.mark.parametrize('n', [50, 300, 1500])
+def test_forces_leave_the_state(gpu, mode, n):
+    r, v, m = planted(n, 5)
+    eng = Engine([n], 1e3, mode=mode)
+    eng.set_state(r, v, G_DEFAULT * m)
+    before = [x.clone() for x in (eng.r, eng.v, eng.pos)]
+    a = eng.forces().clone()
+    two = Engine([n], 1e3, mode=mode, fused=False)
+    assert not two.chained
+    two.set_state(r, v, G_DEFAULT * m)
+    b = two.forces().clone()
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, y) for x, y in zip(before, (eng.r, eng.v, eng.pos)))
+    scale = torch.tensor(magnitudes(r, G_DEFAULT * m), device=a.device)
+    assert float(((a - b).norm(dim=1) / scale).max()) < 2e-5
