@@ -32,12 +32,14 @@ GRAV_S2_PREPARE = 4
 GRAV_MODE_FP32CU = 4
 GRAV_MODE_FP32N = 5
 GRAV_MODE_FP32UN = 6
+GRAV_MODE_FP64U = 8
 GRAV_NEAR_KAPPA = 20
 GRAV_FUSED_MAX_N = 4096
 MODES = {'fp32': GRAV_MODE_FP32, 'fp32c': GRAV_MODE_FP32C, 'fp64': GRAV_MODE_FP64,
          'fp32u': GRAV_MODE_FP32U, 'fp32cu': GRAV_MODE_FP32CU, 'fp32n': GRAV_MODE_FP32N,
          'fp32un': GRAV_MODE_FP32UN}
-PAIR_MODES = ('fp32u', 'fp32cu', 'fp32un', GRAV_MODE_FP32U, GRAV_MODE_FP32CU, GRAV_MODE_FP32UN)
+PAIR_MODES = ('fp32u', 'fp32cu', 'fp32un', GRAV_MODE_FP32U, GRAV_MODE_FP32CU, GRAV_MODE_FP32UN,
+              GRAV_MODE_FP64U)
 
 
 class GravError(RuntimeError):

@@ -43,7 +43,7 @@ int cuda_fail(cudaError_t e, const char* what)
 
 int stage1_table_for(int mode, const grav::Stage1Kernel** tab)
 {
-	if (mode == GRAV_MODE_FP64) return grav::stage1_table_f64(tab);
+	if (grav::fp64_mode(mode)) return grav::stage1_table_f64(tab);
 	if (mode == GRAV_MODE_FP32U || mode == GRAV_MODE_FP32CU || mode == GRAV_MODE_FP32UN)
 		return grav::stage1_table_sym(tab);
 	return grav::stage1_table_f32(tab);
@@ -79,7 +79,7 @@ cudaError_t ensure_smem(const grav::Stage1Kernel* k)
 
 bool valid_mode(int mode)
 {
-	return mode == GRAV_MODE_FP32 || mode == GRAV_MODE_FP32C || mode == GRAV_MODE_FP64 ||
+	return mode == GRAV_MODE_FP32 || mode == GRAV_MODE_FP32C || grav::fp64_mode(mode) ||
 		mode == GRAV_MODE_FP32U || mode == GRAV_MODE_FP32CU || mode == GRAV_MODE_FP32N ||
 		mode == GRAV_MODE_FP32UN;
 }
@@ -101,7 +101,7 @@ int check_batch(const grav_batch* b)
 		return fail(GRAV_E_ARG, "NULL device pointer in grav_batch (univ/seg/pos/r)");
 	if (b->n_pad_total > 0 && b->n_univ <= 0)
 		return fail(GRAV_E_ARG, "rows without universes");
-	if (!(b->eps2 > 0.f) && b->mode != GRAV_MODE_FP64)
+	if (!(b->eps2 > 0.f) && !grav::fp64_mode(b->mode))
 		return fail(GRAV_E_ARG, "eps2 must be > 0 in the FP32 modes (see grav_eps2)");
 	return ok();
 }
@@ -173,7 +173,7 @@ int grav_occupancy(int mode, const grav_tile* tile, int32_t* ctas_per_sm)
 	cudaError_t e = ensure_smem(k);
 	if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute (dynamic shared memory)");
 	int blocks = 0;
-	e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k->fn, k->threads, k->smem_bytes);
+	e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k->fn, k->cta_threads(), k->smem_bytes);
 	if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
 	*ctas_per_sm = blocks;
 	return ok();
@@ -337,7 +337,7 @@ int grav_plan_pairs(int32_t n_univ, const int32_t* n, const double* T, const gra
 int64_t grav_pos_bytes(int mode, int64_t n_pad_total)
 {
 	if (!valid_mode(mode) || n_pad_total < 0) return fail(GRAV_E_ARG, "bad mode or size");
-	if (mode == GRAV_MODE_FP64) return n_pad_total * 32;
+	if (grav::fp64_mode(mode)) return n_pad_total * 32;
 	if (mode == GRAV_MODE_FP32C || mode == GRAV_MODE_FP32CU || mode == GRAV_MODE_FP32N ||
 		mode == GRAV_MODE_FP32UN)
 		return n_pad_total * 32;
@@ -388,8 +388,8 @@ int grav_stage1(const grav_batch* b, void* stream)
 	void* args[] = {&copy};
 	cudaStream_t st = static_cast<cudaStream_t>(stream);
 	e = k->dependent
-		? grav::launch_dependent(k->fn, b->tile.grid, b->tile.threads, k->smem_bytes, st, args)
-		: cudaLaunchKernel(k->fn, dim3(b->tile.grid), dim3(b->tile.threads), args, k->smem_bytes, st);
+		? grav::launch_dependent(k->fn, b->tile.grid, k->cta_threads(), k->smem_bytes, st, args)
+		: cudaLaunchKernel(k->fn, dim3(b->tile.grid), dim3(k->cta_threads()), args, k->smem_bytes, st);
 	if (e != cudaSuccess) return cuda_fail(e, "stage-1 kernel launch");
 	return ok();
 }

@@ -47,7 +47,7 @@ struct PotentialOp {
 			for (int k = 0; k < B; ++k) {
 				const double dx = pj.x - xi[k], dy = pj.y - yi[k], dz = pj.z - zi[k];
 				const double r2 = dx * dx + dy * dy + dz * dz;
-				phi[k] += (r2 > 0.0) ? pj.w * rsqrt(r2) : 0.0;
+				phi[k] += pj.w * inv_root(r2);
 			}
 		}
 	}

@@ -162,6 +162,47 @@ __device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float x)
 	lo += e;
 }
 
+// r2^(-3/2) in FP64 without the library's reciprocal square root, for exponents of r2 in
+// 2^-598 .. 2^1023 (else `in_range` is false and the result 0).  y, the SFU's approximation of
+// r2^(-1/2) (rsqrt.approx.ftz.f64, computed from the high word, its low word zero), leaves e =
+// 1 - r2 y^2 below 2^-19, formed with one rounding of its own size; r2^(-3/2) = y^3 (1 -
+// e)^(-3/2) = y^3 (1 + 3/2 e + 15/8 e^2 + O(2^-56)), the binomial series: six FP64
+// instructions, no branch.
+__device__ __forceinline__ double inv_cube(double r2, bool& in_range)
+{
+	in_range = static_cast<uint32_t>(__double2hiint(r2)) - 0x1a900000u < 0x65500000u;
+	double y;
+	asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+	const double t = y * y;
+	const double e = fma(-r2, t, 1.0);
+	const double y3 = y * t;
+	const double f = fma(y3 * e, fma(1.875, e, 1.5), y3);
+	// selected as words: a floating-point select would be an FP64 instruction
+	return __hiloint2double(in_range ? __double2hiint(f) : 0, in_range ? __double2loint(f) : 0);
+}
+
+// The same for any r2 >= 0 (0 at 0): outside the range by the library's function.
+__device__ __forceinline__ double inv_cube(double r2)
+{
+	bool in_range;
+	const double f = inv_cube(r2, in_range);
+	if (in_range) return f;
+	const double inv = r2 > 0.0 ? rsqrt(r2) : 0.0;
+	return inv * inv * inv;
+}
+
+// r2^(-1/2), 0 at r2 = 0, by the same series: y (1 + 1/2 e + 3/8 e^2); five FP64 instructions.
+__device__ __forceinline__ double inv_root(double r2)
+{
+	if (static_cast<uint32_t>(__double2hiint(r2)) - 0x1a900000u < 0x65500000u) {
+		double y;
+		asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+		const double e = fma(-r2, y * y, 1.0);
+		return fma(y * e, fma(0.375, e, 0.5), y);
+	}
+	return r2 > 0.0 ? rsqrt(r2) : 0.0;
+}
+
 // Programmatic dependent launch.  A kernel launched with programmatic stream
 // serialization may start while the kernel before it in the stream is still running:
 // grid_dep_wait() blocks until that kernel has completed and its memory operations are

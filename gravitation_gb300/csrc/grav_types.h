@@ -10,12 +10,20 @@
 
 namespace grav {
 
+// Modes with FP64 positions and slots.
+__host__ __device__ inline bool fp64_mode(int mode)
+{
+	return mode == GRAV_MODE_FP64 || mode == GRAV_MODE_FP64U;
+}
+
 // Launch-time view of one stage-1 kernel instantiation.
 struct Stage1Kernel {
 	int mode, bpt, threads, jtile;
 	const void* fn;       // __global__ function
 	int smem_bytes;       // dynamic shared memory per CTA
 	bool dependent;       // waits with grid_dep_wait(): may launch as a programmatic dependent
+	int block = 0;        // threads per CTA where they are not the tile's (rows / bpt)
+	int cta_threads() const { return block ? block : threads; }
 };
 
 // Stage-2 kernel (stage2.cu).  dependent = true launches it with programmatic stream

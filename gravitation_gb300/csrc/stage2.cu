@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(S2_THREADS) stage2_kernel(const grav_batch b, 
 
 	if (il >= U.n) {  // the whole lane group
 		if (p != 0) return;
-		if (b.mode == GRAV_MODE_FP64) {
+		if (fp64_mode(b.mode)) {
 			static_cast<drow4*>(b.pos)[g] = drow4{0.0, 0.0, 0.0, 0.0};
 		} else {
 			float4* q = static_cast<float4*>(b.pos);
@@ -86,8 +86,8 @@ __global__ void __launch_bounds__(S2_THREADS) stage2_kernel(const grav_batch b, 
 		const bool pairs = b.mode == GRAV_MODE_FP32U || b.mode == GRAV_MODE_FP32CU ||
 			b.mode == GRAV_MODE_FP32UN;
 		const int nrow = pairs ? S.nslots - S.il0 / IT : S.nslots;
-		if (b.mode == GRAV_MODE_FP64) {
-			// FP64 row slots p, p + TPR, ... added in order; each round issues all its
+		if (fp64_mode(b.mode)) {
+			// FP64 slots (rows, and columns in the unique-pair plan) p, p + TPR, ... added in order; each round issues all its
 			// loads first (the ones past the end are skipped): one latency per round
 			const double* __restrict__ part =
 				b.part + static_cast<int64_t>(S.slot_base) * stride + li;
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(S2_THREADS) stage2_kernel(const grav_batch b, 
 		}
 	}
 
-	if (b.mode == GRAV_MODE_FP64) {
+	if (fp64_mode(b.mode)) {
 		static_cast<drow4*>(b.pos)[g] = r;
 	} else {
 		float4* q = static_cast<float4*>(b.pos);

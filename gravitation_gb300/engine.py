@@ -79,8 +79,8 @@ def occupancy(mode, tile, device=None):
 
 def make_plan(sizes, T, tile, mode='fp32'):
     """Host-side plan (no GPU needed): (PlanInfo, univ ctypes array, seg ctypes array).
-    The unique-pair modes (fp32u, fp32cu, fp32un) use grav_plan_pairs, the others
-    grav_plan."""
+    The unique-pair modes (fp32u, fp32cu, fp32un, GRAV_MODE_FP64U) use grav_plan_pairs, the
+    others grav_plan."""
     L = _lib.load()
     fn = L.grav_plan_pairs if mode in _lib.PAIR_MODES else L.grav_plan
     sizes = [int(x) for x in sizes]
@@ -193,6 +193,28 @@ def default_tile(mode, sizes, device=None):
     return best[1]
 
 
+def fp64_pair_tile(sizes, sm_count, budget=None):
+    """Tile of the FP64 unique-pair kernel for this workload, or None where its slots do not
+    fit the slot budget (the ordered-pair kernel then serves).  The time is the FP64
+    instructions of the busiest SM: ceil(units / SMs) units of 32 columns against a block of
+    32, 64 or 128 rows, 20 per pair, and three per column slot and row in stage 2; small
+    blocks win where units are few (a step at 300 bodies: 12.5 us with 32 rows, 31 with 128;
+    at 8191 1.24-1.26 ms with any), large ones keep the slots few."""
+    if not any(sizes):
+        return None
+    best = None
+    for rows in (32, 64, 128):
+        t = _lib.Tile(1, rows, 32, sm_count)
+        if budget is not None and plan_part_bytes(sizes, t, _lib.GRAV_MODE_FP64U) > budget:
+            continue
+        info = make_plan(sizes, 1.0, t, _lib.GRAV_MODE_FP64U)[0]
+        slots = sum(-(-n // rows) * n / 2 for n in sizes)
+        cost = -(-info.n_units // sm_count) * rows * 20 + slots * 3 / 32 / sm_count
+        if best is None or cost < best[0]:
+            best = (cost, t)
+    return best and best[1]
+
+
 FUSED_MODES = ('fp32', 'fp32n', 'fp32c')
 # (largest n, (threads, rows)) of the single-launch step, the fastest measured on GB300
 # (graph-replayed steps, fp32n / fp32, against the two-launch step's 8.7-9.0 / 7.7-8.3
@@ -264,7 +286,9 @@ class Engine:
             self.mode_name, self.mode = mode, _lib.MODES[mode]
         else:
             self.mode = int(mode)
-            self.mode_name = {v: k for k, v in _lib.MODES.items()}[self.mode]
+            names = {v: k for k, v in _lib.MODES.items()}
+            names[_lib.GRAV_MODE_FP64U] = 'fp64'
+            self.mode_name = names[self.mode]
         self.sizes = [int(x) for x in sizes]
         self.T = list(T) if np.ndim(T) else [float(T)] * len(self.sizes)
         # queued steps in one launch, unless the caller picks the kernels himself
@@ -272,6 +296,12 @@ class Engine:
                         and default_steps(self.mode_name, self.sizes, self.dev_info))
         if fused is None:
             fused = default_fused(self.mode_name, self.sizes, self.dev_info)
+        if tile is None and self.mode == _lib.GRAV_MODE_FP64:
+            tile = fp64_pair_tile(self.sizes, self.dev_info.sm_count,
+                                  slot_budget_bytes(self.dev_info.index))
+            if tile is not None:
+                self.mode = _lib.GRAV_MODE_FP64U
+                tile.grid = 0
         if tile is None:
             if tuner is not None and not fused and not self.chained:
                 tile = tuner.choose(self.mode_name, self.sizes, self.dev_info, T=self.T)
@@ -283,7 +313,7 @@ class Engine:
         if not self.lib.grav_tile_supported(self.mode, ctypes.byref(tile)):
             raise ValueError('tile %r is not compiled for mode %s' % (tile, self.mode_name))
         self.tile = tile
-        self.info, univ, seg = make_plan(self.sizes, self.T, tile, self.mode_name)
+        self.info, univ, seg = make_plan(self.sizes, self.T, tile, self.mode)
         info = self.info
         dev = self.device
         self.univ_dev = _ctypes_to_device(univ, ctypes.sizeof(_lib.UnivDesc) * info.n_univ, dev)

@@ -63,6 +63,9 @@ extern "C" {
 #define GRAV_MODE_FP32UN 6    /* GRAV_MODE_FP32N's correction on unique pairs; plan with
                                  grav_plan_pairs */
 
+#define GRAV_MODE_FP64U 8     /* GRAV_MODE_FP64 on unique pairs (FP64 column slots); plan with
+                                 grav_plan_pairs */
+
 /* Near-pair radius of GRAV_MODE_FP32N / GRAV_MODE_FP32UN in units of the coordinate
  * magnitude: beyond |x| / 20 the FP32 rounding of the positions changes a pair term by
  * at most ~4.5e-6 of itself. */

@@ -72,3 +72,42 @@ def test_pair_tiles_at_block_edges(gpu, mode, case):
             eng.raise_on_device_error()
             err = np.linalg.norm(a - ref, axis=1) / scale
             assert err.max() < TOL, (mode, t, grid, n, err.max())
+
+
+@pytest.mark.parametrize('rows', [32, 64, 128])
+def test_fp64_pair_blocks(gpu, rows):
+    """The FP64 unique-pair kernel at the edges of its row blocks, close and coincident pairs
+    in one block and across blocks: 1e-14 of the pair terms' magnitudes (a term carries about
+    ten roundings of 2^-53, a sum of up to 450 terms the root of their number)."""
+    for n in (1, 31, rows - 1, rows, rows + 1, 3 * rows + 33):
+        r, v, m = planted_cube(n, rows, seed=700 + n)
+        if n > rows + 20:
+            r[rows + 17] = r[5]
+        gm = G_DEFAULT * m
+        ref, scale = oracle.accel_fp64(r, gm, 1.0, coincident=True), magnitudes(r, gm)
+        for grid in (0, 5):
+            eng = Engine([n], 1e3, mode=_lib.GRAV_MODE_FP64U, tile=_lib.Tile(1, rows, 32, grid))
+            assert eng.mode_name == 'fp64'
+            eng.set_state(r, v, gm)
+            a = eng.forces().cpu().numpy()
+            eng.raise_on_device_error()
+            err = np.linalg.norm(a - ref, axis=1)
+            assert np.all(err <= 1e-14 * scale), (rows, n, grid, np.max(err / np.maximum(scale, 1e-300)))
+
+
+def test_fp64_scratch_limits(gpu):
+    """Separations outside the fast reciprocal's range (and huge ones) follow the law: two
+    bodies 1e-120, 1e-60, 1e60 and 1e150 apart, and the default engine takes unique pairs."""
+    for d in (1e-120, 1e-60, 1.0, 1e60, 1e150):
+        r = np.array([[0.0, 0, 0], [d, 0, 0]])
+        gm = np.array([2.0, 3.0]) * d * d      # accelerations 3 and -2
+        eng = Engine([2], 1.0, mode='fp64')
+        assert eng.mode == _lib.GRAV_MODE_FP64U
+        eng.set_state(r, np.zeros((2, 3)), gm)
+        a = eng.forces().cpu().numpy()
+        ordered = Engine([2], 1.0, mode='fp64', tile=_lib.Tile(1, 128, 128, 0))
+        ordered.set_state(r, np.zeros((2, 3)), gm)
+        b = ordered.forces().cpu().numpy()
+        assert np.array_equal(np.isfinite(a), np.isfinite(b)), d
+        if 1e-100 < d < 1e100:
+            assert np.allclose(a, [[3.0, 0, 0], [-2.0, 0, 0]], rtol=1e-15), (d, a)
