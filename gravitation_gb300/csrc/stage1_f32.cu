@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(T) stage1_f32_kernel(const grav_batch b)
 			}
 			if (NEAR) {
 				rowlo[NEAR ? k : 0][NEAR ? tid : 0] = poslo[ibase + tid + k * T];
-				xmax = fmaxf(xmax, near_scale(p.x, p.y, p.z));
+				if (S.il0 + tid + k * T < Uu.n) xmax = fmaxf(xmax, near_scale(p.x, p.y, p.z));
 			}
 			fx[k] = fy[k] = fz[k] = 0.f;
 			hx[k] = hy[k] = hz[k] = lx[k] = ly[k] = lz[k] = 0.f;

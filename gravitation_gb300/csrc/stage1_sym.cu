@@ -174,9 +174,12 @@ __device__ __forceinline__ void expand_tile(ulonglong2* __restrict__ ex,
 }
 
 // B rows per thread, W warps, j-tiles of JT bodies; MINB CTAs per SM (the register limit);
-// COLPAIR: the even and odd rows' column sums rotate apart (two shuffles per component, for
-// DS and NEAR: 1.56 against 1.60 and 1.34 against 1.37 ms) or added up in each step (one
-// shuffle and two additions, for PLAIN: 1.17 against 1.19 ms).
+// COLPAIR: the even and odd rows' column sums rotate apart, a chain of 16 B terms each (two
+// shuffles per component), or the rows of a step are added up before they join the rotating
+// sum, a chain of 32 (one shuffle and two additions).  The shorter chain is the more exact
+// one: rows of 4 keep the sums apart, rows of 8 add them (rms force error at 65536 bodies
+// 5.6e-8 against 1.0e-7 and 1.3e-7 against 7e-8; within 3 % in time either way).  The plain
+// mode, whose error is the rounding of the positions, adds them always (2 % faster).
 template <int B, int W, int JT, int KIND, int UNROLL, int MINB, bool COLPAIR>
 __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_batch b)
 {
@@ -298,7 +301,9 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 			if (NEAR) {
 				rowlo[(2 * h) * T] = pos[b.n_pad_total + ibase + (2 * h) * 32];
 				rowlo[(2 * h + 1) * T] = pos[b.n_pad_total + ibase + (2 * h + 1) * 32];
-				xmax = fmaxf(xmax, fmaxf(near_scale(p.x, p.y, p.z), near_scale(q.x, q.y, q.z)));
+				const int row = S.il0 + warp * 32 * B + (2 * h) * 32 + lane;   // of the universe
+				if (row < Uu.n) xmax = fmaxf(xmax, near_scale(p.x, p.y, p.z));
+				if (row + 32 < Uu.n) xmax = fmaxf(xmax, near_scale(q.x, q.y, q.z));
 			}
 			fx[h] = fy[h] = fz[h] = 0ull;
 		}
@@ -525,8 +530,8 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 		reinterpret_cast<const void*>(&stage1_sym_kernel<B, W, J, KIND, UN, MINB, CP>), \
 		SymSmem<B, W, J, KIND>::BYTES, false}
 #define GRAV_SYM_ENTRY(B, W, J, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32U, SYM_PLAIN, B, W, J, 4, MINB, false)
-#define GRAV_SYMC_ENTRY(B, W, J, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32CU, SYM_DS, B, W, J, 4, MINB, true)
-#define GRAV_SYMN_ENTRY(B, W, J, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32UN, SYM_NEAR, B, W, J, 4, MINB, true)
+#define GRAV_SYMC_ENTRY(B, W, J, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32CU, SYM_DS, B, W, J, 4, MINB, B < 8)
+#define GRAV_SYMN_ENTRY(B, W, J, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32UN, SYM_NEAR, B, W, J, 4, MINB, B < 8)
 
 // The step loop is unrolled by 4 (by 2 fp32un 1.38, by 8 1.34, by 4 1.34 ms; by 16 and more it
 // spills).  MINB is the occupancy at which the loop keeps its registers: 8 rows per thread

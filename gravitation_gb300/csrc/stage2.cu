@@ -7,7 +7,8 @@
 //     v = a*T + v ;  r = v*T + r          (_base_.py:58-62, np2.py:110-115)
 // exactly as the reference's Python floats / numpy arrays round them, and finally
 // rewrites the row of the stage-1 position array (FP32 hi[, lo] or FP64).  Padding
-// rows get zeros (G*m = 0), so padded j-tiles contribute nothing.
+// rows get G*m = 0, so padded j-tiles contribute nothing, and zeros for coordinates (FAR_PAD
+// in the near modes).
 #include "grav_device.cuh"
 
 namespace grav {
@@ -61,7 +62,8 @@ __global__ void __launch_bounds__(S2_THREADS) stage2_kernel(const grav_batch b, 
 			static_cast<drow4*>(b.pos)[g] = drow4{0.0, 0.0, 0.0, 0.0};
 		} else {
 			float4* q = static_cast<float4*>(b.pos);
-			q[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+			const float far = b.mode == GRAV_MODE_FP32N || b.mode == GRAV_MODE_FP32UN ? FAR_PAD : 0.f;
+			q[g] = make_float4(far, far, far, 0.f);
 			if (has_lo(b.mode)) q[b.n_pad_total + g] = make_float4(0.f, 0.f, 0.f, 0.f);
 		}
 		return;

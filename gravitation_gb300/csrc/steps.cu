@@ -235,10 +235,9 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 		vv = vd[e];
 	}
 
-	// positions of every body; padding columns sit far away with Gm = 0: no contribution, and
-	// never near (the origin might be)
+	// positions of every body; padding columns as FAR_PAD says
 	for (int p = tid; p < NB * 32; p += ST_T) {
-		const float4 far = make_float4(1e18f, 1e18f, 1e18f, 0.f), z = make_float4(0.f, 0.f, 0.f, 0.f);
+		const float4 far = make_float4(FAR_PAD, FAR_PAD, FAR_PAD, 0.f), z = make_float4(0.f, 0.f, 0.f, 0.f);
 		const int j = 2 * p;
 		const float4 a = j < n ? pos[j] : far, c = j + 1 < n ? pos[j + 1] : far;
 		set_pair(cols, p, a, c);
@@ -536,7 +535,7 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 					const int j1 = min(j + 1, n - 1);
 					ok = ok && wait_word(src + j, want, w0[i]) && wait_word(src + j1, want, w1[i]);
 					float4 c = word_position(w1[i]);
-					if (j + 1 >= n) c = make_float4(1e18f, 1e18f, 1e18f, 0.f);
+					if (j + 1 >= n) c = make_float4(FAR_PAD, FAR_PAD, FAR_PAD, 0.f);
 					set_pair(cols, p, word_position(w0[i]), c);
 					if (lo_here) {
 						ok = ok && wait_word(src + words + j, want, l0[i]) &&
