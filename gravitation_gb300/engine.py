@@ -161,33 +161,71 @@ def _ctypes_to_device(arr, nbytes, device):
     return dev
 
 
+# SM time per pair of every compiled tile with three or more warps per scheduler (picoseconds;
+# an ordered pair of the all-pairs modes, an unordered one of the others), from stage 1 at
+# 65536 / 131072 bodies on GB300.
+TILE_COST = {
+    'fp32': {(1, 128, 128): 73, (2, 128, 128): 70, (4, 128, 128): 70, (4, 128, 256): 69,
+             (8, 128, 256): 72, (2, 256, 256): 66, (4, 256, 256): 69, (8, 256, 256): 69},
+    'fp32n': {(1, 128, 128): 94, (2, 128, 128): 82, (4, 128, 128): 74, (4, 128, 256): 73,
+              (8, 128, 256): 72, (4, 256, 256): 73},
+    'fp32c': {(1, 128, 128): 108, (2, 128, 128): 100, (4, 128, 256): 98, (4, 256, 256): 95},
+    'fp32u': {(4, 128, 128): 88, (4, 256, 256): 85, (8, 128, 256): 62, (4, 128, 256): 69,
+              (2, 256, 256): 101, (8, 256, 256): 60, (8, 128, 128): 81, (8, 128, 64): 90,
+              (4, 64, 64): 91},
+    'fp32un': {(4, 128, 128): 99, (8, 128, 256): 69, (8, 128, 128): 73, (8, 128, 64): 99,
+               (4, 128, 256): 74, (4, 256, 256): 74, (4, 64, 64): 101, (8, 64, 64): 96,
+               (8, 64, 128): 70},
+    'fp32cu': {(4, 128, 128): 118, (8, 128, 256): 57, (4, 128, 256): 71, (4, 256, 256): 84,
+               (8, 128, 128): 81, (4, 64, 64): 122, (8, 64, 64): 117},
+}
+
+
+def tile_time(mode, tile, info, sm_count, resident):
+    """Estimated step time (us) of a plan: the busiest SM's units at the tile's cost, slower
+    where fewer than three warps per scheduler are resident (half the rate with one, 0.8 with
+    two), plus the slots' traffic in stage 2 (24 bytes per entry, written and read, at ~8
+    TB/s).  Over the six FP32 modes at 300-131072 bodies (96 measured sets of tiles) the tile
+    it picks ran within 0.4 % of the fastest on average, at worst 12 % (fp32cu at 6500
+    bodies); the rule before it, which did not count the CTAs that share an SM, was 5-30 %
+    off above 8192 bodies."""
+    grid = min(info.grid, info.n_units)
+    on_sm = min(-(-grid // sm_count), resident)
+    warps = on_sm * tile.threads / 128.0
+    rate = (1.0 if warps >= 3 else 0.8 + 0.2 * (warps - 2) if warps >= 2 else
+            0.5 + 0.3 * (warps - 1) if warps >= 1 else 0.5 * warps)
+    cost = TILE_COST.get(mode, {}).get(tile.key(), 100.0)
+    units = -(-info.n_units // grid) * on_sm
+    return (units * info.itile * tile.jtile * cost * 1e-6 / rate +
+            info.n_slots * info.itile * 24 / 8e6)
+
+
+# Longest j-tile the default picks: its FP32 partial sums run over one j-tile, and twice the
+# length is ~10 % more rms force error (fp32un at 65536 bodies: 1.22e-7 with 64-body tiles,
+# 1.51e-7 with 128, 2.4e-7 with 256) for 2 % of time.
+DEFAULT_JTILE_MAX = {'fp32u': 64, 'fp32un': 64}
+
+
 def default_tile(mode, sizes, device=None):
-    """Tile shape used when no tuned entry exists: the largest i-tile that still gives
-    every resident CTA several work units."""
+    """Tile shape used when no tuned entry exists: of the shapes with short partial sums
+    (DEFAULT_JTILE_MAX, else 128 bodies) the one with the smallest estimated step time
+    (tile_time)."""
     info = device_info(device)
     cands = fitting_tiles(sizes, mode) or tile_list(mode)
+    longest = DEFAULT_JTILE_MAX.get(mode, 128)
+    cands = [t for t in cands if t.jtile <= longest] or cands
     best = None
     for t in cands:
         occ = occupancy(mode, t, device)
         if occ <= 0:
             continue
-        grid = info.sm_count * occ
-        t.grid = grid
+        t.grid = info.sm_count * occ
         pinfo, _, _ = make_plan(sizes, 1.0, t, mode)
-        if pinfo.n_units == 0:
-            # no pairs at all (only empty universes): stage 1 launches nothing, any
-            # compiled shape serves
-            if best is None:
-                best = (float('inf'), _lib.Tile(t.bpt, t.threads, t.jtile, grid))
-            continue
-        # padded work (interactions) and the slowest CTA's share of it
-        work = pinfo.n_units * pinfo.itile * t.jtile
-        per_cta = -(-pinfo.n_units // min(grid, pinfo.n_units)) * pinfo.itile * t.jtile
-        # register-blocked shapes issue fewer shared loads per interaction
-        eff = {1: 0.80, 2: 0.90, 4: 0.97, 8: 1.0}.get(t.bpt, 0.9)
-        score = per_cta / eff + 0.02 * work / grid
+        # no pairs at all (only empty universes): stage 1 launches nothing, any compiled
+        # shape serves
+        score = tile_time(mode, t, pinfo, info.sm_count, occ) if pinfo.n_units else float('inf')
         if best is None or score < best[0]:
-            best = (score, _lib.Tile(t.bpt, t.threads, t.jtile, grid))
+            best = (score, t)
     if best is None:
         raise RuntimeError('no compiled tile shape fits mode %r' % (mode,))
     return best[1]
