@@ -529,13 +529,19 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 	{MODE, B, 32 * W, J, \
 		reinterpret_cast<const void*>(&stage1_sym_kernel<B, W, J, KIND, UN, MINB, CP>), \
 		SymSmem<B, W, J, KIND>::BYTES, false}
-#define GRAV_SYM_ENTRY(B, W, J, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32U, SYM_PLAIN, B, W, J, 4, MINB, false)
-#define GRAV_SYMC_ENTRY(B, W, J, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32CU, SYM_DS, B, W, J, 4, MINB, B < 8)
-#define GRAV_SYMN_ENTRY(B, W, J, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32UN, SYM_NEAR, B, W, J, 4, MINB, B < 8)
+#define GRAV_SYM_ENTRY(B, W, J, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32U, SYM_PLAIN, B, W, J, 16, MINB, false)
+#define GRAV_SYMC_ENTRY(B, W, J, UN, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32CU, SYM_DS, B, W, J, UN, MINB, B < 8)
+#define GRAV_SYMN_ENTRY(B, W, J, UN, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32UN, SYM_NEAR, B, W, J, UN, MINB, B < 8)
 
-// The step loop is unrolled by 4 (by 2 fp32un 1.38, by 8 1.34, by 4 1.34 ms; by 16 and more it
-// spills).  MINB is the occupancy at which the loop keeps its registers: 8 rows per thread
-// want ~165 (fp32cu ~200); at 128 registers it measured 5-9 % slower.
+// UN (unrolling of the step loop) and MINB (the occupancy that ptxas must leave room for) as
+// measured per shape over 2, 4, 8 and 16 steps and the occupancies around each; no sum's order
+// depends on them.  Stage 1 at 65536 bodies, unrolled by 4 at the higher occupancy and as
+// compiled here:
+//   fp32un 8/64/64 1376 (6 CTAs, 168 registers, 8 bytes spilled) and 1352 us (4 CTAs, 200),
+//     at 16384 bodies 102 and 94; fp32un 8/64/128 1353 and 1326;
+//   fp32cu 8/64/64 1682 (6 CTAs, 165 registers) and 1580 us (4 CTAs, 194);
+//   fp32u 8/128/64 1297 and 1225, 8/64/64 1210 and 1200, at 16384 bodies 88 and 82.
+// Two warps per scheduler with every operand in registers beat three that reload some.
 static const Stage1Kernel k_table_sym[] = {
 	GRAV_SYM_ENTRY(4, 4, 128, 4),
 	GRAV_SYM_ENTRY(4, 8, 256, 2),
@@ -546,22 +552,23 @@ static const Stage1Kernel k_table_sym[] = {
 	GRAV_SYM_ENTRY(8, 4, 128, 3),
 	GRAV_SYM_ENTRY(8, 4, 64, 3),
 	GRAV_SYM_ENTRY(4, 2, 64, 8),
-	GRAV_SYMC_ENTRY(4, 4, 128, 3),
-	GRAV_SYMC_ENTRY(8, 4, 256, 1),
-	GRAV_SYMC_ENTRY(4, 4, 256, 2),
-	GRAV_SYMC_ENTRY(4, 8, 256, 1),
-	GRAV_SYMC_ENTRY(8, 4, 128, 2),
-	GRAV_SYMC_ENTRY(4, 2, 64, 6),
-	GRAV_SYMC_ENTRY(8, 2, 64, 5),
-	GRAV_SYMN_ENTRY(4, 4, 128, 3),
-	GRAV_SYMN_ENTRY(8, 4, 256, 2),
-	GRAV_SYMN_ENTRY(8, 4, 128, 3),
-	GRAV_SYMN_ENTRY(8, 4, 64, 3),
-	GRAV_SYMN_ENTRY(4, 4, 256, 2),
-	GRAV_SYMN_ENTRY(4, 8, 256, 1),
-	GRAV_SYMN_ENTRY(4, 2, 64, 7),
-	GRAV_SYMN_ENTRY(8, 2, 64, 5),
-	GRAV_SYMN_ENTRY(8, 2, 128, 4),
+	GRAV_SYM_ENTRY(8, 2, 64, 4),
+	GRAV_SYMC_ENTRY(4, 4, 128, 16, 3),
+	GRAV_SYMC_ENTRY(8, 4, 256, 4, 1),
+	GRAV_SYMC_ENTRY(4, 4, 256, 16, 2),
+	GRAV_SYMC_ENTRY(4, 8, 256, 16, 1),
+	GRAV_SYMC_ENTRY(8, 4, 128, 4, 2),
+	GRAV_SYMC_ENTRY(4, 2, 64, 16, 5),
+	GRAV_SYMC_ENTRY(8, 2, 64, 4, 4),
+	GRAV_SYMN_ENTRY(4, 4, 128, 8, 3),
+	GRAV_SYMN_ENTRY(8, 4, 256, 8, 2),
+	GRAV_SYMN_ENTRY(8, 4, 128, 8, 2),
+	GRAV_SYMN_ENTRY(8, 4, 64, 8, 2),
+	GRAV_SYMN_ENTRY(4, 4, 256, 16, 2),
+	GRAV_SYMN_ENTRY(4, 8, 256, 16, 1),
+	GRAV_SYMN_ENTRY(4, 2, 64, 8, 7),
+	GRAV_SYMN_ENTRY(8, 2, 64, 4, 4),
+	GRAV_SYMN_ENTRY(8, 2, 128, 8, 4),
 };
 
 int stage1_table_sym(const Stage1Kernel** out)

@@ -170,14 +170,14 @@ TILE_COST = {
     'fp32n': {(1, 128, 128): 94, (2, 128, 128): 82, (4, 128, 128): 74, (4, 128, 256): 73,
               (8, 128, 256): 72, (4, 256, 256): 73},
     'fp32c': {(1, 128, 128): 108, (2, 128, 128): 100, (4, 128, 256): 98, (4, 256, 256): 95},
-    'fp32u': {(4, 128, 128): 88, (4, 256, 256): 85, (8, 128, 256): 62, (4, 128, 256): 69,
-              (2, 256, 256): 101, (8, 256, 256): 60, (8, 128, 128): 81, (8, 128, 64): 90,
-              (4, 64, 64): 91},
-    'fp32un': {(4, 128, 128): 99, (8, 128, 256): 69, (8, 128, 128): 73, (8, 128, 64): 99,
-               (4, 128, 256): 74, (4, 256, 256): 74, (4, 64, 64): 101, (8, 64, 64): 96,
-               (8, 64, 128): 70},
-    'fp32cu': {(4, 128, 128): 118, (8, 128, 256): 57, (4, 128, 256): 71, (4, 256, 256): 84,
-               (8, 128, 128): 81, (4, 64, 64): 122, (8, 64, 64): 117},
+    'fp32u': {(4, 128, 128): 87, (4, 256, 256): 85, (8, 128, 256): 64, (4, 128, 256): 71,
+              (2, 256, 256): 101, (8, 256, 256): 63, (8, 128, 128): 81, (8, 128, 64): 85,
+              (4, 64, 64): 90, (8, 64, 64): 67},
+    'fp32un': {(4, 128, 128): 96, (8, 128, 256): 72, (8, 128, 128): 73, (8, 128, 64): 76,
+               (4, 128, 256): 76, (4, 256, 256): 73, (4, 64, 64): 100, (8, 64, 64): 75,
+               (8, 64, 128): 73},
+    'fp32cu': {(4, 128, 128): 114, (8, 128, 256): 57, (4, 128, 256): 61, (4, 256, 256): 88,
+               (8, 128, 128): 86, (4, 64, 64): 118, (8, 64, 64): 88},
 }
 
 
@@ -185,9 +185,9 @@ def tile_time(mode, tile, info, sm_count, resident):
     """Estimated step time (us) of a plan: the busiest SM's units at the tile's cost, slower
     where fewer than three warps per scheduler are resident (half the rate with one, 0.8 with
     two), plus the slots' traffic in stage 2 (24 bytes per entry, written and read, at ~8
-    TB/s).  Over the six FP32 modes at 300-131072 bodies (96 measured sets of tiles) the tile
-    it picks ran within 0.4 % of the fastest on average, at worst 12 % (fp32cu at 6500
-    bodies); the rule before it, which did not count the CTAs that share an SM, was 5-30 %
+    TB/s).  Over the unique-pair modes at 300-131072 bodies (42 measured sets of tiles) the
+    tile it picks ran within 0.3 % of the fastest on average, at worst 7 % (fp32cu at 6500
+    bodies), over the all-pairs modes within 0.4 %; the rule before it, which did not count the CTAs that share an SM, was 5-30 %
     off above 8192 bodies."""
     grid = min(info.grid, info.n_units)
     on_sm = min(-(-grid // sm_count), resident)
