@@ -5,12 +5,13 @@
 // dependent launches per step (the persistent stage-1 grid, then stage 2 over its slots)
 // spend most of it on launch, drain and memory latency: 8.8 us per step at 64 bodies, 9.2 us
 // at 1000, 17.7 us at 4096 (fp32n, graph-replayed).  Here one grid of at most one CTA per SM
-// stays for all K steps: 2.1, 4.1 and 14.4 us per step of 20.  Each CTA keeps the FP64 state
+// stays for all K steps: 1.9, 3.6 and 11.6 us per step of 20.  Each CTA keeps the FP64 state
 // of its R rows in registers and every body's FP32 position in shared memory; per step it
 // completes its rows' accelerations over all columns, integrates the rows and exchanges the
-// new positions with the other CTAs.  At 1000 bodies a step is ~0.9 us of pair work, ~0.8 us
-// of FP64 update (a chain of eleven FP64 instructions of 67 cycles each) and ~2 us of
-// exchange and waiting for the slowest CTA; from ~4000 bodies the pair loop is most of it.
+// new positions with the other CTAs.  At 1000 bodies a step is ~1 us of pair work and ~0.5 us
+// of the slowest warp's near pairs, ~0.8 us of FP64 update (a chain of eleven FP64
+// instructions of 67 cycles each) and ~1.4 us of exchange; at 4096 the pair loop takes 7.8 us,
+// 70 % of what its FMA-pipe instructions need.
 //
 // Exchange.  There is no grid barrier between steps.  A row's new position is published as
 // a 128-bit word (x, y, z, tag) by one relaxed 128-bit store and read by one relaxed
@@ -33,8 +34,17 @@
 // pairs.  12 packed FMA-pipe instructions and two reciprocal square roots per row and pair
 // (24 + 4 cycles), one 128-bit shared load; with one row per lane and two loads the loads'
 // return path was as long as the arithmetic.  Partials are FP32 over 16 blocks (32
-// terms per lane and column parity) and added into a second FP32 level; the warps' pieces of a row are added by
-// TwoSum (48 bits) in warp order: nothing depends on scheduling.
+// terms per lane and column parity) and added into a second FP32 level; the warps' pieces of
+// a row are added by TwoSum (48 bits) in warp order: nothing depends on scheduling.
+//
+// Near pairs.  The loop keeps one bit per block and lane that met a pair within the near
+// radius; after every 32 blocks each lane goes through its own blocks' near pairs, all lanes
+// side by side.  The CTAs run in step, so the warp with the most near pairs sets everyone's
+// pace: with the warp going through the union of its lanes' blocks after every 16, a step took
+// 4.5 us at 1000 bodies (2.9 without the near pairs) and 14.0 at 4096; so 3.8 and 11.6.  The
+// low parts are not kept in shared memory (unless one CTA holds every row): the few that near
+// pairs need come from the exchange buffer, and the exchange moves half the bytes (14.0 to
+// 12.6 us at 4096).
 #include "grav_device.cuh"
 
 namespace grav {
@@ -44,7 +54,8 @@ constexpr int ST_T = 512;            // threads per CTA
 constexpr int ST_W = ST_T / 32;
 constexpr int ST_RG = 4;             // rows per group
 constexpr int ST_CB = 64;            // columns per block
-constexpr int ST_CHUNK = 16;          // blocks per first-level FP32 sum
+constexpr int ST_CHUNK = 16;         // blocks per first-level FP32 sum
+constexpr int ST_SEG = 32;           // blocks between two passes over the near pairs met
 constexpr int ST_RPW = 10;           // rows whose state one warp holds (3 lanes each)
 constexpr int ST_MAX_ROWS = ST_RPW * ST_W;
 constexpr int ST_SMEM_MAX = 227 * 1024;
@@ -119,7 +130,7 @@ __device__ __forceinline__ unsigned steps_cluster_ctas()
 // Shared memory of one CTA for n bodies and R rows per CTA (byte offsets, 16-byte units).
 struct StepsSmem {
 	int cols;     // [blocks][2][32] ulonglong2: (x0, x1 | y0, y1), (z0, z1 | Gm0, Gm1)
-	int colslo;   // the same for the low parts (DS, and NEAR where they fit: lo_here)
+	int colslo;   // the same for the low parts (DS, and NEAR with one CTA: lo_here)
 	int rown;     // [rows][2] ulonglong2: (-x, -x | -y, -y), (-z, -z | near radius^2)
 	int rownlo;   // the same for the low parts (DS, NEAR)
 	int red;      // [groups + warps][ST_RG][3] float: the pieces' sums
@@ -130,8 +141,7 @@ struct StepsSmem {
 		const int nb = (n + ST_CB - 1) / ST_CB;
 		const int ng = (rows + ST_RG - 1) / ST_RG;
 		const int r4 = ng * ST_RG;
-		const int tail = r4 * 64 + (ng + ST_W) * ST_RG * 3 * 4;
-		lo_here = kind == STEPS_DS || nb * 2048 + tail <= ST_SMEM_MAX;
+		lo_here = kind == STEPS_DS || rows >= n;
 		cols = 0;
 		colslo = cols + nb * 1024;
 		rown = colslo + (lo_here ? nb * 1024 : 0);
@@ -295,110 +305,114 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 				sx[r] = sy[r] = sz[r] = 0ull;
 			}
 			do {
-				const int m = min(ST_CHUNK, left);
+				const int m = min(ST_SEG, left);
 				const ulonglong2* __restrict__ cp = cols + cb * 64 + c16;
 				const ulonglong2* __restrict__ cl = colslo + cb * 64 + c16;
-				u64 fx[2], fy[2], fz[2];
 				uint32_t nmask = 0;   // NEAR: bit q of a block q that holds a near pair
+#pragma unroll 1
+				for (int q0 = 0; q0 < m; q0 += ST_CHUNK) {
+					const int q1 = min(m, q0 + ST_CHUNK);
+					u64 fx[2], fy[2], fz[2];
 #pragma unroll
-				for (int r = 0; r < 2; ++r) fx[r] = fy[r] = fz[r] = 0ull;
-#pragma unroll 2
-				for (int q = 0; q < m; ++q, cp += 64, cl += 64) {
-					uint32_t rmin[2] = {0xffffffffu, 0xffffffffu};
+					for (int r = 0; r < 2; ++r) fx[r] = fy[r] = fz[r] = 0ull;
+#pragma unroll (NEAR ? 4 : 2)
+					for (int q = q0; q < q1; ++q, cp += 64, cl += 64) {
+						uint32_t rmin[2] = {0xffffffffu, 0xffffffffu};
 #pragma unroll
-					for (int i = 0; i < 2; ++i) {
-						const ulonglong2 cxy = cp[16 * i], czw = cp[16 * i + 32];
-						ulonglong2 dxy = make_ulonglong2(0ull, 0ull), dzz = dxy;
-						if (DS) {
-							dxy = cl[16 * i];
-							dzz = cl[16 * i + 32];
-						}
-#pragma unroll
-						for (int r = 0; r < 2; ++r) {
-							u64 dx = add2(cxy.x, nx[r]), dy = add2(cxy.y, ny[r]), dz = add2(czw.x, nz[r]);
+						for (int i = 0; i < 2; ++i) {
+							const ulonglong2 cxy = cp[16 * i], czw = cp[16 * i + 32];
+							ulonglong2 dxy = make_ulonglong2(0ull, 0ull), dzz = dxy;
 							if (DS) {
-								dx = add2(dx, add2(dxy.x, lx[r]));
-								dy = add2(dy, add2(dxy.y, ly[r]));
-								dz = add2(dz, add2(dzz.x, lz[r]));
+								dxy = cl[16 * i];
+								dzz = cl[16 * i + 32];
 							}
-							float ra, rb;
-							unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
-							if (NEAR)
-								rmin[r] = min(__float_as_uint(ra) - eps_bits,
-									min(__float_as_uint(rb) - eps_bits, rmin[r]));
-							const u64 inv = pack2(rsqrt_sfu(ra), rsqrt_sfu(rb));
-							const u64 w = mul2(mul2(czw.y, inv), mul2(inv, inv));
-							fx[r] = fma2(dx, w, fx[r]);
-							fy[r] = fma2(dy, w, fy[r]);
-							fz[r] = fma2(dz, w, fz[r]);
+#pragma unroll
+							for (int r = 0; r < 2; ++r) {
+								u64 dx = add2(cxy.x, nx[r]), dy = add2(cxy.y, ny[r]), dz = add2(czw.x, nz[r]);
+								if (DS) {
+									dx = add2(dx, add2(dxy.x, lx[r]));
+									dy = add2(dy, add2(dxy.y, ly[r]));
+									dz = add2(dz, add2(dzz.x, lz[r]));
+								}
+								float ra, rb;
+								unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
+								if (NEAR)
+									rmin[r] = min(__float_as_uint(ra) - eps_bits,
+										min(__float_as_uint(rb) - eps_bits, rmin[r]));
+								const u64 inv = pack2(rsqrt_sfu(ra), rsqrt_sfu(rb));
+								const u64 w = mul2(mul2(czw.y, inv), mul2(inv, inv));
+								fx[r] = fma2(dx, w, fx[r]);
+								fy[r] = fma2(dy, w, fy[r]);
+								fz[r] = fma2(dz, w, fz[r]);
+							}
 						}
+						if (NEAR && (rmin[0] < near_below[0] || rmin[1] < near_below[1])) nmask |= 1u << q;
 					}
-					if (NEAR && (rmin[0] < near_below[0] || rmin[1] < near_below[1])) nmask |= 1u << q;
+#pragma unroll
+					for (int r = 0; r < 2; ++r) {
+						sx[r] = add2(sx[r], fx[r]);
+						sy[r] = add2(sy[r], fy[r]);
+						sz[r] = add2(sz[r], fz[r]);
+					}
 				}
 				if (NEAR) {
-					// cold path: the blocks that met a pair within the near radius, pair by pair
-					uint32_t todo = __reduce_or_sync(0xffffffffu, nmask);
-					while (todo) {
-						const int q = __ffs(todo) - 1;
-						todo &= todo - 1;
-#pragma unroll 1
+					// cold path: each lane goes through the blocks where it met a pair within the near
+					// radius, one such pair at a time, all lanes side by side
+					while (nmask) {
+						const int at = (cb + __ffs(nmask) - 1) * 64 + c16;
+						nmask &= nmask - 1;
+						uint32_t found = 0;   // bit 4 i + 2 r + h: column h of pair i against row r
+#pragma unroll
 						for (int i = 0; i < 2; ++i) {
-							const int at = (cb + q) * 64 + 16 * i + c16;
-							const ulonglong2 cxy = cols[at], czw = cols[at + 32];
-							float4 l0, l1;
-							bool have = false;
+							const ulonglong2 cxy = cols[at + 16 * i], czw = cols[at + 16 * i + 32];
 #pragma unroll
 							for (int r = 0; r < 2; ++r) {
 								const u64 dx = add2(cxy.x, nx[r]), dy = add2(cxy.y, ny[r]), dz = add2(czw.x, nz[r]);
 								float ra, rb;
 								unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
-								const bool na = (ra < thr[r]) & (ra > eps2), nb = (rb < thr[r]) & (rb > eps2);
-								if (!(na | nb)) continue;
-								if (!have) {   // the two columns' low parts
-									const int j = (cb + q) * ST_CB + 2 * (16 * i + c16), j1 = min(j + 1, n - 1);
-									have = true;
-									if (lo_here) {
-										const ulonglong2 dxy = colslo[at], dzz = colslo[at + 32];
-										unpack2(dxy.x, l0.x, l1.x);
-										unpack2(dxy.y, l0.y, l1.y);
-										unpack2(dzz.x, l0.z, l1.z);
-									} else if (k == 0) {
-										l0 = poslo[j];
-										l1 = poslo[j1];
-									} else {
-										const float4* glo = xbuf + (((k - 1) & 1) * 2 + 1) * words;
-										const uint32_t tag = tag0 + static_cast<uint32_t>(k) - 1;
-										u128 w0 = load_word(glo + j), w1 = load_word(glo + j1);
-										ok = wait_word(glo + j, tag, w0) && wait_word(glo + j1, tag, w1) && ok;
-										l0 = word_position(w0);
-										l1 = word_position(w1);
-									}
-								}
-								const ulonglong2 lxy = rlp[2 * r], lzz = rlp[2 * r + 1];
-								float4 li;
-								float x0, x1, y0, y1, z0, z1, ex0, ey0, ez0, ex1, ey1, ez1;
-								unpack2(lxy.x, li.x, x0);
-								unpack2(lxy.y, li.y, x0);
-								unpack2(lzz.x, li.z, x0);
-								li = make_float4(-li.x, -li.y, -li.z, 0.f);
-								unpack2(dx, x0, x1);
-								unpack2(dy, y0, y1);
-								unpack2(dz, z0, z1);
-								near_delta(x0, y0, z0, ra, l0, li, eps2, na, ex0, ey0, ez0);
-								near_delta(x1, y1, z1, rb, l1, li, eps2, nb, ex1, ey1, ez1);
-								fx[r] = fma2(pack2(ex0, ex1), czw.y, fx[r]);
-								fy[r] = fma2(pack2(ey0, ey1), czw.y, fy[r]);
-								fz[r] = fma2(pack2(ez0, ez1), czw.y, fz[r]);
+								if ((ra < thr[r]) & (ra > eps2)) found |= 1u << (4 * i + 2 * r);
+								if ((rb < thr[r]) & (rb > eps2)) found |= 2u << (4 * i + 2 * r);
 							}
 						}
-						__syncwarp();
+						while (found) {
+							const int bit = __ffs(found) - 1;
+							found &= found - 1;
+							const int i = bit >> 2, r = bit >> 1 & 1, h = bit & 1;
+							const float* cf = reinterpret_cast<const float*>(cols + at + 16 * i) + h;
+							const float* rf = reinterpret_cast<const float*>(rp + 2 * r);
+							const float* lf = reinterpret_cast<const float*>(rlp + 2 * r);
+							// the padding columns are near only a body that sits where they do
+							const int j = min((at & ~63) + 2 * (16 * i + c16) + h, n - 1);
+							float4 lj;
+							if (lo_here) {
+								const float* clf = reinterpret_cast<const float*>(colslo + at + 16 * i) + h;
+								lj = make_float4(clf[0], clf[2], clf[128], 0.f);
+							} else if (k == 0) {
+								lj = poslo[j];
+							} else {
+								const float4* glo = xbuf + (((k - 1) & 1) * 2 + 1) * words + j;
+								u128 w = load_word(glo);
+								ok = wait_word(glo, tag0 + static_cast<uint32_t>(k) - 1, w) && ok;
+								lj = word_position(w);
+							}
+							const float dx = cf[0] + rf[0], dy = cf[2] + rf[2], dz = cf[128] + rf[4];
+							const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
+							float ex, ey, ez;
+							near_delta(dx, dy, dz, r2, lj, make_float4(-lf[0], -lf[2], -lf[4], 0.f), eps2,
+								true, ex, ey, ez);
+							const u64 gm = pack2(cf[130], 0.f);
+							if (r) {
+								sx[1] = fma2(pack2(ex, 0.f), gm, sx[1]);
+								sy[1] = fma2(pack2(ey, 0.f), gm, sy[1]);
+								sz[1] = fma2(pack2(ez, 0.f), gm, sz[1]);
+							} else {
+								sx[0] = fma2(pack2(ex, 0.f), gm, sx[0]);
+								sy[0] = fma2(pack2(ey, 0.f), gm, sy[0]);
+								sz[0] = fma2(pack2(ez, 0.f), gm, sz[0]);
+							}
+						}
 					}
-				}
-#pragma unroll
-				for (int r = 0; r < 2; ++r) {
-					sx[r] = add2(sx[r], fx[r]);
-					sy[r] = add2(sy[r], fy[r]);
-					sz[r] = add2(sz[r], fz[r]);
+					__syncwarp();
 				}
 				left -= m;
 				cb += m;
@@ -513,37 +527,22 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 		if (multi && !last) {
 			const float4* __restrict__ src = xbuf + (k & 1) * 2 * words;
 			const uint32_t want = tag0 + k;
-			constexpr int IN_FLIGHT = 2;
-			for (int p0 = tid; 2 * p0 < n; p0 += IN_FLIGHT * ST_T) {
-				u128 w0[IN_FLIGHT], w1[IN_FLIGHT], l0[IN_FLIGHT], l1[IN_FLIGHT];
-#pragma unroll
-				for (int i = 0; i < IN_FLIGHT; ++i) {
-					const int j = 2 * (p0 + i * ST_T);
-					if (j >= n) continue;
-					const int j1 = min(j + 1, n - 1);
-					w0[i] = load_word(src + j);
-					w1[i] = load_word(src + j1);
-					if (lo_here) {
-						l0[i] = load_word(src + words + j);
-						l1[i] = load_word(src + words + j1);
-					}
+			for (int p = tid; 2 * p < n; p += ST_T) {
+				const int j = 2 * p, j1 = min(j + 1, n - 1);
+				u128 w0 = load_word(src + j), w1 = load_word(src + j1), l0 = 0, l1 = 0;
+				if (lo_here) {
+					l0 = load_word(src + words + j);
+					l1 = load_word(src + words + j1);
 				}
-#pragma unroll
-				for (int i = 0; i < IN_FLIGHT; ++i) {
-					const int p = p0 + i * ST_T, j = 2 * p;
-					if (j >= n) continue;
-					const int j1 = min(j + 1, n - 1);
-					ok = ok && wait_word(src + j, want, w0[i]) && wait_word(src + j1, want, w1[i]);
-					float4 c = word_position(w1[i]);
-					if (j + 1 >= n) c = make_float4(FAR_PAD, FAR_PAD, FAR_PAD, 0.f);
-					set_pair(cols, p, word_position(w0[i]), c);
-					if (lo_here) {
-						ok = ok && wait_word(src + words + j, want, l0[i]) &&
-							wait_word(src + words + j1, want, l1[i]);
-						float4 cl = word_position(l1[i]);
-						if (j + 1 >= n) cl = make_float4(0.f, 0.f, 0.f, 0.f);
-						set_pair(colslo, p, word_position(l0[i]), cl);
-					}
+				ok = ok && wait_word(src + j, want, w0) && wait_word(src + j1, want, w1);
+				float4 c = word_position(w1);
+				if (j + 1 >= n) c = make_float4(FAR_PAD, FAR_PAD, FAR_PAD, 0.f);
+				set_pair(cols, p, word_position(w0), c);
+				if (lo_here) {
+					ok = ok && wait_word(src + words + j, want, l0) && wait_word(src + words + j1, want, l1);
+					c = word_position(l1);
+					if (j + 1 >= n) c = make_float4(0.f, 0.f, 0.f, 0.f);
+					set_pair(colslo, p, word_position(l0), c);
 				}
 			}
 		}
@@ -612,11 +611,14 @@ const void* steps_fn(int kind)
 
 }  // namespace
 
-// Rows per CTA: up to 64 bodies one CTA; up to 512 at most 16 CTAs (one cluster); above, one
-// CTA per SM, whole groups of 4 rows.
-int steps_rows(int n, int sms)
+// Rows per CTA: few bodies one CTA; up to 512 at most 16 CTAs (one cluster); above, one CTA per
+// SM, whole groups of 4 rows.  One CTA needs no exchange, but from 41 rows on two warps of a
+// scheduler share its FP64 unit: a step of a long launch takes 1.65 us at 17 bodies, 1.92 at 48
+// and 2.19 at 64 in one CTA, 1.95 in a cluster at any of them.  A cluster's launch costs 1.4 us
+// more, which eight steps of 64 bodies win back.
+int steps_rows(int n, int sms, int steps)
 {
-	if (n <= 64) return 64;
+	if (n <= 48 || (n <= 64 && steps < 8)) return 64;
 	const int ctas = n <= 512 ? static_cast<int>(ST_CLUSTER_MAX) : sms;
 	return (n + ST_RG * ctas - 1) / (ST_RG * ctas) * ST_RG;
 }
@@ -627,7 +629,7 @@ bool steps_supported(int mode, int n, int sms)
 {
 	const int kind = steps_kind(mode);
 	if (kind < 0 || n < 1 || sms < 1 || n > ST_MAX_ROWS * sms) return false;
-	const int R = steps_rows(n, sms);
+	const int R = steps_rows(n, sms, 1);
 	return R <= ST_MAX_ROWS && StepsSmem(kind, n, R).bytes <= ST_SMEM_MAX;
 }
 
@@ -643,7 +645,7 @@ cudaError_t launch_steps(const grav_batch& b, int flags, int steps, int64_t a_st
 	const int n = static_cast<int>(b.n_bodies);
 	const int kind = steps_kind(b.mode);
 	const void* fn = steps_fn(kind);
-	int R = steps_rows(n, sms);
+	int R = steps_rows(n, sms, steps);
 	const int smem = StepsSmem(kind, n, R).bytes;
 	cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 	if (e != cudaSuccess) return e;

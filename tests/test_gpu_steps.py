@@ -1,5 +1,5 @@
 """GPU tests of many steps of one universe in one launch (grav_steps, steps.cu): one CTA (up
-to 64 bodies), one cluster (up to 512) and one CTA per SM, at the edges of its row groups,
+to 48 bodies, 64 for fewer than eight steps), one cluster (up to 512) and one CTA per SM, at the edges of its row groups,
 column blocks and grids.
 
   - the accelerations of every step against the FP64 oracle on that step's own state,
@@ -83,7 +83,7 @@ def test_steps_against_oracle(gpu, mode, n):
                                     ('fp32n', 12288), ('fp32c', 6144), ('fp32un', 5000),
                                     ('fp32cu', 4999)])
 def test_steps_large(gpu, mode, n):
-    """Near the largest sizes: with and without the low parts in shared memory."""
+    """Near the largest sizes."""
     check_steps(mode, n, 2)
 
 
@@ -130,3 +130,42 @@ def test_forces_leave_the_state(gpu, mode, n):
     assert all(torch.equal(x, y) for x, y in zip(before, (eng.r, eng.v, eng.pos)))
     scale = torch.tensor(magnitudes(r, G_DEFAULT * m), device=a.device)
     assert float(((a - b).norm(dim=1) / scale).max()) < 2e-5
+
+
+@pytest.mark.parametrize('mode', MODES)
+@pytest.mark.parametrize('n', [48, 49, 57, 64])
+def test_steps_one_cta_or_cluster(gpu, mode, n):
+    """Eight steps of 49 to 64 bodies run in a cluster, fewer in one CTA: the same bits."""
+    check_steps(mode, n, 8)
+    r, v, m = planted(n, 9)
+    one, two = (Engine([n], 1e3, mode=mode) for _ in range(2))
+    for e in (one, two):
+        e.set_state(r, v, G_DEFAULT * m)
+    one.step(8)
+    two.step(7)
+    two.step(1)
+    torch.cuda.synchronize()
+    assert torch.equal(one.r, two.r) and torch.equal(one.v, two.v) and torch.equal(one.pos, two.pos)
+
+
+@pytest.mark.parametrize('n', [48, 64, 500, 1000])
+def test_steps_clump(gpu, n):
+    """40 bodies within 1e-3 of one another at |x| ~ 1000: a lane meets several near pairs in
+    one block of columns, with both of its rows and both columns of a packed pair."""
+    r, v, m = uniform_cube(n, seed=n)
+    rng = np.random.default_rng(n)
+    r[n // 5:n // 5 + 38] = np.array([990.0, -985.0, 991.0]) + rng.uniform(-1e-3, 1e-3, (38, 3))
+    r[[0, n - 1]] = r[n // 5] + np.array([[5e-4, 3e-4, 0.0], [-2e-4, 0.0, 4e-4]])
+    gm = G_DEFAULT * m
+    eng = Engine([n], 1.0, mode='fp32n')
+    eng.set_state(r, v, gm)
+    acc = torch.zeros((2, n, 4), dtype=torch.float64, device=eng.device)
+    eng.steps_to(acc)
+    torch.cuda.synchronize()
+    eng.raise_on_device_error()
+    acc = acc.cpu().numpy()
+    for k in range(2):
+        ref = oracle.accel_fp64(r, gm, 1.0, coincident=True)
+        err = np.linalg.norm(acc[k, :, :3] - ref, axis=1)
+        assert np.all(err <= TOL * magnitudes(r, gm)), (n, k)
+        r, v = oracle.stage2_fp64(r, v, acc[k, :, :3], 1.0)
