@@ -152,6 +152,10 @@ _DECLS = {
     'grav_adjoint_occupancy': (ctypes.c_int, [ctypes.c_int, _P(Tile), _P(ctypes.c_int32)]),
     'grav_adjoint_prepare': (ctypes.c_int, [_P(Adjoint), ctypes.c_void_p]),
     'grav_adjoint_step': (ctypes.c_int, [_P(Adjoint), ctypes.c_void_p]),
+    'grav_adjoint_steps_supported': (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32]),
+    'grav_adjoint_steps_scratch_bytes': (ctypes.c_int64, [ctypes.c_int32]),
+    'grav_adjoint_steps': (ctypes.c_int, [_P(Adjoint), ctypes.c_int32, ctypes.c_int64,
+                                          ctypes.c_void_p, ctypes.c_void_p]),
     'grav_forces_noalloc': (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32,
                                            ctypes.c_double, ctypes.c_void_p, ctypes.c_void_p]),
 }

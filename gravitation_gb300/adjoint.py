@@ -70,13 +70,15 @@ class AdjointEngine:
     pairs: True -- the unique-pair backward kernel (each unordered pair once, plan of
     grav_plan_pairs); False -- every ordered pair (plan of grav_plan); None -- by size.
     tile: (bpt, threads, jtile) of that kernel, default by size, optionally with a fourth
-    entry, the persistent grid (default: SMs x resident CTAs)."""
+    entry, the persistent grid (default: SMs x resident CTAs).  chained: steps() runs many
+    backward steps in one launch (one universe, neither pairs nor tile given)."""
 
     def __init__(self, sizes, T, device=None, tile=None, pairs=None):
         self.lib = _lib.load()
         self.dev_info = device_info(device)
         self.device = torch.device('cuda', self.dev_info.index)
         self.sizes = [int(n) for n in sizes]
+        by_size = pairs is None and tile is None
         if pairs is None:
             pairs = default_adjoint_pairs(self.sizes)
         self.pairs = bool(pairs)
@@ -125,6 +127,14 @@ class AdjointEngine:
         a.a_in = None
         self.adj = a
         self._aref = ctypes.byref(a)
+        self.scratch = None
+        # a backward step takes 2.2 us in a chain of 64 bodies, 3.9 at 1000, 20.0 at 4096 and
+        # 52 at 6900 (the largest that fits); with two launches 13.3, 13.8, 22.9 and 55
+        self.chained = by_size and len(self.sizes) == 1 and bool(
+            self.lib.grav_adjoint_steps_supported(self.sizes[0], self.dev_info.sm_count))
+        if self.chained:
+            self.scratch = torch.zeros(self.lib.grav_adjoint_steps_scratch_bytes(self.sizes[0]),
+                                       dtype=torch.uint8, device=dev)
 
     def _h(self, stream):
         s = stream if stream is not None else torch.cuda.current_stream(self.device)
@@ -145,6 +155,20 @@ class AdjointEngine:
         self.adj.a_in = None if a_in is None else a_in.data_ptr()
         try:
             check(self.lib.grav_adjoint_step(self._aref, self._h(stream)))
+        finally:
+            self.adj.a_in = None
+
+    def steps(self, a_in, stream=None):
+        """Backward steps over the forward's accelerations a_in (float64 [steps, n_bodies, 4],
+        in forward order: the last is reversed first), in one launch where self.chained."""
+        if not self.chained or len(a_in) < 2 or not a_in.is_contiguous():
+            for a in reversed(a_in):
+                self.step(stream, a_in=a)
+            return
+        self.adj.a_in = a_in[-1].data_ptr()
+        try:
+            check(self.lib.grav_adjoint_steps(self._aref, len(a_in), -a_in.stride(0),
+                                              self.scratch.data_ptr(), self._h(stream)))
         finally:
             self.adj.a_in = None
 
@@ -245,8 +269,11 @@ class Rollout:
         with torch.cuda.stream(self.fwd._stream(stream)):
             a.set_state(self.ck_r[si + 1], self.ck_v[si + 1])
         a.prepare(stream)
-        for k in reversed(range(s0, s1)):
-            a.step(stream, a_in=self.acc[k] if self.store_a else None)
+        if self.store_a:
+            a.steps(self.acc[s0:s1], stream)
+        else:
+            for _ in range(s0, s1):
+                a.step(stream)
 
     def forward(self, r0, v0, gm, stream=None):
         """Run the steps; keep the FP64 state at the start of every segment.

@@ -554,3 +554,37 @@ extern "C" int grav_adjoint_step(const grav_adjoint* a, void* stream)
 	cudaError_t e = grav::launch_adjoint_stage2(copy, *a, ADJ_STEP | ADJ_PREPARE, fa ? 7 : 4, st);
 	return e == cudaSuccess ? GRAV_OK : grav::record_error(GRAV_E_CUDA, cudaGetErrorString(e));
 }
+
+extern "C" int grav_adjoint_steps_supported(int32_t n, int32_t sm_count)
+{
+	return grav::adjoint_steps_supported(n, sm_count) ? 1 : 0;
+}
+
+extern "C" int64_t grav_adjoint_steps_scratch_bytes(int32_t n)
+{
+	if (n < 0) return grav::record_error(GRAV_E_ARG, "n < 0");
+	return grav::adjoint_steps_scratch(n);
+}
+
+extern "C" int grav_adjoint_steps(const grav_adjoint* a, int32_t steps, int64_t a_stride,
+	void* scratch, void* stream)
+{
+	int rc = check_adj(a);
+	if (rc) return rc;
+	const grav_batch& b = *a->b;
+	if (b.n_univ != 1) return grav::record_error(GRAV_E_ARG, "grav_adjoint_steps takes one universe");
+	if (steps < 0) return grav::record_error(GRAV_E_ARG, "steps < 0");
+	if (!scratch) return grav::record_error(GRAV_E_ARG, "scratch is NULL");
+	if (!a->a_in) return grav::record_error(GRAV_E_ARG, "grav_adjoint_steps needs the accelerations (a_in)");
+	if (b.n_bodies == 0 || steps == 0) return GRAV_OK;
+	// one step alone overwrites the positions it reads, which only two launches keep apart
+	if (steps == 1) return grav_adjoint_step(a, stream);
+	int dev = 0, sms = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+	if (e != cudaSuccess) return grav::record_error(GRAV_E_CUDA, cudaGetErrorString(e));
+	if (b.n_bodies > INT32_MAX || !grav::adjoint_steps_supported(static_cast<int>(b.n_bodies), sms))
+		return grav::record_error(GRAV_E_SIZE, "grav_adjoint_steps does not take this many bodies");
+	e = grav::launch_adjoint_steps(b, *a, steps, a_stride, scratch, sms, static_cast<cudaStream_t>(stream));
+	return e == cudaSuccess ? GRAV_OK : grav::record_error(GRAV_E_CUDA, cudaGetErrorString(e));
+}

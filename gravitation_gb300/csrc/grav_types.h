@@ -44,6 +44,12 @@ int64_t steps_scratch(int n);
 cudaError_t launch_steps(const grav_batch& b, int flags, int steps, int64_t a_stride, void* scratch,
 	int sms, cudaStream_t stream);
 
+// K backward steps of one universe in one launch (adjoint_steps.cu).
+bool adjoint_steps_supported(int n, int sms);
+int64_t adjoint_steps_scratch(int n);
+cudaError_t launch_adjoint_steps(const grav_batch& b, const grav_adjoint& a, int steps,
+	int64_t a_stride, void* scratch, int sms, cudaStream_t stream);
+
 // Kernel tables, one per translation unit (stage1_f32.cu, stage1_f64.cu).
 int stage1_table_f32(const Stage1Kernel** out);
 int stage1_table_f64(const Stage1Kernel** out);

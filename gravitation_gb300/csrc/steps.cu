@@ -45,7 +45,7 @@
 // low parts are not kept in shared memory (unless one CTA holds every row): the few that near
 // pairs need come from the exchange buffer, and the exchange moves half the bytes (14.0 to
 // 12.6 us at 4096).
-#include "grav_device.cuh"
+#include "exchange.cuh"
 
 namespace grav {
 
@@ -59,73 +59,6 @@ constexpr int ST_SEG = 32;           // blocks between two passes over the near 
 constexpr int ST_RPW = 10;           // rows whose state one warp holds (3 lanes each)
 constexpr int ST_MAX_ROWS = ST_RPW * ST_W;
 constexpr int ST_SMEM_MAX = 227 * 1024;
-constexpr unsigned ST_CLUSTER_MAX = 16;
-constexpr unsigned ST_CLUSTER_PORTABLE = 8;
-
-// Head of the scratch buffer; the two position buffers (hi, then lo, `rows` 16-byte words
-// each) follow at ST_HEAD_BYTES.
-struct StepsHead {
-	uint32_t epoch;     // tags used so far
-	int32_t departed;   // CTAs done with the launch
-};
-constexpr int ST_HEAD_BYTES = 128;
-
-typedef unsigned __int128 u128;
-
-__device__ __forceinline__ u128 load_word(const void* p)
-{
-	u128 v;
-	asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(v) : "l"(p) : "memory");
-	return v;
-}
-
-__device__ __forceinline__ void store_word(void* p, float x, float y, float z, uint32_t tag)
-{
-	const u64 lo = static_cast<u64>(__float_as_uint(y)) << 32 | __float_as_uint(x);
-	const u64 hi = static_cast<u64>(tag) << 32 | __float_as_uint(z);
-	const u128 v = static_cast<u128>(hi) << 64 | lo;
-	asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(v) : "memory");
-}
-
-__device__ __forceinline__ uint32_t word_tag(u128 v) { return static_cast<uint32_t>(v >> 96); }
-
-__device__ __forceinline__ float4 word_position(u128 v)
-{
-	return make_float4(__uint_as_float(static_cast<uint32_t>(v)),
-		__uint_as_float(static_cast<uint32_t>(v >> 32)),
-		__uint_as_float(static_cast<uint32_t>(v >> 64)), 0.f);
-}
-
-// Poll one published position until its tag is `tag`; false when the bounded wait expired.
-__device__ __forceinline__ bool wait_word(const void* p, uint32_t tag, u128& v)
-{
-	if (word_tag(v) == tag) return true;
-	const uint64_t t0 = global_ns();
-	for (;;) {
-		for (int k = 0; k < 64; ++k) {
-			v = load_word(p);
-			if (word_tag(v) == tag) return true;
-		}
-		if (global_ns() - t0 > GRAV_WAIT_NS) return false;
-	}
-}
-
-__device__ __forceinline__ void steps_cluster_arrive()
-{
-	asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void steps_cluster_wait()
-{
-	asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ unsigned steps_cluster_ctas()
-{
-	unsigned v;
-	asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(v));
-	return v;
-}
 
 // Shared memory of one CTA for n bodies and R rows per CTA (byte offsets, 16-byte units).
 struct StepsSmem {
@@ -188,7 +121,7 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 	const int n = static_cast<int>(b.n_bodies);
 	const int G = gridDim.x;
 	const bool multi = G > 1;
-	const bool clustered = multi && steps_cluster_ctas() == static_cast<unsigned>(G);
+	const bool clustered = multi && cluster_ctas() == static_cast<unsigned>(G);
 	const int row0 = blockIdx.x * R;
 	const int rows_here = max(0, min(R, n - row0));
 	const int NB = (n + ST_CB - 1) / ST_CB;
@@ -205,9 +138,9 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 	float* const red = reinterpret_cast<float*>(steps_smem + L.red);
 	const bool lo_here = L.lo_here;
 
-	StepsHead* const head = reinterpret_cast<StepsHead*>(scratch);
+	ExchangeHead* const head = reinterpret_cast<ExchangeHead*>(scratch);
 	const int64_t words = static_cast<int64_t>(NB) * ST_CB;   // per array and buffer
-	float4* const xbuf = reinterpret_cast<float4*>(scratch + ST_HEAD_BYTES);  // [2][hi, lo][words]
+	float4* const xbuf = reinterpret_cast<float4*>(scratch + EXCHANGE_HEAD_BYTES);  // [2][hi, lo][words]
 	const double Tu = b.univ[0].T;
 
 	// this warp's units [u0, u1) of the CTA's NG x NB
@@ -461,7 +394,7 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 		// done with them, else the last CTA out copies them over (with more steps, each CTA has
 		// by now read every other CTA's later ones)
 		const bool settle = integrate && clustered && K == 1;
-		if (settle) steps_cluster_arrive();
+		if (settle) cluster_arrive();
 
 		// ---- stage 2 of this lane's row component ----
 		if (warp_rows) {
@@ -490,7 +423,7 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 					store_word(xbuf + ((k & 1) * 2 + 1) * words + row0 + rl, lx, ly, lz, tag0 + k);
 				if (last) {
 					// ---- the launch's results: state and stage-1 positions ----
-					if (settle) steps_cluster_wait();
+					if (settle) cluster_wait();
 					if (mine) {
 						rd[e] = rr;
 						vd[e] = vv;
@@ -520,7 +453,7 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 				if (rc == 2) __stcs(ao + 1, 0.0);
 			}
 		} else if (settle) {
-			steps_cluster_wait();
+			cluster_wait();
 		}
 
 		// ---- every body's new position ----
@@ -619,7 +552,7 @@ const void* steps_fn(int kind)
 int steps_rows(int n, int sms, int steps)
 {
 	if (n <= 48 || (n <= 64 && steps < 8)) return 64;
-	const int ctas = n <= 512 ? static_cast<int>(ST_CLUSTER_MAX) : sms;
+	const int ctas = n <= 512 ? static_cast<int>(EXCHANGE_CLUSTER_MAX) : sms;
 	return (n + ST_RG * ctas - 1) / (ST_RG * ctas) * ST_RG;
 }
 
@@ -636,7 +569,7 @@ bool steps_supported(int mode, int n, int sms)
 int64_t steps_scratch(int n)
 {
 	const int64_t words = (static_cast<int64_t>(n) + ST_CB - 1) / ST_CB * ST_CB;
-	return ST_HEAD_BYTES + 4 * words * 16;
+	return EXCHANGE_HEAD_BYTES + 4 * words * 16;
 }
 
 cudaError_t launch_steps(const grav_batch& b, int flags, int steps, int64_t a_stride, void* scratch,
@@ -647,52 +580,13 @@ cudaError_t launch_steps(const grav_batch& b, int flags, int steps, int64_t a_st
 	const void* fn = steps_fn(kind);
 	int R = steps_rows(n, sms, steps);
 	const int smem = StepsSmem(kind, n, R).bytes;
-	cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-	if (e != cudaSuccess) return e;
 	const unsigned grid = static_cast<unsigned>((n + R - 1) / R);
 	grav_batch copy = b;
 	int f = flags, K = steps;
 	unsigned char* s = static_cast<unsigned char*>(scratch);
 	void* args[] = {&copy, &f, &K, &a_stride, &R, &s};
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3(grid);
-	cfg.blockDim = dim3(ST_T);
-	cfg.dynamicSmemBytes = static_cast<size_t>(smem);
-	cfg.stream = stream;
-	cudaLaunchAttribute attr[2];
-	cfg.attrs = attr;
-	cfg.numAttrs = 0;
 	const bool integrate = grid > 1 && (flags & GRAV_S2_INTEGRATE);
-	const bool waits = integrate && steps > 1;
-	bool cluster = integrate && grid <= ST_CLUSTER_MAX;
-	if (cluster) {
-		attr[0].id = cudaLaunchAttributeClusterDimension;
-		attr[0].val.clusterDim.x = grid;
-		attr[0].val.clusterDim.y = 1;
-		attr[0].val.clusterDim.z = 1;
-		cfg.numAttrs = 1;
-		if (grid > ST_CLUSTER_PORTABLE) {
-			int fits = 0;
-			e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-			if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fits, fn, &cfg);
-			if (e != cudaSuccess) {
-				cudaGetLastError();  // a refused query is not sticky: fall back
-				fits = 0;
-			}
-			cluster = fits > 0;
-			if (!cluster) cfg.numAttrs = 0;
-		}
-	}
-	if (waits && !cluster) {
-		attr[0].id = cudaLaunchAttributeCooperative;
-		attr[0].val.cooperative = 1;
-		cfg.numAttrs = 1;
-	} else {
-		attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-		attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
-		++cfg.numAttrs;
-	}
-	return cudaLaunchKernelExC(&cfg, fn, args);
+	return launch_exchanging(fn, grid, ST_T, smem, integrate, integrate && steps > 1, stream, args);
 }
 
 }  // namespace grav

@@ -347,6 +347,27 @@ int grav_adjoint_prepare(const grav_adjoint* a, void* stream);
  */
 int grav_adjoint_step(const grav_adjoint* a, void* stream);
 
+/* 1 if grav_adjoint_steps takes one universe of n bodies on a GPU of sm_count SMs, else 0:
+ * every CTA holds all positions and u in shared memory (up to ~7k bodies). */
+int grav_adjoint_steps_supported(int32_t n, int32_t sm_count);
+
+/* Bytes of device scratch grav_adjoint_steps needs for n bodies: zeroed once by the caller,
+ * then left alone between calls (it numbers the exchanged words). */
+int64_t grav_adjoint_steps_scratch_bytes(int32_t n);
+
+/*
+ * `steps` backward steps of a batch holding one universe in one launch, as that many
+ * grav_adjoint_step calls with the accelerations kept: step i reverses with the rows at
+ * a->a_in + i * a_stride (doubles; negative for accelerations kept in forward order).  The
+ * pair arithmetic is grav_adjoint_step's over ordered pairs, summed in another order: results
+ * agree to FP32 rounding of the partial sums.  Positions and u (b->pos, a->upos) are read as
+ * grav_adjoint_prepare or a step left them; the state and gradients are read at the start and
+ * written at the end of the launch, b->pos and a->upos prepared for a further step.  Co-scheduled
+ * and bounded like grav_steps: after 2 s of waiting it sets GRAV_DEV_TIMEOUT in b->err.
+ */
+int grav_adjoint_steps(const grav_adjoint* a, int32_t steps, int64_t a_stride, void* scratch,
+	void* stream);
+
 /* ---- allocation-free variant ------------------------------------------------------- */
 
 /* Largest universe grav_forces_noalloc accepts. */

@@ -432,3 +432,14 @@ def test_steps_rejects_bad_calls_on_host(L):
     assert L.grav_steps(bb, 1, 0, 0, scratch, None) == _lib.GRAV_OK           # no steps
     b.n_univ = 2
     assert L.grav_steps(bb, 1, 1, 0, scratch, None) == _lib.GRAV_E_ARG
+
+
+def test_adjoint_steps_rejects_bad_calls_on_host():
+    lib = _lib.load()
+    assert [lib.grav_adjoint_steps_supported(n, 152) for n in (0, 1, 512, 513, 6900, 9000)] == [
+        0, 1, 1, 1, 1, 0]
+    assert lib.grav_adjoint_steps_scratch_bytes(65) == 128 + 5 * 128 * 16
+    assert lib.grav_adjoint_steps_scratch_bytes(-1) < 0
+    assert lib.grav_adjoint_steps(None, 2, 0, None, None) == _lib.GRAV_E_ARG
+    a = _lib.Adjoint()
+    assert lib.grav_adjoint_steps(ctypes.byref(a), 2, 0, ctypes.c_void_p(16), None) == _lib.GRAV_E_ARG
