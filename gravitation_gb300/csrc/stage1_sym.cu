@@ -71,7 +71,10 @@ struct SymSmem {
 	static constexpr int CSUM = EX + 2 * EX_TILE * 16;            // [3][B][T] float2
 	static constexpr int COL = CSUM + 3 * B * T * 8;              // [2][W][3][JT] float
 	static constexpr int ROWLO = COL + 2 * W * 3 * JT * 4;        // [B][T] float4 (SYM_NEAR)
-	static constexpr int BYTES = ROWLO + (KIND == SYM_NEAR ? B * T * 16 : 0);
+	// near pairs gone through once per j-tile, lane by lane, rather than once per chunk and step
+	static constexpr bool BY_LANE = KIND == SYM_NEAR && B >= 8 && JT <= 128;
+	static constexpr int MASK = ROWLO + (KIND == SYM_NEAR ? B * T * 16 : 0);   // [JT / 32][T] uint32 (BY_LANE)
+	static constexpr int BYTES = MASK + (BY_LANE ? JT / 32 * T * 4 : 0);
 };
 
 // Column sums of the j-tile `jt` (block J > I) -> column slot of (I, J), the warps added in
@@ -111,8 +114,8 @@ __device__ __forceinline__ void fold_pair(float2* sums, int T, u64 f)
 
 // The near correction of one column body (pj, low part lj) against a thread's rows: pairs
 // closer than the near radius again, from the double-single separation, the difference
-// added to the rows' sums f and (COLS) the rows' column terms, Gm_i e, to q.  Warp-uniform:
-// every lane calls it with its own body and the votes keep the lanes together.
+// added to the rows' sums f and (COLS) the rows' column terms, Gm_i e, to q.  Every lane of
+// the warp calls it, with a body and a radius thr of its own (0: none).
 template <int H, int T, bool COLS>
 __device__ __forceinline__ void near_rows(const float4& pj, const float4& lj, float eps2, float thr,
 	const u64 (&nx)[H], const u64 (&ny)[H], const u64 (&nz)[H], const u64 (&g2)[H],
@@ -121,13 +124,23 @@ __device__ __forceinline__ void near_rows(const float4& pj, const float4& lj, fl
 {
 	const u64 px = pack2(pj.x, pj.x), py = pack2(pj.y, pj.y), pz = pack2(pj.z, pj.z);
 	const u64 pw = pack2(pj.w, pj.w), eps22 = pack2(eps2, eps2);
+	uint32_t rows = 0;   // bit k: row k of this lane is near
 #pragma unroll
 	for (int h = 0; h < H; ++h) {
 		const u64 dx = add2(px, nx[h]), dy = add2(py, ny[h]), dz = add2(pz, nz[h]);
 		float ra, rb;
 		unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
-		const bool na = (ra < thr) & (ra > eps2), nb = (rb < thr) & (rb > eps2);
-		if (__any_sync(0xffffffffu, na | nb)) {
+		if ((ra < thr) & (ra > eps2)) rows |= 1u << (2 * h);
+		if ((rb < thr) & (rb > eps2)) rows |= 2u << (2 * h);
+	}
+	const uint32_t any = __reduce_or_sync(0xffffffffu, rows);
+#pragma unroll
+	for (int h = 0; h < H; ++h) {
+		if (any >> (2 * h) & 3u) {
+			const u64 dx = add2(px, nx[h]), dy = add2(py, ny[h]), dz = add2(pz, nz[h]);
+			float ra, rb;
+			unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
+			const bool na = rows >> (2 * h) & 1u, nb = rows >> (2 * h) & 2u;
 			float x0, x1, y0, y1, z0, z1, ex0, ey0, ez0, ex1, ey1, ez1;
 			unpack2(dx, x0, x1);
 			unpack2(dy, y0, y1);
@@ -146,6 +159,14 @@ __device__ __forceinline__ void near_rows(const float4& pj, const float4& lj, fl
 			}
 		}
 	}
+}
+
+// This lane's next step with a near pair, taken out of its mask (bit 31 - st: step st).
+__device__ __forceinline__ int next_step(uint32_t& mask)
+{
+	const int st = __clz(mask) & 31;
+	mask &= ~(0x80000000u >> st);
+	return st;
 }
 
 // Expand a j-tile for the packed loops: every coordinate twice in a 64-bit pair, (x, x | y, y)
@@ -193,6 +214,7 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 	constexpr int NP = L::NP;                       // position arrays copied per j-tile
 	constexpr bool DS = KIND == SYM_DS;             // double-single separations everywhere
 	constexpr bool NEAR = KIND == SYM_NEAR;         // double-single for near pairs only
+	constexpr bool BY_LANE = L::BY_LANE;
 	static_assert(B % 2 == 0 && R % JT == 0 && JT % 32 == 0 && (NCH & (NCH - 1)) == 0, "tile shapes");
 	extern __shared__ __align__(128) unsigned char sym_smem[];
 	float4* const raw = reinterpret_cast<float4*>(sym_smem + L::RAW);
@@ -205,6 +227,8 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 	float* const colacc = reinterpret_cast<float*>(sym_smem + L::COL);
 	// low parts of this thread's rows (NEAR), read back on the cold path only
 	float4* const rowlo = reinterpret_cast<float4*>(sym_smem + L::ROWLO) + threadIdx.x;  // [k]: k * T
+	// steps of each chunk that met near pairs, this thread's (BY_LANE)
+	uint32_t* const masks = reinterpret_cast<uint32_t*>(sym_smem + L::MASK) + threadIdx.x;  // [cc]: cc * T
 	__shared__ __align__(8) uint64_t bar[2];
 
 	const int tid = threadIdx.x;
@@ -372,16 +396,15 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 							fy[h] = fma2(dy, w, fy[h]);
 							fz[h] = fma2(dz, w, fz[h]);
 						}
-						if (NEAR && near) nmask |= 1u << j;
+						if (NEAR && near) nmask |= 0x80000000u >> j;
 					}
 					if (NEAR) {
-						uint32_t todo = __reduce_or_sync(0xffffffffu, nmask);
-						while (todo) {
-							const int j = __ffs(todo) - 1;
-							todo &= todo - 1;
+						while (__any_sync(0xffffffffu, nmask != 0u)) {
+							const float radius = nmask ? thr : 0.f;
+							const int j = ch * 32 + next_step(nmask);
 							float qx = 0.f, qy = 0.f, qz = 0.f;
-							near_rows<H, T, false>(sj[ch * 32 + j], sjl[ch * 32 + j], eps2, thr, nx, ny, nz,
-								g2, rowlo, fx, fy, fz, qx, qy, qz);
+							near_rows<H, T, false>(sj[j], sjl[j], eps2, radius, nx, ny, nz, g2, rowlo, fx, fy, fz,
+								qx, qy, qz);
 						}
 					}
 				}
@@ -389,6 +412,7 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 			} else {
 				// unique pairs with block J > I: rotate the chunk's column sums
 				float* __restrict__ cw = colacc + (bs * W + warp) * 3 * JT;
+				uint32_t met = 0;   // BY_LANE: this lane's steps with near pairs, any chunk
 #pragma unroll 1
 				for (int cc = 0; cc < NCH; ++cc) {
 					const int ch = (cc + warp) & (NCH - 1);
@@ -464,18 +488,20 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 						unpack2(cz, a0, a1);
 						sz = a0 + a1;
 					}
-					if (NEAR) {
-						// cold path: the steps that met pairs closer than the near radius again,
-						// from the double-single separation; their column terms belong to the
-						// body the lane met then, whose sum lane (lane + st) mod 32 now holds
+					if (BY_LANE) {
+						masks[cc * T] = nmask;
+						met |= nmask;
+					} else if (NEAR) {
+						// cold path: the steps that met near pairs again, every lane with the body it met
+						// then; their column terms belong to that body, whose sum lane (lane + st) mod 32
+						// now holds
 						uint32_t todo = __reduce_or_sync(0xffffffffu, nmask);
 						while (todo) {
-							const int st = __clz(todo);
-							todo &= ~(0x80000000u >> st);
-							const int jb = ch * 32 + ((lane + st) & 31);
+							const int st = next_step(todo);
+							const int j = ch * 32 + ((lane + st) & 31);
 							float qx = 0.f, qy = 0.f, qz = 0.f;
-							near_rows<H, T, true>(sj[jb], sjl[jb], eps2, thr, nx, ny, nz, g2, rowlo, fx, fy,
-								fz, qx, qy, qz);
+							near_rows<H, T, true>(sj[j], sjl[j], eps2, thr, nx, ny, nz, g2, rowlo, fx, fy, fz, qx,
+								qy, qz);
 							const int from = (lane - st) & 31;
 							sx += __shfl_sync(0xffffffffu, qx, from);
 							sy += __shfl_sync(0xffffffffu, qy, from);
@@ -485,6 +511,34 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 					cw[ch * 32 + lane] = -sx;
 					cw[JT + ch * 32 + lane] = -sy;
 					cw[2 * JT + ch * 32 + lane] = -sz;
+				}
+				if (BY_LANE && __any_sync(0xffffffffu, met != 0u)) {
+					// cold path, once per tile: each lane's own steps that met near pairs, all lanes
+					// side by side; the column terms go to the body met, lanes that met the same one
+					// in turn
+					__syncwarp();
+					int cc = 0;
+					uint32_t mask = masks[0];
+					for (;;) {
+						while (!mask && cc + 1 < NCH) mask = masks[++cc * T];
+						if (!__any_sync(0xffffffffu, mask != 0u)) break;
+						const float radius = mask ? thr : 0.f;
+						const int j = ((cc + warp) & (NCH - 1)) * 32 + ((lane + next_step(mask)) & 31);
+						float qx = 0.f, qy = 0.f, qz = 0.f;
+						near_rows<H, T, true>(sj[j], sjl[j], eps2, radius, nx, ny, nz, g2, rowlo, fx, fy, fz, qx,
+							qy, qz);
+						const uint32_t same = __match_any_sync(0xffffffffu, radius > 0.f ? j : JT + lane);
+						const unsigned turn = __popc(same & ((1u << lane) - 1u));
+						const unsigned turns = __reduce_max_sync(0xffffffffu, turn);
+						for (unsigned i = 0; i <= turns; ++i) {
+							if (turn == i && radius > 0.f) {
+								cw[j] -= qx;
+								cw[JT + j] -= qy;
+								cw[2 * JT + j] -= qz;
+							}
+							__syncwarp();
+						}
+					}
 				}
 				blk_done = blkJ;
 			}
@@ -534,14 +588,25 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 #define GRAV_SYMN_ENTRY(B, W, J, UN, MINB) GRAV_SYM_KERNEL(GRAV_MODE_FP32UN, SYM_NEAR, B, W, J, UN, MINB, B < 8)
 
 // UN (unrolling of the step loop) and MINB (the occupancy that ptxas must leave room for) as
-// measured per shape over 2, 4, 8 and 16 steps and the occupancies around each; no sum's order
+// measured per shape over 1 to 16 steps and the occupancies around each; no sum's order
 // depends on them.  Stage 1 at 65536 bodies, unrolled by 4 at the higher occupancy and as
 // compiled here:
-//   fp32un 8/64/64 1376 (6 CTAs, 168 registers, 8 bytes spilled) and 1352 us (4 CTAs, 200),
-//     at 16384 bodies 102 and 94; fp32un 8/64/128 1353 and 1326;
 //   fp32cu 8/64/64 1682 (6 CTAs, 165 registers) and 1580 us (4 CTAs, 194);
 //   fp32u 8/128/64 1297 and 1225, 8/64/64 1210 and 1200, at 16384 bodies 88 and 82.
-// Two warps per scheduler with every operand in registers beat three that reload some.
+// Two warps per scheduler with every operand in registers beat three that reload some.  16
+// rows per thread (fp32u) share a step's loads, shuffles and column additions: from 32768
+// bodies on 2-3 % faster than 8 (131072 bodies 4746 -> 4604 us), below slower, their blocks of
+// 1024 rows being too coarse.
+//
+// Near pairs (fp32un).  A chunk of 32 columns against a warp's rows of 8 holds 0.5 near pairs
+// in a cube at rest and 1.2 in a Gaussian cloud.  Going through the chunk's steps that met any,
+// the whole warp at each, is a chain of some 500 cycles that two warps per scheduler hide
+// badly; once per j-tile with every lane at its own steps it runs once or twice per tile.
+// Stage 1 at 65536 bodies, cube / cloud (without any near pass 1290 / 1290):
+//   8/128/128 1329 / 1401 -> 1311 / 1339 us, 8/64/128 1326 / 1385 -> 1320 / 1348,
+//   8/64/64 1352 / 1417 -> 1341 / 1374.
+// Rows of 4 meet half as many and keep the pass per chunk (4/256/256 1323 / 1341, by lane
+// 1366 / 1394), as does 8/128/256, whose second CTA per SM would not fit the masks.
 static const Stage1Kernel k_table_sym[] = {
 	GRAV_SYM_ENTRY(4, 4, 128, 4),
 	GRAV_SYM_ENTRY(4, 8, 256, 2),
@@ -553,6 +618,7 @@ static const Stage1Kernel k_table_sym[] = {
 	GRAV_SYM_ENTRY(8, 4, 64, 3),
 	GRAV_SYM_ENTRY(4, 2, 64, 8),
 	GRAV_SYM_ENTRY(8, 2, 64, 4),
+	GRAV_SYM_KERNEL(GRAV_MODE_FP32U, SYM_PLAIN, 16, 2, 64, 8, 4, false),
 	GRAV_SYMC_ENTRY(4, 4, 128, 16, 3),
 	GRAV_SYMC_ENTRY(8, 4, 256, 4, 1),
 	GRAV_SYMC_ENTRY(4, 4, 256, 16, 2),
@@ -563,11 +629,11 @@ static const Stage1Kernel k_table_sym[] = {
 	GRAV_SYMN_ENTRY(4, 4, 128, 8, 3),
 	GRAV_SYMN_ENTRY(8, 4, 256, 8, 2),
 	GRAV_SYMN_ENTRY(8, 4, 128, 8, 2),
-	GRAV_SYMN_ENTRY(8, 4, 64, 8, 2),
+	GRAV_SYMN_ENTRY(8, 4, 64, 1, 2),
 	GRAV_SYMN_ENTRY(4, 4, 256, 16, 2),
 	GRAV_SYMN_ENTRY(4, 8, 256, 16, 1),
 	GRAV_SYMN_ENTRY(4, 2, 64, 8, 7),
-	GRAV_SYMN_ENTRY(8, 2, 64, 4, 4),
+	GRAV_SYMN_ENTRY(8, 2, 64, 8, 4),
 	GRAV_SYMN_ENTRY(8, 2, 128, 8, 4),
 };
 

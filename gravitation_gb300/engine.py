@@ -163,7 +163,7 @@ def _ctypes_to_device(arr, nbytes, device):
 
 # SM time per pair of every compiled tile with three or more warps per scheduler (picoseconds;
 # an ordered pair of the all-pairs modes, an unordered one of the others), from stage 1 at
-# 65536 / 131072 bodies on GB300.
+# 65536 / 131072 bodies on GB300 (fp32un: the mean of a cube at rest and a Gaussian cloud).
 TILE_COST = {
     'fp32': {(1, 128, 128): 73, (2, 128, 128): 70, (4, 128, 128): 70, (4, 128, 256): 69,
              (8, 128, 256): 72, (2, 256, 256): 66, (4, 256, 256): 69, (8, 256, 256): 69},
@@ -172,10 +172,10 @@ TILE_COST = {
     'fp32c': {(1, 128, 128): 108, (2, 128, 128): 100, (4, 128, 256): 98, (4, 256, 256): 95},
     'fp32u': {(4, 128, 128): 87, (4, 256, 256): 85, (8, 128, 256): 64, (4, 128, 256): 71,
               (2, 256, 256): 101, (8, 256, 256): 63, (8, 128, 128): 81, (8, 128, 64): 85,
-              (4, 64, 64): 90, (8, 64, 64): 67},
-    'fp32un': {(4, 128, 128): 96, (8, 128, 256): 72, (8, 128, 128): 73, (8, 128, 64): 76,
-               (4, 128, 256): 76, (4, 256, 256): 73, (4, 64, 64): 100, (8, 64, 64): 75,
-               (8, 64, 128): 73},
+              (4, 64, 64): 90, (8, 64, 64): 67, (16, 64, 64): 64},
+    'fp32un': {(4, 128, 128): 97, (8, 128, 256): 74, (8, 128, 128): 73, (8, 128, 64): 77,
+               (4, 128, 256): 77, (4, 256, 256): 73, (4, 64, 64): 101, (8, 64, 64): 76,
+               (8, 64, 128): 74},
     'fp32cu': {(4, 128, 128): 114, (8, 128, 256): 57, (4, 128, 256): 61, (4, 256, 256): 88,
                (8, 128, 128): 86, (4, 64, 64): 118, (8, 64, 64): 88},
 }
@@ -185,8 +185,8 @@ def tile_time(mode, tile, info, sm_count, resident):
     """Estimated step time (us) of a plan: the busiest SM's units at the tile's cost, slower
     where fewer than three warps per scheduler are resident (half the rate with one, 0.8 with
     two), plus the slots' traffic in stage 2 (24 bytes per entry, written and read, at ~8
-    TB/s).  Over the unique-pair modes at 300-131072 bodies (42 measured sets of tiles) the
-    tile it picks ran within 0.3 % of the fastest on average, at worst 7 % (fp32cu at 6500
+    TB/s).  Over the unique-pair modes at 300-131072 bodies (56 measured sets of tiles) the
+    tile it picks ran within 0.2 % of the fastest on average, at worst 7 % (fp32cu at 6500
     bodies), over the all-pairs modes within 0.4 %; the rule before it, which did not count the CTAs that share an SM, was 5-30 %
     off above 8192 bodies."""
     grid = min(info.grid, info.n_units)
@@ -200,10 +200,11 @@ def tile_time(mode, tile, info, sm_count, resident):
             info.n_slots * info.itile * 24 / 8e6)
 
 
-# Longest j-tile the default picks: its FP32 partial sums run over one j-tile, and twice the
-# length is ~10 % more rms force error (fp32un at 65536 bodies: 1.22e-7 with 64-body tiles,
-# 1.51e-7 with 128, 2.4e-7 with 256) for 2 % of time.
+# Longest j-tile the default picks, and other shapes it may: FP32 partial sums run over one
+# j-tile.  rms force error of fp32un at 8191 / 65536 bodies: 4/64/64 1.3e-7 / 5.6e-8, 8/64/64
+# 1.5 / 7.5, 8/128/128 1.7 / 7.0, 8/64/128 1.7 / 8.0, 8/128/256 1.9 / 7.4.
 DEFAULT_JTILE_MAX = {'fp32u': 64, 'fp32un': 64}
+DEFAULT_ALSO = {'fp32un': [(8, 128, 128)]}
 
 
 def default_tile(mode, sizes, device=None):
@@ -213,7 +214,8 @@ def default_tile(mode, sizes, device=None):
     info = device_info(device)
     cands = fitting_tiles(sizes, mode) or tile_list(mode)
     longest = DEFAULT_JTILE_MAX.get(mode, 128)
-    cands = [t for t in cands if t.jtile <= longest] or cands
+    also = DEFAULT_ALSO.get(mode, ())
+    cands = [t for t in cands if t.jtile <= longest or t.key() in also] or cands
     best = None
     for t in cands:
         occ = occupancy(mode, t, device)
