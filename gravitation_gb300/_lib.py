@@ -127,6 +127,11 @@ _DECLS = {
     'grav_part_bytes': (ctypes.c_int64, [_P(PlanInfo)]),
     'grav_eps2': (ctypes.c_float, [ctypes.c_double]),
     'grav_prepare': (ctypes.c_int, [_P(Batch), ctypes.c_void_p]),
+    'grav_gm_range': (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
+                                     ctypes.c_void_p]),
+    'grav_load_state': (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
+                                       ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p,
+                                       ctypes.c_void_p]),
     'grav_stage1': (ctypes.c_int, [_P(Batch), ctypes.c_void_p]),
     'grav_stage2': (ctypes.c_int, [_P(Batch), ctypes.c_int, ctypes.c_void_p]),
     'grav_step': (ctypes.c_int, [_P(Batch), ctypes.c_int, ctypes.c_void_p]),

@@ -416,6 +416,10 @@ class Engine:
     def set_state(self, r, v, gm, stream=None):
         """Load positions, velocities and G*m (already scaled) for all bodies, packed."""
         n = self.info.n_bodies
+        if n and self.r.is_cuda and all(torch.is_tensor(x) and x.device == self.r.device
+                                        for x in (r, v, gm)):
+            self._load(r, v, gm, stream)
+            return
         r = torch.as_tensor(np.asarray(r, dtype=np.float64).reshape(n, 3) if not torch.is_tensor(r)
                             else r.reshape(n, 3), dtype=torch.float64)
         v = torch.as_tensor(np.asarray(v, dtype=np.float64).reshape(n, 3) if not torch.is_tensor(v)
@@ -431,6 +435,24 @@ class Engine:
             self.r[:n, 3].copy_(gm)
             self.v[:n, :3].copy_(v)
             self.v[:n, 3].zero_()
+        self.prepare(stream)
+
+    def _load(self, r, v, gm, stream):
+        """set_state from tensors on the engine's device: two launches and one wait."""
+        n = self.info.n_bodies
+        r, v, gm = (x.detach().reshape(shape).to(torch.float64).contiguous()
+                    for x, shape in ((r, (n, 3)), (v, (n, 3)), (gm, (n,))))
+        span = torch.empty(2, dtype=torch.float64, device=self.r.device)
+        check(self.lib.grav_gm_range(gm.data_ptr(), n, span.data_ptr(), self._h(None)))
+        max_gm, bad = span.tolist()
+        if bad:
+            raise ValueError('G*m must be finite and >= 0')
+        self.batch.eps2 = float(self.lib.grav_eps2(max_gm))
+        check(self.lib.grav_load_state(r.data_ptr(), v.data_ptr(), gm.data_ptr(), n,
+                                       self.r.data_ptr(), self.v.data_ptr(), self._h(stream)))
+        if stream is not None:
+            for x in (r, v, gm):
+                x.record_stream(stream)
         self.prepare(stream)
 
     def generate_state(self, scenarios, G, stream=None):

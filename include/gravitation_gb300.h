@@ -201,6 +201,16 @@ float grav_eps2(double max_gm);
 
 /* ---- stages (device work, asynchronous on `stream`) ---------------------------- */
 
+/* Range of n device values of G*m: out[0] (device) = the largest, 0 if none is above 0, out[1] =
+ * 0, or 1 if one is negative, infinite or NaN.  What a caller checks, and passes to grav_eps2,
+ * before grav_load_state. */
+int grav_gm_range(const double* gm, int64_t n, double* out, void* stream);
+
+/* Rows r4 = (x, y, z, G*m) and v4 = (vx, vy, vz, 0) from packed device arrays r, v (n x 3) and
+ * gm (n). */
+int grav_load_state(const double* r, const double* v, const double* gm, int64_t n, double* r4,
+	double* v4, void* stream);
+
 /* Refresh the padded stage-1 positions from r (after r was written by the host). */
 int grav_prepare(const grav_batch* b, void* stream);
 

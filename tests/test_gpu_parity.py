@@ -466,3 +466,32 @@ def test_precision_workload_short(gpu):
     for mode in ('fp32un', 'fp32u', 'fp64'):
         assert np.isfinite(out[mode]['energy_drift_max'])
         assert out[mode]['momentum_drift_max'] < 1e-9
+
+
+@pytest.mark.parametrize('n', [1, 63, 64, 65, 1000])
+def test_state_from_device_tensors(gpu, n):
+    """Device tensors (strided, single precision, on another stream) load the rows, eps2 and
+    positions that host arrays load, and the same G*m are refused before anything changes."""
+    rng = np.random.default_rng(n)
+    r, v = rng.normal(size=(n, 3)), rng.normal(size=(n, 3))
+    gm = rng.uniform(0.0, 1.0, n).astype(np.float32).astype(np.float64)
+    gm[0] = 0.0
+    host, dev = (Engine([n], 1.0, mode='fp32') for _ in range(2))
+    host.set_state(r, v, gm)
+    wide = torch.zeros((n, 5), dtype=torch.float64, device='cuda')
+    wide[:, 1:4] = torch.tensor(r)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    dev.set_state(wide[:, 1:4], torch.tensor(v, device='cuda'),
+                  torch.tensor(gm, dtype=torch.float32, device='cuda'), stream=side)
+    torch.cuda.synchronize()
+    assert torch.equal(host.r, dev.r) and torch.equal(host.v, dev.v)
+    assert torch.equal(host.pos, dev.pos) and host.batch.eps2 == dev.batch.eps2
+    before = dev.r.clone()
+    for bad in (-1e-300, float('nan'), float('inf')):
+        wrong = torch.tensor(gm, device='cuda')
+        wrong[n // 2] = bad
+        with pytest.raises(ValueError):
+            dev.set_state(wide[:, :3], wide[:, :3], wrong)
+    torch.cuda.synchronize()
+    assert torch.equal(before, dev.r)
