@@ -2,8 +2,8 @@
 //
 // One or TPR lanes per row of the padded position array.  For a real body they add the
 // partial-sum slots of its segment (each lane its share, in slot order, then a fixed
-// butterfly: deterministic), then lane 0 applies the base class's update in FP64 with
-// separately rounded products and sums,
+// butterfly: deterministic), then the base class's update is applied in FP64 with separately
+// rounded products and sums,
 //     v = a*T + v ;  r = v*T + r          (_base_.py:58-62, np2.py:110-115)
 // exactly as the reference's Python floats / numpy arrays round them, and finally
 // rewrites the row of the stage-1 position array (FP32 hi[, lo] or FP64).  Padding
@@ -22,6 +22,9 @@ struct __align__(32) drow4 {
 // of memory latency, and the lanes' partial sums are combined by a butterfly, which
 // gives every lane the same bits.  For large batches one lane per row: there the extra
 // lanes and their combining work cost more than the latency they hide.
+// A split row's update is split too, lane c taking component c: an FP64 warp instruction costs
+// 67 cycles of its scheduler whatever its active lanes, and one lane doing the whole row
+// issued 34 of them per 8 rows, 12 now (16384 bodies: prepared and integrated 11.1 -> 7.9 us).
 constexpr int S2_THREADS = 128;
 constexpr int SPLIT_ROWS_MAX = 32768;  // TPR = 4 up to this many padded rows, else 1
 constexpr int ROW_BATCH = 8;           // FP64 row-slot loads in flight per lane
@@ -73,14 +76,21 @@ __global__ void __launch_bounds__(S2_THREADS) stage2_kernel(const grav_batch b, 
 	drow4* rr = reinterpret_cast<drow4*>(b.r);
 	drow4* vv = reinterpret_cast<drow4*>(b.v);
 	const bool integrate = !(flags & GRAV_S2_PREPARE) && (flags & GRAV_S2_INTEGRATE);
-	// lane 0 owns the row's update: its state loads go out before the slot loads
+	// the state goes out before the slot loads: component p to lane p of a split row, else the
+	// row to its lane
+	constexpr bool SPLIT = TPR >= 4;
+	const int64_t e = 4 * row + (p < 3 ? p : 3);
 	drow4 r = {0.0, 0.0, 0.0, 0.0}, v = {0.0, 0.0, 0.0, 0.0};
-	if (p == 0) {
+	double rc = 0.0, vc = 0.0;
+	if (SPLIT) {
+		if (p < 4) rc = b.r[e];
+		if (p < 3 && integrate) vc = b.v[e];
+	} else if (p == 0) {
 		r = rr[row];
 		if (integrate) v = vv[row];
 	}
 
-	double ax = 0.0, ay = 0.0, az = 0.0;
+	double ax = 0.0, ay = 0.0, az = 0.0;   // SPLIT: ax holds the lane's component
 	if (!(flags & GRAV_S2_PREPARE)) {
 		const int64_t stride = 3 * static_cast<int64_t>(IT);  // 8-byte entries per slot
 		// unique-pair plans: the last (row block index) slots of a segment are column
@@ -120,6 +130,7 @@ __global__ void __launch_bounds__(S2_THREADS) stage2_kernel(const grav_batch b, 
 				ay += __shfl_xor_sync(gmask, ay, o);
 				az += __shfl_xor_sync(gmask, az, o);
 			}
+			if (SPLIT) ax = p == 0 ? ax : (p == 1 ? ay : az);
 		} else {
 			// FP32 modes: row slots hold the stage-1 pieces' compensated sums as FP32
 			// (hi, lo) pairs; they and the column slots are added in slot order into a
@@ -181,10 +192,39 @@ __global__ void __launch_bounds__(S2_THREADS) stage2_kernel(const grav_batch b, 
 			group_sum_pair<TPR>(hx, lx, gmask);
 			group_sum_pair<TPR>(hy, ly, gmask);
 			group_sum_pair<TPR>(hz, lz, gmask);
+			if (SPLIT) {
+				hx = p == 0 ? hx : (p == 1 ? hy : hz);
+				lx = p == 0 ? lx : (p == 1 ? ly : lz);
+			}
 			ax = static_cast<double>(hx) + static_cast<double>(lx);
-			ay = static_cast<double>(hy) + static_cast<double>(ly);
-			az = static_cast<double>(hz) + static_cast<double>(lz);
+			if (!SPLIT) ay = static_cast<double>(hy) + static_cast<double>(ly);
+			if (!SPLIT) az = static_cast<double>(hz) + static_cast<double>(lz);
 		}
+	}
+
+	if (SPLIT) {
+		if (p >= 4) return;
+		if (!(flags & GRAV_S2_PREPARE)) {
+			if ((flags & GRAV_S2_WRITE_A) && b.a_out) __stcs(b.a_out + e, p < 3 ? ax : 0.0);
+			if (integrate && p < 3) {
+				vc = __dadd_rn(__dmul_rn(ax, U.T), vc);
+				rc = __dadd_rn(__dmul_rn(vc, U.T), rc);
+				b.v[e] = vc;
+				b.r[e] = rc;
+			}
+		}
+		if (fp64_mode(b.mode)) {
+			static_cast<double*>(b.pos)[4 * g + p] = rc;
+		} else {
+			float* q = static_cast<float*>(b.pos) + 4 * g + p;
+			const float hi = __double2float_rn(rc);
+			q[0] = hi;
+			if (has_lo(b.mode)) {
+				const float lo = __double2float_rn(__dsub_rn(rc, static_cast<double>(hi)));
+				q[4 * b.n_pad_total] = p < 3 ? lo : 0.f;
+			}
+		}
+		return;
 	}
 	if (p != 0) return;
 
