@@ -245,6 +245,32 @@ __device__ __forceinline__ float near_threshold(float max_abs_coord)
 	return max_abs_coord * max_abs_coord * inv_k2;
 }
 
+// The scale (largest |coordinate|) whose near radius a thread's rows share, so that one minimum
+// per step tests them all: the largest of the first `real` rows', unless half of them or more are
+// nearer the origin than the outermost by a factor of 8 (of 16 with few rows, which meet 8 by
+// chance).  With the radius of such a row, a body that escaped, the others would meet
+// near pairs everywhere (fp32un at 65536 bodies, one of them 1000 times farther out: 7.8 ms a
+// step against 1.3); it is left out and the warp tests every row against its own radius.
+template <int B>
+__device__ __forceinline__ float common_scale(const float (&scale)[B], int real)
+{
+	constexpr float FAR = B <= 4 ? 16.f : 8.f;
+	float xmax = 3e38f;
+	for (int i = 0; i < B; ++i) {   // each round leaves one more row out
+		float top = 0.f;
+		int far = 0;
+#pragma unroll
+		for (int k = 0; k < B; ++k)
+			if (scale[k] <= xmax) top = fmaxf(top, scale[k]);
+		xmax = top;
+#pragma unroll
+		for (int k = 0; k < B; ++k) far += FAR * scale[k] > xmax;
+		if (2 * far > real || far >= real || xmax == 0.f || i == B - 1) break;
+		xmax *= 1.f / FAR;
+	}
+	return xmax;
+}
+
 // Three-input minimum (min.f32 with three operands, sm_100 and later).
 __device__ __forceinline__ float min3f(float a, float b, float c)
 {
@@ -286,10 +312,11 @@ __device__ __forceinline__ void near_delta(float dx, float dy, float dz, float r
 }
 
 // One j-tile against a thread's B rows, every ordered pair, rows only: the inner loop
-// of the all-pairs kernel (stage1_f32.cu); the rows' low parts are rowlo[k * T + tid].  NEAR adds the near
-// test (one three-input min per two rows and a compare; with SELF -- tiles that hold the
-// thread block's own rows -- a test per pair that also excludes r2 = eps2, so that self
-// pairs do not count) whose result is a bit per step, and after every 32 steps a cold
+// of the all-pairs kernel (stage1_f32.cu); rowlo[k * T + tid] holds the rows' low parts and near
+// radii squared.  NEAR adds the near test (one three-input min per two rows and a compare with
+// thr, the radius the rows share; with SELF -- tiles that hold the thread block's own rows, and
+// warps with rows of another radius -- a test per pair that also excludes r2 = eps2, so that
+// self pairs do not count) whose result is a bit per step, and after every 32 steps a cold
 // path over the steps where some lane of the warp met a near pair.
 template <int B, int JT, bool DS, bool NEAR, bool SELF>
 __device__ __forceinline__ void rows_tile(const float4* __restrict__ sj,
@@ -318,7 +345,7 @@ __device__ __forceinline__ void rows_tile(const float4* __restrict__ sj,
 					dz = dz + (lj.z - zl[k]);
 				}
 				const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
-				if (NEAR && SELF) near |= (r2 < thr) & (r2 > eps2);
+				if (NEAR && SELF) near |= (r2 < rowlo[k * T + tid].w) & (r2 > eps2);
 				if (NEAR && !SELF) near_min_step<B>(k, r2, rmin, rprev);
 				const float inv = rsqrt_sfu(r2);
 				float w = pj.w * inv;
@@ -341,10 +368,11 @@ __device__ __forceinline__ void rows_tile(const float4* __restrict__ sj,
 				for (int k = 0; k < B; ++k) {
 					const float dx = pj.x - xi[k], dy = pj.y - yi[k], dz = pj.z - zi[k];
 					const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
-					const bool nk = (r2 < thr) & (r2 > eps2);
+					const float4 li = rowlo[k * T + tid];
+					const bool nk = (r2 < li.w) & (r2 > eps2);
 					if (__any_sync(0xffffffffu, nk)) {
 						float ex, ey, ez;
-						near_delta(dx, dy, dz, r2, lj, rowlo[k * T + tid], eps2, nk, ex, ey, ez);
+						near_delta(dx, dy, dz, r2, lj, li, eps2, nk, ex, ey, ez);
 						fx[k] = fmaf(ex, pj.w, fx[k]);
 						fy[k] = fmaf(ey, pj.w, fy[k]);
 						fz[k] = fmaf(ez, pj.w, fz[k]);

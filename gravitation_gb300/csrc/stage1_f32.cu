@@ -42,7 +42,8 @@ __global__ void __launch_bounds__(T) stage1_f32_kernel(const grav_batch b)
 	constexpr uint32_t TILE_BYTES = J * sizeof(float4);
 	extern __shared__ __align__(128) float4 smem_tiles[];   // [2 buffers][NP][J]
 	__shared__ __align__(8) uint64_t bar[2];
-	// low parts of this thread's rows (NEAR), read back only by the thread that wrote them
+	// low parts and near radii squared of this thread's rows (NEAR), read back only by the
+	// thread that wrote them
 	__shared__ float4 rowlo[NEAR ? B : 1][NEAR ? T : 1];
 
 	const int tid = threadIdx.x;
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(T) stage1_f32_kernel(const grav_batch b)
 		float xl[B], yl[B], zl[B];
 		float fx[B], fy[B], fz[B];
 		float hx[B], hy[B], hz[B], lx[B], ly[B], lz[B];  // compensated per-body sums
-		float xmax = 0.f;                                // NEAR: largest |coordinate| of the rows
+		float scale[B];                                  // NEAR: largest |coordinate| of each row
 #pragma unroll
 		for (int k = 0; k < B; ++k) {
 			const float4 p = pos[ibase + tid + k * T];
@@ -116,13 +117,28 @@ __global__ void __launch_bounds__(T) stage1_f32_kernel(const grav_batch b)
 				xl[k] = yl[k] = zl[k] = 0.f;
 			}
 			if (NEAR) {
-				rowlo[NEAR ? k : 0][NEAR ? tid : 0] = poslo[ibase + tid + k * T];
-				if (S.il0 + tid + k * T < Uu.n) xmax = fmaxf(xmax, near_scale(p.x, p.y, p.z));
+				scale[k] = S.il0 + tid + k * T < Uu.n ? near_scale(p.x, p.y, p.z) : 0.f;
 			}
 			fx[k] = fy[k] = fz[k] = 0.f;
 			hx[k] = hy[k] = hz[k] = lx[k] = ly[k] = lz[k] = 0.f;
 		}
-		const float thr = near_threshold(xmax);
+		// NEAR: the near radius that the rows share; in a warp with rows that are left out of it
+		// (apart) every row is tested against its own
+		float thr = 0.f;
+		bool apart = false;
+		if (NEAR) {
+			const float xmax = common_scale<B>(scale, min(B, (Uu.n - (S.il0 + tid) + T - 1) / T));
+			thr = near_threshold(xmax);
+			bool stray = false;
+#pragma unroll
+			for (int k = 0; k < B; ++k) {
+				float4 lo = poslo[ibase + tid + k * T];
+				lo.w = near_threshold(fmaxf(scale[k], xmax));
+				rowlo[NEAR ? k : 0][NEAR ? tid : 0] = lo;
+				stray |= scale[k] > xmax;
+			}
+			apart = __any_sync(0xffffffffu, stray);
+		}
 
 		for (int t = 0; t < nt; ++t, ++gt) {
 			const int bs = gt & 1;
@@ -144,7 +160,7 @@ __global__ void __launch_bounds__(T) stage1_f32_kernel(const grav_batch b)
 			// NEAR: does this j-tile hold rows of this CTA (their self pairs)?
 			const int64_t jl0 = (jt0 + t) * J;
 			const bool own = jl0 < S.il0 + IT && jl0 + J > S.il0;
-			if (NEAR && own)
+			if (NEAR && (own || apart))
 				rows_tile<B, J, DS, NEAR, true>(sj, sl, eps2, thr, xi, yi, zi, xl, yl, zl, fx, fy,
 					fz, &rowlo[0][0], tid, T);
 			else

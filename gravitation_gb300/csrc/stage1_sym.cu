@@ -40,6 +40,8 @@
 // fp32cu 2.07 -> 1.58 ms, fp32un 1.40 -> 1.34 ms; at 16384 bodies 98 -> 88, 129 -> 118,
 // 106 -> 100 us.  One barrier per j-tile: a warp that is done with tile t expands its share
 // of tile t + 1 and meets the others once; the column sums of tile t leave after that.
+#include <type_traits>
+
 #include "grav_device.cuh"
 
 namespace grav {
@@ -115,9 +117,10 @@ __device__ __forceinline__ void fold_pair(float2* sums, int T, u64 f)
 // The near correction of one column body (pj, low part lj) against a thread's rows: pairs
 // closer than the near radius again, from the double-single separation, the difference
 // added to the rows' sums f and (COLS) the rows' column terms, Gm_i e, to q.  Every lane of
-// the warp calls it, with a body and a radius thr of its own (0: none).
+// the warp calls it with a body of its own (on: it has one); a row's radius squared stands in
+// rowlo's fourth component.
 template <int H, int T, bool COLS>
-__device__ __forceinline__ void near_rows(const float4& pj, const float4& lj, float eps2, float thr,
+__device__ __forceinline__ void near_rows(const float4& pj, const float4& lj, float eps2, bool on,
 	const u64 (&nx)[H], const u64 (&ny)[H], const u64 (&nz)[H], const u64 (&g2)[H],
 	const float4* __restrict__ rowlo, u64 (&fx)[H], u64 (&fy)[H], u64 (&fz)[H], float& qx,
 	float& qy, float& qz)
@@ -130,8 +133,8 @@ __device__ __forceinline__ void near_rows(const float4& pj, const float4& lj, fl
 		const u64 dx = add2(px, nx[h]), dy = add2(py, ny[h]), dz = add2(pz, nz[h]);
 		float ra, rb;
 		unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
-		if ((ra < thr) & (ra > eps2)) rows |= 1u << (2 * h);
-		if ((rb < thr) & (rb > eps2)) rows |= 2u << (2 * h);
+		if (on & (ra < rowlo[(2 * h) * T].w) & (ra > eps2)) rows |= 1u << (2 * h);
+		if (on & (rb < rowlo[(2 * h + 1) * T].w) & (rb > eps2)) rows |= 2u << (2 * h);
 	}
 	const uint32_t any = __reduce_or_sync(0xffffffffu, rows);
 #pragma unroll
@@ -225,7 +228,7 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 	// once, and the flush adds the warps in a fixed order (no shared-memory atomics, whose
 	// order would depend on warp timing)
 	float* const colacc = reinterpret_cast<float*>(sym_smem + L::COL);
-	// low parts of this thread's rows (NEAR), read back on the cold path only
+	// low parts of this thread's rows and their near radii squared (NEAR), for the cold path
 	float4* const rowlo = reinterpret_cast<float4*>(sym_smem + L::ROWLO) + threadIdx.x;  // [k]: k * T
 	// steps of each chunk that met near pairs, this thread's (BY_LANE)
 	uint32_t* const masks = reinterpret_cast<uint32_t*>(sym_smem + L::MASK) + threadIdx.x;  // [cc]: cc * T
@@ -305,7 +308,7 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 		const int64_t ibase = Uu.pad_off + S.il0 + warp * 32 * B + lane;
 		u64 nx[H], ny[H], nz[H], g2[H], fx[H], fy[H], fz[H];
 		u64 nxl[H], nyl[H], nzl[H];                      // low parts (DS)
-		float xmax = 0.f;                                // NEAR: largest |coordinate| of the rows
+		float scale[B];                                  // NEAR: largest |coordinate| of each row
 #pragma unroll
 		for (int h = 0; h < H; ++h) {
 			const float4 p = load_row(pos + ibase + (2 * h) * 32);
@@ -323,17 +326,32 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 				nzl[h] = pack2(-pl.z, -ql.z);
 			}
 			if (NEAR) {
-				rowlo[(2 * h) * T] = pos[b.n_pad_total + ibase + (2 * h) * 32];
-				rowlo[(2 * h + 1) * T] = pos[b.n_pad_total + ibase + (2 * h + 1) * 32];
 				const int row = S.il0 + warp * 32 * B + (2 * h) * 32 + lane;   // of the universe
-				if (row < Uu.n) xmax = fmaxf(xmax, near_scale(p.x, p.y, p.z));
-				if (row + 32 < Uu.n) xmax = fmaxf(xmax, near_scale(q.x, q.y, q.z));
+				scale[2 * h] = row < Uu.n ? near_scale(p.x, p.y, p.z) : 0.f;
+				scale[2 * h + 1] = row + 32 < Uu.n ? near_scale(q.x, q.y, q.z) : 0.f;
 			}
 			fx[h] = fy[h] = fz[h] = 0ull;
 		}
 #pragma unroll
 		for (int e = 0; e < 3 * B; ++e) csum[e * T] = make_float2(0.f, 0.f);
-		const float thr = near_threshold(xmax);
+		// NEAR: the near radius that the rows share; in a warp with rows that are left out of it
+		// (apart) every row is tested against its own, rowlo's fourth component
+		float thr = 0.f;
+		bool apart = false;
+		if (NEAR) {
+			const int row = S.il0 + warp * 32 * B + lane;   // of the universe
+			const float xmax = common_scale<B>(scale, min(B, (Uu.n - row + 31) / 32));
+			thr = near_threshold(xmax);
+			bool stray = false;
+#pragma unroll
+			for (int k = 0; k < B; ++k) {
+				float4 lo = pos[b.n_pad_total + ibase + k * 32];
+				lo.w = near_threshold(fmaxf(scale[k], xmax));
+				rowlo[k * T] = lo;
+				stray |= scale[k] > xmax;
+			}
+			apart = __any_sync(0xffffffffu, stray);
+		}
 
 		bool ok = expand(0);
 		int blk_done = 0;   // block J of the previous tile when it left column sums, else 0
@@ -387,9 +405,15 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 							}
 							float ra, rb;
 							unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
-							if (NEAR)
-								near |= own ? ((ra < thr) & (ra > eps2)) | ((rb < thr) & (rb > eps2))
-								            : (ra < thr) | (rb < thr);
+							if (NEAR) {
+								float ta = thr, tb = thr;
+								if (apart) {
+									ta = rowlo[(2 * h) * T].w;
+									tb = rowlo[(2 * h + 1) * T].w;
+								}
+								near |= own ? ((ra < ta) & (ra > eps2)) | ((rb < tb) & (rb > eps2))
+								            : (ra < ta) | (rb < tb);
+							}
 							const u64 inv = pack2(rsqrt_sfu(ra), rsqrt_sfu(rb));
 							const u64 w = mul2(mul2(pzw.y, inv), mul2(inv, inv));
 							fx[h] = fma2(dx, w, fx[h]);
@@ -400,11 +424,11 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 					}
 					if (NEAR) {
 						while (__any_sync(0xffffffffu, nmask != 0u)) {
-							const float radius = nmask ? thr : 0.f;
+							const bool on = nmask != 0u;
 							const int j = ch * 32 + next_step(nmask);
 							float qx = 0.f, qy = 0.f, qz = 0.f;
-							near_rows<H, T, false>(sj[j], sjl[j], eps2, radius, nx, ny, nz, g2, rowlo, fx, fy, fz,
-								qx, qy, qz);
+							near_rows<H, T, false>(sj[j], sjl[j], eps2, on, nx, ny, nz, g2, rowlo, fx, fy, fz, qx,
+								qy, qz);
 						}
 					}
 				}
@@ -420,8 +444,9 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 					u64 cx = 0ull, cy = 0ull, cz = 0ull;     // even and odd rows' column sums
 					float sx = 0.f, sy = 0.f, sz = 0.f;
 					uint32_t nmask = 0;   // NEAR: bit 31 - st of a step st that met a near pair
-#pragma unroll UNROLL
-					for (int st = 0; st < 32; ++st) {
+					// one column against the rows; by_row: every row against its own near radius
+					const auto step = [&](int st, auto by_row_t) {
+						constexpr bool by_row = decltype(by_row_t)::value;
 						const ulonglong2 pxy = se[st], pzw = se[64 + st];
 						ulonglong2 lxy = make_ulonglong2(0ull, 0ull), lz = lxy;
 						if (DS) {
@@ -429,6 +454,7 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 							lz = se[192 + st];
 						}
 						float rmin = 0.f;   // NEAR: smallest r2 of this step
+						bool near = false;
 						if (!COLPAIR) cx = cy = cz = 0ull;
 #pragma unroll
 						for (int h = 0; h < H; ++h) {
@@ -440,7 +466,9 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 							}
 							float ra, rb;
 							unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
-							if (NEAR) rmin = h == 0 ? fminf(ra, rb) : min3f(rmin, ra, rb);
+							if (NEAR && by_row)
+								near |= (ra < rowlo[(2 * h) * T].w) | (rb < rowlo[(2 * h + 1) * T].w);
+							else if (NEAR) rmin = h == 0 ? fminf(ra, rb) : min3f(rmin, ra, rb);
 							const u64 inv = pack2(rsqrt_sfu(ra), rsqrt_sfu(rb));
 							const u64 inv3 = mul2(inv, mul2(inv, inv));
 							const u64 wj = mul2(pzw.y, inv3);
@@ -459,7 +487,8 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 							}
 						}
 						// both are >= 0, so they compare as integers; the sign goes into the mask
-						if (NEAR)
+						if (NEAR && by_row) nmask = nmask << 1 | (near ? 1u : 0u);
+						else if (NEAR)
 							nmask = __funnelshift_l(__float_as_uint(rmin) - __float_as_uint(thr), nmask, 1);
 						const int src = (lane + 1) & 31;
 						float a0, a1;
@@ -478,6 +507,13 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 							unpack2(cz, a0, a1);
 							sz = __shfl_sync(0xffffffffu, sz + (a0 + a1), src);
 						}
+					};
+					if (NEAR && apart) {
+#pragma unroll 1
+						for (int st = 0; st < 32; ++st) step(st, std::true_type());
+					} else {
+#pragma unroll UNROLL
+						for (int st = 0; st < 32; ++st) step(st, std::false_type());
 					}
 					if (COLPAIR) {
 						float a0, a1;
@@ -500,7 +536,7 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 							const int st = next_step(todo);
 							const int j = ch * 32 + ((lane + st) & 31);
 							float qx = 0.f, qy = 0.f, qz = 0.f;
-							near_rows<H, T, true>(sj[j], sjl[j], eps2, thr, nx, ny, nz, g2, rowlo, fx, fy, fz, qx,
+							near_rows<H, T, true>(sj[j], sjl[j], eps2, true, nx, ny, nz, g2, rowlo, fx, fy, fz, qx,
 								qy, qz);
 							const int from = (lane - st) & 31;
 							sx += __shfl_sync(0xffffffffu, qx, from);
@@ -522,16 +558,16 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 					for (;;) {
 						while (!mask && cc + 1 < NCH) mask = masks[++cc * T];
 						if (!__any_sync(0xffffffffu, mask != 0u)) break;
-						const float radius = mask ? thr : 0.f;
+						const bool on = mask != 0u;
 						const int j = ((cc + warp) & (NCH - 1)) * 32 + ((lane + next_step(mask)) & 31);
 						float qx = 0.f, qy = 0.f, qz = 0.f;
-						near_rows<H, T, true>(sj[j], sjl[j], eps2, radius, nx, ny, nz, g2, rowlo, fx, fy, fz, qx,
-							qy, qz);
-						const uint32_t same = __match_any_sync(0xffffffffu, radius > 0.f ? j : JT + lane);
+						near_rows<H, T, true>(sj[j], sjl[j], eps2, on, nx, ny, nz, g2, rowlo, fx, fy, fz, qx, qy,
+							qz);
+						const uint32_t same = __match_any_sync(0xffffffffu, on ? j : JT + lane);
 						const unsigned turn = __popc(same & ((1u << lane) - 1u));
 						const unsigned turns = __reduce_max_sync(0xffffffffu, turn);
 						for (unsigned i = 0; i <= turns; ++i) {
-							if (turn == i && radius > 0.f) {
+							if (turn == i && on) {
 								cw[j] -= qx;
 								cw[JT + j] -= qy;
 								cw[2 * JT + j] -= qz;
@@ -603,10 +639,12 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 // the whole warp at each, is a chain of some 500 cycles that two warps per scheduler hide
 // badly; once per j-tile with every lane at its own steps it runs once or twice per tile.
 // Stage 1 at 65536 bodies, cube / cloud (without any near pass 1290 / 1290):
-//   8/128/128 1329 / 1401 -> 1311 / 1339 us, 8/64/128 1326 / 1385 -> 1320 / 1348,
-//   8/64/64 1352 / 1417 -> 1341 / 1374.
-// Rows of 4 meet half as many and keep the pass per chunk (4/256/256 1323 / 1341, by lane
-// 1366 / 1394), as does 8/128/256, whose second CTA per SM would not fit the masks.
+//   8/128/128 1329 / 1401 -> 1315 / 1344 us, 8/64/64 1352 / 1417 -> 1359 / 1391, and by lane
+//   4/256/256 1323 / 1341 -> 1366 / 1394: rows of 4 meet half as many and keep the pass per
+//   chunk, as does 8/128/256, whose second CTA per SM would not fit the masks.
+// The separate loop for warps with rows far out costs the others nothing at the unrolling
+// chosen with it; a step of 65536 bodies with one body 1000 times farther out than the others
+// takes 1.33 ms (7.8 with one radius per thread), with twenty 1.46.
 static const Stage1Kernel k_table_sym[] = {
 	GRAV_SYM_ENTRY(4, 4, 128, 4),
 	GRAV_SYM_ENTRY(4, 8, 256, 2),
@@ -626,15 +664,15 @@ static const Stage1Kernel k_table_sym[] = {
 	GRAV_SYMC_ENTRY(8, 4, 128, 4, 2),
 	GRAV_SYMC_ENTRY(4, 2, 64, 16, 5),
 	GRAV_SYMC_ENTRY(8, 2, 64, 4, 4),
-	GRAV_SYMN_ENTRY(4, 4, 128, 8, 3),
-	GRAV_SYMN_ENTRY(8, 4, 256, 8, 2),
-	GRAV_SYMN_ENTRY(8, 4, 128, 8, 2),
-	GRAV_SYMN_ENTRY(8, 4, 64, 1, 2),
+	GRAV_SYMN_ENTRY(4, 4, 128, 7, 3),
+	GRAV_SYMN_ENTRY(8, 4, 256, 4, 2),
+	GRAV_SYMN_ENTRY(8, 4, 128, 2, 2),
+	GRAV_SYMN_ENTRY(8, 4, 64, 8, 2),
 	GRAV_SYMN_ENTRY(4, 4, 256, 16, 2),
 	GRAV_SYMN_ENTRY(4, 8, 256, 16, 1),
-	GRAV_SYMN_ENTRY(4, 2, 64, 8, 7),
-	GRAV_SYMN_ENTRY(8, 2, 64, 8, 4),
-	GRAV_SYMN_ENTRY(8, 2, 128, 8, 4),
+	GRAV_SYMN_ENTRY(4, 2, 64, 6, 7),
+	GRAV_SYMN_ENTRY(8, 2, 64, 6, 4),
+	GRAV_SYMN_ENTRY(8, 2, 128, 6, 4),
 };
 
 int stage1_table_sym(const Stage1Kernel** out)

@@ -173,8 +173,8 @@ TILE_COST = {
     'fp32u': {(4, 128, 128): 87, (4, 256, 256): 85, (8, 128, 256): 64, (4, 128, 256): 71,
               (2, 256, 256): 101, (8, 256, 256): 63, (8, 128, 128): 81, (8, 128, 64): 85,
               (4, 64, 64): 90, (8, 64, 64): 67, (16, 64, 64): 64},
-    'fp32un': {(4, 128, 128): 97, (8, 128, 256): 74, (8, 128, 128): 73, (8, 128, 64): 77,
-               (4, 128, 256): 77, (4, 256, 256): 73, (4, 64, 64): 101, (8, 64, 64): 76,
+    'fp32un': {(4, 128, 128): 96, (8, 128, 256): 73, (8, 128, 128): 73, (8, 128, 64): 78,
+               (4, 128, 256): 78, (4, 256, 256): 74, (4, 64, 64): 100, (8, 64, 64): 77,
                (8, 64, 128): 74},
     'fp32cu': {(4, 128, 128): 114, (8, 128, 256): 57, (4, 128, 256): 61, (4, 256, 256): 88,
                (8, 128, 128): 86, (4, 64, 64): 118, (8, 64, 64): 88},

@@ -113,3 +113,28 @@ def test_fp64_scratch_limits(gpu):
         assert np.array_equal(np.isfinite(a), np.isfinite(b)), d
         if 1e-100 < d < 1e100:
             assert np.allclose(a, [[3.0, 0, 0], [-2.0, 0, 0]], rtol=1e-15), (d, a)
+
+
+@pytest.mark.parametrize('mode', ['fp32n', 'fp32un'])
+def test_near_modes_with_escaped_bodies(gpu, mode):
+    """Rows far out test apart from the others of their thread, each against its own near
+    radius: one escaped body, two that are near each other, and a thread whose rows are mostly
+    such."""
+    n = 2100
+    rng = np.random.default_rng(3)
+    r = rng.uniform(-1e3, 1e3, (n, 3))
+    m = rng.uniform(1.0, 100.0, n)
+    r[5] = [2e6, -1e6, 5e5]
+    r[700], r[1500] = [-3e5, 2e5, 1e5], [-3e5 + 0.5, 2e5, 1e5 + 0.25]
+    r[64:64 + 256] *= 40.0
+    r[900], r[901] = 0.0, [0.0, 1e-3, -2e-3]     # at the origin and next to it
+    gm = G_DEFAULT * m
+    ref = oracle.accel_fp64(r, gm, 1.0, coincident=True)
+    scale = magnitudes(r, gm)
+    for t in tile_list(mode):
+        eng = Engine([n], 1.0, mode=mode, tile=t, fused=False)
+        eng.set_state(r, np.zeros((n, 3)), gm)
+        a = eng.forces().cpu().numpy()
+        eng.raise_on_device_error()
+        err = np.linalg.norm(a - ref, axis=1) / scale
+        assert err.max() < TOL, (t.key(), int(err.argmax()), err.max())
