@@ -164,6 +164,49 @@ __device__ __forceinline__ void near_rows(const float4& pj, const float4& lj, fl
 	}
 }
 
+// A column body (p, low part l) against a thread's rows, every pair from its double-single
+// separation, pairs whose FP32 separation is zero contributing nothing; COLS: the column's
+// packed sums too.  Returns whether some row met it within its near radius.
+template <int H, int T, bool COLS>
+__device__ __forceinline__ bool ds_column(const float4& p, const float4& l, float eps2,
+	const u64 (&nx)[H], const u64 (&ny)[H], const u64 (&nz)[H], const u64 (&g2)[H],
+	const float4* __restrict__ rowlo, u64 (&fx)[H], u64 (&fy)[H], u64 (&fz)[H], u64& cx, u64& cy,
+	u64& cz)
+{
+	const u64 px = pack2(p.x, p.x), py = pack2(p.y, p.y), pz = pack2(p.z, p.z);
+	const u64 lx = pack2(l.x, l.x), ly = pack2(l.y, l.y), lz = pack2(l.z, l.z);
+	const u64 pw = pack2(p.w, p.w), eps22 = pack2(eps2, eps2);
+	bool near = false;
+#pragma unroll
+	for (int h = 0; h < H; ++h) {
+		const float4 la = rowlo[(2 * h) * T], lb = rowlo[(2 * h + 1) * T];
+		u64 dx = add2(px, nx[h]), dy = add2(py, ny[h]), dz = add2(pz, nz[h]);
+		float xa, xb, ya, yb, za, zb, ra, rb;
+		unpack2(dx, xa, xb);
+		unpack2(dy, ya, yb);
+		unpack2(dz, za, zb);
+		const bool na = fabsf(xa) + fabsf(ya) + fabsf(za) > 0.f, nb = fabsf(xb) + fabsf(yb) + fabsf(zb) > 0.f;
+		dx = add2(dx, add2(lx, pack2(-la.x, -lb.x)));
+		dy = add2(dy, add2(ly, pack2(-la.y, -lb.y)));
+		dz = add2(dz, add2(lz, pack2(-la.z, -lb.z)));
+		unpack2(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps22))), ra, rb);
+		near |= (na & (ra < la.w)) | (nb & (rb < lb.w));
+		const u64 inv = pack2(na ? rsqrt_sfu(ra) : 0.f, nb ? rsqrt_sfu(rb) : 0.f);
+		const u64 inv3 = mul2(inv, mul2(inv, inv));
+		const u64 wj = mul2(pw, inv3);
+		fx[h] = fma2(dx, wj, fx[h]);
+		fy[h] = fma2(dy, wj, fy[h]);
+		fz[h] = fma2(dz, wj, fz[h]);
+		if (COLS) {
+			const u64 wi = mul2(g2[h], inv3);
+			cx = fma2(dx, wi, cx);
+			cy = fma2(dy, wi, cy);
+			cz = fma2(dz, wi, cz);
+		}
+	}
+	return near;
+}
+
 // This lane's next step with a near pair, taken out of its mask (bit 31 - st: step st).
 __device__ __forceinline__ int next_step(uint32_t& mask)
 {
@@ -354,6 +397,11 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 		}
 
 		bool ok = expand(0);
+		// NEAR: the tile (first: the chunk) before met so many near pairs (marks: this lane's
+		// steps that met one) that double-single separations for all pairs of the next are
+		// cheaper: two Plummer spheres of 16384 bodies, 8/64/64, 473 us a step without
+		bool dense = false;
+		int marks = 0;
 		int blk_done = 0;   // block J of the previous tile when it left column sums, else 0
 		for (int t = 0; t < nt; ++t) {
 			// every warp has finished tile t - 1, its share of tile t is expanded, and its
@@ -384,6 +432,14 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 				const bool own = jl0 < (warp + 1) * 32 * B && jl0 + JT > warp * 32 * B;
 #pragma unroll 1
 				for (int ch = 0; ch < NCH; ++ch) {
+					if (NEAR && dense) {
+						u64 unused = 0ull;
+#pragma unroll 1
+						for (int j = ch * 32; j < ch * 32 + 32; ++j)
+							marks += ds_column<H, T, false>(sj[j], sjl[j], eps2, nx, ny, nz, g2, rowlo, fx, fy, fz,
+								unused, unused, unused);
+						continue;
+					}
 					const ulonglong2* __restrict__ se = et + ch * (L::EXA * 64);
 					uint32_t nmask = 0;
 #pragma unroll 2
@@ -422,6 +478,8 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 						}
 						if (NEAR && near) nmask |= 0x80000000u >> j;
 					}
+					if (NEAR) marks += __popc(nmask);
+					if (NEAR && t == 0 && ch == 0) dense = __any_sync(0xffffffffu, marks > 32 / 6);
 					if (NEAR) {
 						while (__any_sync(0xffffffffu, nmask != 0u)) {
 							const bool on = nmask != 0u;
@@ -444,6 +502,26 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 					u64 cx = 0ull, cy = 0ull, cz = 0ull;     // even and odd rows' column sums
 					float sx = 0.f, sy = 0.f, sz = 0.f;
 					uint32_t nmask = 0;   // NEAR: bit 31 - st of a step st that met a near pair
+					// the column sums move on to the lane that meets their body next
+					const auto rotate = [&]() {
+						const int src = (lane + 1) & 31;
+						float a0, a1;
+						if (COLPAIR) {
+							unpack2(cx, a0, a1);
+							cx = pack2(__shfl_sync(0xffffffffu, a0, src), __shfl_sync(0xffffffffu, a1, src));
+							unpack2(cy, a0, a1);
+							cy = pack2(__shfl_sync(0xffffffffu, a0, src), __shfl_sync(0xffffffffu, a1, src));
+							unpack2(cz, a0, a1);
+							cz = pack2(__shfl_sync(0xffffffffu, a0, src), __shfl_sync(0xffffffffu, a1, src));
+						} else {
+							unpack2(cx, a0, a1);
+							sx = __shfl_sync(0xffffffffu, sx + (a0 + a1), src);
+							unpack2(cy, a0, a1);
+							sy = __shfl_sync(0xffffffffu, sy + (a0 + a1), src);
+							unpack2(cz, a0, a1);
+							sz = __shfl_sync(0xffffffffu, sz + (a0 + a1), src);
+						}
+					};
 					// one column against the rows; by_row: every row against its own near radius
 					const auto step = [&](int st, auto by_row_t) {
 						constexpr bool by_row = decltype(by_row_t)::value;
@@ -490,25 +568,19 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 						if (NEAR && by_row) nmask = nmask << 1 | (near ? 1u : 0u);
 						else if (NEAR)
 							nmask = __funnelshift_l(__float_as_uint(rmin) - __float_as_uint(thr), nmask, 1);
-						const int src = (lane + 1) & 31;
-						float a0, a1;
-						if (COLPAIR) {
-							unpack2(cx, a0, a1);
-							cx = pack2(__shfl_sync(0xffffffffu, a0, src), __shfl_sync(0xffffffffu, a1, src));
-							unpack2(cy, a0, a1);
-							cy = pack2(__shfl_sync(0xffffffffu, a0, src), __shfl_sync(0xffffffffu, a1, src));
-							unpack2(cz, a0, a1);
-							cz = pack2(__shfl_sync(0xffffffffu, a0, src), __shfl_sync(0xffffffffu, a1, src));
-						} else {
-							unpack2(cx, a0, a1);
-							sx = __shfl_sync(0xffffffffu, sx + (a0 + a1), src);
-							unpack2(cy, a0, a1);
-							sy = __shfl_sync(0xffffffffu, sy + (a0 + a1), src);
-							unpack2(cz, a0, a1);
-							sz = __shfl_sync(0xffffffffu, sz + (a0 + a1), src);
-						}
+						rotate();
 					};
-					if (NEAR && apart) {
+					if (NEAR && dense) {
+						// every pair from its double-single separation, hi-part separations of zero
+						// contributing nothing; the near pairs are only counted
+#pragma unroll 1
+						for (int st = 0; st < 32; ++st) {
+							const int j = ch * 32 + ((lane + st) & 31);
+							if (!COLPAIR) cx = cy = cz = 0ull;
+							marks += ds_column<H, T, true>(sj[j], sjl[j], eps2, nx, ny, nz, g2, rowlo, fx, fy, fz, cx, cy, cz);
+							rotate();
+						}
+					} else if (NEAR && apart) {
 #pragma unroll 1
 						for (int st = 0; st < 32; ++st) step(st, std::true_type());
 					} else {
@@ -524,6 +596,8 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 						unpack2(cz, a0, a1);
 						sz = a0 + a1;
 					}
+					if (NEAR) marks += __popc(nmask);
+					if (NEAR && t == 0 && cc == 0) dense = __any_sync(0xffffffffu, marks > 32 / 6);
 					if (BY_LANE) {
 						masks[cc * T] = nmask;
 						met |= nmask;
@@ -577,6 +651,10 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 					}
 				}
 				blk_done = blkJ;
+			}
+			if (NEAR) {
+				dense = __any_sync(0xffffffffu, marks > JT / 6);
+				marks = 0;
 			}
 			// fold the tile's row partials into the compensated sums
 #pragma unroll
@@ -639,12 +717,14 @@ __global__ void __launch_bounds__(32 * W, MINB) stage1_sym_kernel(const grav_bat
 // the whole warp at each, is a chain of some 500 cycles that two warps per scheduler hide
 // badly; once per j-tile with every lane at its own steps it runs once or twice per tile.
 // Stage 1 at 65536 bodies, cube / cloud (without any near pass 1290 / 1290):
-//   8/128/128 1329 / 1401 -> 1315 / 1344 us, 8/64/64 1352 / 1417 -> 1359 / 1391, and by lane
+//   8/128/128 1329 / 1401 -> 1318 / 1354 us, 8/64/64 1352 / 1417 -> 1359 / 1387, and by lane
 //   4/256/256 1323 / 1341 -> 1366 / 1394: rows of 4 meet half as many and keep the pass per
 //   chunk, as does 8/128/256, whose second CTA per SM would not fit the masks.
 // The separate loop for warps with rows far out costs the others nothing at the unrolling
 // chosen with it; a step of 65536 bodies with one body 1000 times farther out than the others
-// takes 1.33 ms (7.8 with one radius per thread), with twenty 1.46.
+// takes 1.33 ms (7.8 with one radius per thread), with twenty 1.46.  Tiles full of near pairs
+// (dense clusters) go through ds_column: two Plummer spheres of 16384 bodies 172 us a step, of
+// 65536 2.07 ms (marked steps corrected one by one, in the loop: 239 us and 3.25 ms).
 static const Stage1Kernel k_table_sym[] = {
 	GRAV_SYM_ENTRY(4, 4, 128, 4),
 	GRAV_SYM_ENTRY(4, 8, 256, 2),
@@ -664,15 +744,15 @@ static const Stage1Kernel k_table_sym[] = {
 	GRAV_SYMC_ENTRY(8, 4, 128, 4, 2),
 	GRAV_SYMC_ENTRY(4, 2, 64, 16, 5),
 	GRAV_SYMC_ENTRY(8, 2, 64, 4, 4),
-	GRAV_SYMN_ENTRY(4, 4, 128, 7, 3),
-	GRAV_SYMN_ENTRY(8, 4, 256, 4, 2),
-	GRAV_SYMN_ENTRY(8, 4, 128, 2, 2),
+	GRAV_SYMN_ENTRY(4, 4, 128, 16, 3),
+	GRAV_SYMN_ENTRY(8, 4, 256, 10, 2),
+	GRAV_SYMN_ENTRY(8, 4, 128, 8, 2),
 	GRAV_SYMN_ENTRY(8, 4, 64, 8, 2),
 	GRAV_SYMN_ENTRY(4, 4, 256, 16, 2),
 	GRAV_SYMN_ENTRY(4, 8, 256, 16, 1),
-	GRAV_SYMN_ENTRY(4, 2, 64, 6, 7),
-	GRAV_SYMN_ENTRY(8, 2, 64, 6, 4),
-	GRAV_SYMN_ENTRY(8, 2, 128, 6, 4),
+	GRAV_SYMN_ENTRY(4, 2, 64, 2, 7),
+	GRAV_SYMN_ENTRY(8, 2, 64, 2, 4),
+	GRAV_SYMN_ENTRY(8, 2, 128, 4, 4),
 };
 
 int stage1_table_sym(const Stage1Kernel** out)
