@@ -167,15 +167,15 @@ def _ctypes_to_device(arr, nbytes, device):
 TILE_COST = {
     'fp32': {(1, 128, 128): 73, (2, 128, 128): 70, (4, 128, 128): 70, (4, 128, 256): 69,
              (8, 128, 256): 72, (2, 256, 256): 66, (4, 256, 256): 69, (8, 256, 256): 69},
-    'fp32n': {(1, 128, 128): 94, (2, 128, 128): 82, (4, 128, 128): 74, (4, 128, 256): 73,
-              (8, 128, 256): 72, (4, 256, 256): 73},
+    'fp32n': {(1, 128, 128): 93, (2, 128, 128): 81, (4, 128, 128): 72, (4, 128, 256): 71,
+              (8, 128, 256): 74, (4, 256, 256): 73},
     'fp32c': {(1, 128, 128): 108, (2, 128, 128): 100, (4, 128, 256): 98, (4, 256, 256): 95},
     'fp32u': {(4, 128, 128): 87, (4, 256, 256): 85, (8, 128, 256): 64, (4, 128, 256): 71,
               (2, 256, 256): 101, (8, 256, 256): 63, (8, 128, 128): 81, (8, 128, 64): 85,
               (4, 64, 64): 90, (8, 64, 64): 67, (16, 64, 64): 64},
-    'fp32un': {(4, 128, 128): 96, (8, 128, 256): 73, (8, 128, 128): 73, (8, 128, 64): 78,
-               (4, 128, 256): 78, (4, 256, 256): 74, (4, 64, 64): 100, (8, 64, 64): 77,
-               (8, 64, 128): 74},
+    'fp32un': {(4, 128, 128): 98, (8, 128, 256): 74, (8, 128, 128): 74, (8, 128, 64): 78,
+               (4, 128, 256): 79, (4, 256, 256): 75, (4, 64, 64): 103, (8, 64, 64): 77,
+               (8, 64, 128): 75},
     'fp32cu': {(4, 128, 128): 114, (8, 128, 256): 57, (4, 128, 256): 61, (4, 256, 256): 88,
                (8, 128, 128): 86, (4, 64, 64): 118, (8, 64, 64): 88},
 }
@@ -257,11 +257,11 @@ def fp64_pair_tile(sizes, sm_count, budget=None):
 
 FUSED_MODES = ('fp32', 'fp32n', 'fp32c')
 # (largest n, (threads, rows)) of the single-launch step, the fastest measured on GB300
-# (graph-replayed steps, fp32n / fp32, against the two-launch step's 8.7-9.0 / 7.7-8.3
-# us): n <= 32 -- 3.6 / 3.5 us (one CTA); 64 -- 4.2 / 4.0 (one CTA); 128 -- 4.8 / 4.5 (a
-# cluster of 4 CTAs); 256 -- 5.3 / 5.2 (8); 512 -- 6.5 / 5.9 (16).  From 1024 bodies
-# the two-launch step, whose stage 1 spreads the pairs over every SM, is faster (9.4 us
-# against 9.9 at 1024, 10.2 against 13.6 at 2048).
+# (graph-replayed steps of plain fp32, against the two-launch step's 7.6-8.3 us): n <= 32 --
+# 3.5 us (one CTA); 64 -- 4.0 (one CTA); 128 -- 4.5 (a cluster of 4 CTAs); 256 -- 5.2 (8);
+# 512 -- 5.9 (16).  From 1024 bodies the two-launch step, whose stage 1 spreads the pairs over
+# every SM, is faster (8.4 us against 9.0).  fp32n and fp32c take grav_steps instead (1.9 us at
+# 64 bodies, 3.6 at 1000) unless `fused` is given.
 FUSED_RULE = ((32, (256, 64)), (64, (512, 64)), (128, (256, 32)), (512, (512, 32)))
 
 
