@@ -328,6 +328,9 @@ __device__ __forceinline__ void rows_tile(const float4* __restrict__ sj,
 	const float4* __restrict__ rowlo, int tid, int T)
 {
 	static_assert(JT % 32 == 0, "j-tiles of whole 32-body groups");
+	float radius2[B];   // SELF: the rows' near radii squared
+#pragma unroll
+	for (int k = 0; k < B; ++k) radius2[k] = NEAR && SELF && B > 1 ? rowlo[k * T + tid].w : thr;
 #pragma unroll 1
 	for (int j0 = 0; j0 < JT; j0 += 32) {
 		uint32_t nmask = 0;
@@ -347,7 +350,7 @@ __device__ __forceinline__ void rows_tile(const float4* __restrict__ sj,
 					dz = dz + (lj.z - zl[k]);
 				}
 				const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
-				if (NEAR && SELF) near |= (r2 < rowlo[k * T + tid].w) & (r2 > eps2);
+				if (NEAR && SELF) near |= (r2 < radius2[k]) & (r2 > eps2);
 				if (NEAR && !SELF) near_min_step<B>(k, r2, rmin, rprev);
 				const float inv = rsqrt_sfu(r2);
 				float w = pj.w * inv;
@@ -371,7 +374,7 @@ __device__ __forceinline__ void rows_tile(const float4* __restrict__ sj,
 					const float dx = pj.x - xi[k], dy = pj.y - yi[k], dz = pj.z - zi[k];
 					const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
 					const float4 li = rowlo[k * T + tid];
-					const bool nk = (r2 < li.w) & (r2 > eps2);
+					const bool nk = (r2 < (B > 1 ? li.w : thr)) & (r2 > eps2);
 					float ex, ey, ez;
 					near_delta(dx, dy, dz, r2, lj, li, eps2, nk, ex, ey, ez);
 					fx[k] = fmaf(ex, pj.w, fx[k]);

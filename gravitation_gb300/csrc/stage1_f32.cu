@@ -118,23 +118,22 @@ __global__ void __launch_bounds__(T) stage1_f32_kernel(const grav_batch b)
 			}
 			if (NEAR) {
 				scale[k] = S.il0 + tid + k * T < Uu.n ? near_scale(p.x, p.y, p.z) : 0.f;
+				rowlo[NEAR ? k : 0][NEAR ? tid : 0] = poslo[ibase + tid + k * T];
 			}
 			fx[k] = fy[k] = fz[k] = 0.f;
 			hx[k] = hy[k] = hz[k] = lx[k] = ly[k] = lz[k] = 0.f;
 		}
 		// NEAR: the near radius that the rows share; in a warp with rows that are left out of it
 		// (apart) every row is tested against its own
-		float thr = 0.f;
+		float thr = NEAR ? near_threshold(scale[0]) : 0.f;
 		bool apart = false;
-		if (NEAR) {
+		if (NEAR && B > 1) {
 			const float xmax = common_scale<B>(scale, min(B, (Uu.n - (S.il0 + tid) + T - 1) / T));
 			thr = near_threshold(xmax);
 			bool stray = false;
 #pragma unroll
 			for (int k = 0; k < B; ++k) {
-				float4 lo = poslo[ibase + tid + k * T];
-				lo.w = near_threshold(fmaxf(scale[k], xmax));
-				rowlo[NEAR ? k : 0][NEAR ? tid : 0] = lo;
+				rowlo[NEAR ? k : 0][NEAR ? tid : 0].w = near_threshold(fmaxf(scale[k], xmax));
 				stray |= scale[k] > xmax;
 			}
 			apart = __any_sync(0xffffffffu, stray);
