@@ -14,7 +14,8 @@ accelerations (steps x 32 bytes per body), the reversal uses them and the pair k
 forms only the transposed terms, without recomputing stage 1.  By default ('auto') they
 are kept whenever they fit the slot budget (engine.slot_budget_bytes: 1000 steps of
 65536 bodies take 2.1 GB), which measured forward + adjoint 10-13 % faster from 8192
-bodies up on GB300.
+bodies up on GB300.  One universe of up to ~7000 bodies then also runs a segment's
+backward steps in one launch (csrc/adjoint_steps.cu).
 """
 
 import ctypes

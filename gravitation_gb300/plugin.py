@@ -60,9 +60,9 @@ from .engine import Engine
 # float32 runs the FP32 arithmetic with near pairs corrected, either on unique pairs
 # (fp32un: each pair once, like the reference's CPU kernels) or on all ordered pairs
 # (fp32n: finer work units, faster for small universes); the results agree to FP32
-# rounding.  Measured on GB300 (graph-replayed steps on an evolved cube, each mode with
-# its tuned tile), fp32n against fp32un: 3072 bodies 12.9 / 17.1 us, 4096 17.8 / 18.6,
-# 4608 21.3 / 21.4, 6144 30.0 / 25.5, 8192 49.4 / 39.1, 16384 156 / 118.
+# rounding.  One universe of up to 6144 bodies queues its steps in one launch, over ordered
+# pairs, in either mode.  In two launches per step (batches, larger universes) on GB300,
+# fp32n against fp32un: 4096 bodies 17.7 / 18.4 us, 16384 156 / 103, 65536 2107 / 1326.
 _DTYPE_MODE = {'float32': 'fp32n', 'float64': 'fp64'}
 UNIQUE_PAIRS_FROM_N = 4608
 

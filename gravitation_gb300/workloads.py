@@ -67,13 +67,13 @@ def run_adjoint(n=4096, steps=1000, every=32, seed=3, reps=3, tuner=None, device
                 'forward_tile': [ro.fwd.tile.bpt, ro.fwd.tile.threads, ro.fwd.tile.jtile,
                                  ro.fwd.info.grid],
                 'backward_kernel': '%s, %s' % (
+                    'a segment in one launch' if ro.adj.chained and ro.store_a else
                     'unique pairs' if ro.adj.pairs else 'all pairs',
                     'forward accelerations kept' if ro.store_a else 'accelerations recomputed')}
 
     out = {'workload': 'N=%d uniform cube seed %d, %d steps, checkpoint every %d, loss = mean '
                        '|r_K - r_target|^2 (target: masses x U[0.99,1.01])' % (n, seed, steps,
-                                                                             every),
-           'launches_per_step': {'forward': 2, 'adjoint': 2}}
+                                                                             every)}
     out['graphs'] = measure(True)
     out['launched'] = measure(False)
     out['recomputed_accelerations'] = measure(True, store_a=False)
