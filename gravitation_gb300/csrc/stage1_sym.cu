@@ -36,9 +36,9 @@
 // cycles per pair, FMA pipe 79 % (66 %) busy.  What is left is the pipe itself (16 cycles),
 // the SFU's reciprocal square root (it costs the scheduler ~2 more) and, in the near mode,
 // the three-input minima, whose register reads compete with the packed operands'.
-// Stage 1 at 65536 bodies, best tile, scalar loop -> this one: fp32u 1.335 -> 1.166 ms,
-// fp32cu 2.07 -> 1.58 ms, fp32un 1.40 -> 1.34 ms; at 16384 bodies 98 -> 88, 129 -> 118,
-// 106 -> 100 us.  One barrier per j-tile: a warp that is done with tile t expands its share
+// Stage 1 at 65536 bodies, best tile, scalar loop -> this one: fp32u 1.335 -> 1.155 ms,
+// fp32cu 2.07 -> 1.56 ms, fp32un 1.40 -> 1.32 ms; at 16384 bodies 98 -> 82, 129 -> 118,
+// 106 -> 94 us.  One barrier per j-tile: a warp that is done with tile t expands its share
 // of tile t + 1 and meets the others once; the column sums of tile t leave after that.
 #include <type_traits>
 
@@ -53,13 +53,12 @@ namespace grav {
 //             far from the origin the bodies are (+6 FADD per pair).
 //   SYM_NEAR  (GRAV_MODE_FP32UN): the SYM_PLAIN loop plus a running minimum of r2 over the
 //             thread's rows, compared with the near radius once per step (grav_device.cuh,
-//             near_threshold) into a bit mask; after a chunk of 32 steps those that met a
-//             near pair in some lane of the warp re-evaluate the near pairs from the
-//             double-single separation and add the difference (near_delta).  Near pairs
+//             near_threshold) into a bit mask; the steps that met a near pair re-evaluate the
+//             near pairs from the double-single separation and add the difference
+//             (near_delta), after the chunk or, with rows of 8, after the j-tile.  Near pairs
 //             are rare (~3e-5 of the pairs of the N = 65536 uniform cube), so this path is
-//             cold; it is warp-uniform, so it costs no divergence.  (With a vote and the
-//             cold path in every step the loop could not be unrolled; with the mask it is,
-//             1.41 -> 1.34 ms.)
+//             cold; a warp that met many evaluates every pair of its next tile that way
+//             (ds_column).
 enum { SYM_PLAIN = 0, SYM_DS = 1, SYM_NEAR = 2 };
 
 // Dynamic shared memory of one CTA, in this order (16-byte units throughout).
