@@ -17,7 +17,7 @@ import pytest
 import oracle
 from gravitation_gb300 import _lib
 from gravitation_gb300.engine import Engine, tile_list
-from gravitation_gb300.scenarios import G_DEFAULT, uniform_cube
+from gravitation_gb300.scenarios import G_DEFAULT, plummer_pair, uniform_cube
 
 pytestmark = pytest.mark.gpu
 
@@ -136,5 +136,27 @@ def test_near_modes_with_escaped_bodies(gpu, mode):
         eng.set_state(r, np.zeros((n, 3)), gm)
         a = eng.forces().cpu().numpy()
         eng.raise_on_device_error()
+        err = np.linalg.norm(a - ref, axis=1) / scale
+        assert err.max() < TOL, (t.key(), int(err.argmax()), err.max())
+
+
+def test_near_mode_in_dense_clusters(gpu):
+    """Two Plummer spheres away from the origin: most j-tiles meet so many near pairs that they
+    run on double-single separations, in diagonal blocks too.  Two bodies closer than the FP32
+    resolution of their coordinates contribute nothing to each other there either."""
+    n = 3000
+    r, _, m = plummer_pair(n, seed=4)
+    r[40] = np.float32(r[40]).astype(np.float64)
+    same = r.copy()
+    r[41], same[41] = r[40] + 1e-9, r[40]
+    gm = G_DEFAULT * m
+    ref = oracle.accel_fp64(same, gm, 1.0, coincident=True)
+    scale = magnitudes(same, gm)
+    for t in tile_list('fp32un'):
+        eng = Engine([n], 1.0, mode='fp32un', tile=t, fused=False)
+        eng.set_state(r, np.zeros((n, 3)), gm)
+        a = eng.forces().cpu().numpy()
+        eng.raise_on_device_error()
+        assert np.array_equal(a, eng.forces().cpu().numpy())
         err = np.linalg.norm(a - ref, axis=1) / scale
         assert err.max() < TOL, (t.key(), int(err.argmax()), err.max())
