@@ -163,8 +163,9 @@ class AdjointEngine:
         """Backward steps over the forward's accelerations a_in (float64 [steps, n_bodies, 4],
         in forward order: the last is reversed first), in one launch where self.chained."""
         if not self.chained or len(a_in) < 2 or not a_in.is_contiguous():
-            for a in reversed(a_in):
-                self.step(stream, a_in=a)
+            # by index: reversed(a_in) would be a flipped copy, made on the current stream
+            for k in reversed(range(len(a_in))):
+                self.step(stream, a_in=a_in[k])
             return
         self.adj.a_in = a_in[-1].data_ptr()
         try:

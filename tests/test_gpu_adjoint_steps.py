@@ -140,3 +140,31 @@ def test_adjoint_steps_choice(gpu):
     assert not AdjointEngine([700], 1.0, tile=(1, 128, 128)).chained
     assert not AdjointEngine([300, 400], 1.0).chained
     assert not AdjointEngine([9000], 1.0).chained
+
+
+@pytest.mark.parametrize('sizes,pairs', [([700], True), ([700], False), ([300, 450], None),
+                                         ([7300], None)])
+def test_adjoint_steps_unchained_on_another_stream(gpu, sizes, pairs):
+    """Two launches per step on a stream that is not the current one: the bits of the steps one
+    by one, and no memory taken."""
+    n = sum(sizes)
+    r, gm, gr, gv = state(n, 3)
+    v = np.random.default_rng(4).normal(size=(n, 3))
+    engines = [AdjointEngine(sizes, 0.5, pairs=pairs) for _ in range(2)]
+    a = torch.randn((4, n, 4), dtype=torch.float64, device=engines[0].device)
+    a[:, :, 3] = 0.0
+    for e in engines:
+        assert not e.chained
+        load(e, r, v, gm, gr, gv)
+    for k in reversed(range(4)):
+        engines[0].step(a_in=a[k])
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    engines[1].steps(a, stream=side)
+    assert torch.cuda.max_memory_allocated() == before
+    torch.cuda.synchronize()
+    engines[1].raise_on_device_error()
+    for x in ('r', 'v', 'gr', 'gv', 'ggm', 'pos', 'upos'):
+        assert torch.equal(getattr(engines[0], x), getattr(engines[1], x)), x
