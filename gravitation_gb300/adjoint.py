@@ -18,6 +18,7 @@ bodies up on GB300.  One universe of up to ~7000 bodies then also runs a segment
 backward steps in one launch (csrc/adjoint_steps.cu).
 """
 
+import contextlib
 import ctypes
 
 import numpy as np
@@ -245,6 +246,19 @@ class Rollout:
         else:
             self.fwd.step(s1 - s0, stream=stream)
 
+    @contextlib.contextmanager
+    def _on(self, stream):
+        """Work on the caller's stream: everything queued inside, graph replays too, goes there,
+        after what the current stream holds and before what it is given next."""
+        if stream is None:
+            yield
+            return
+        current = torch.cuda.current_stream(self.fwd.device)
+        stream.wait_stream(current)
+        with torch.cuda.stream(stream):
+            yield
+        current.wait_stream(stream)
+
     def _graph(self, cache, key, device, enqueue):
         g = cache.get(key)
         if g is None:
@@ -285,13 +299,13 @@ class Rollout:
         n = self.fwd.info.n_bodies
         self.fwd.set_state(r0, v0, gm, stream=stream)
         segs = self._segments()
-        for si, (s0, s1) in enumerate(segs):
-            if self.graphs:
-                self._graph(self._fwd_graphs, si, self.fwd.device,
-                            lambda st, a=si, b=s0, c=s1: self._fwd_segment(a, b, c, st)).replay()
-            else:
-                self._fwd_segment(si, s0, s1, stream)
-        with torch.cuda.stream(self.fwd._stream(stream)):
+        with self._on(stream):
+            for si, (s0, s1) in enumerate(segs):
+                if self.graphs:
+                    self._graph(self._fwd_graphs, si, self.fwd.device,
+                                lambda st, a=si, b=s0, c=s1: self._fwd_segment(a, b, c, st)).replay()
+                else:
+                    self._fwd_segment(si, s0, s1, stream)
             self.ck_r[len(segs)].copy_(self.fwd.r[:n])
             self.ck_v[len(segs)].copy_(self.fwd.v[:n])
         self.checkpoints = [(self.ck_r[i], self.ck_v[i]) for i in range(len(segs))]
@@ -304,22 +318,25 @@ class Rollout:
         CUDA graph captured on first use."""
         a = self.adj
         n = a.info.n_bodies
-        with torch.cuda.stream(self.fwd._stream(stream)):
+        with self._on(stream):
             a.gr.zero_()
             a.gv.zero_()
             a.ggm.zero_()
             a.gr[:n, :3].copy_(g_r)
             a.gv[:n, :3].copy_(g_v)
-        segs = self._segments()
-        for si in reversed(range(len(segs))):
-            s0, s1 = segs[si]
-            if self.graphs:
-                self._graph(self._adj_graphs, si, a.device,
-                            lambda st, x=si, y=s0, z=s1: self._adj_segment(x, y, z, st)).replay()
-            else:
-                self._adj_segment(si, s0, s1, stream)
+            segs = self._segments()
+            for si in reversed(range(len(segs))):
+                s0, s1 = segs[si]
+                if self.graphs:
+                    self._graph(self._adj_graphs, si, a.device,
+                                lambda st, x=si, y=s0, z=s1: self._adj_segment(x, y, z, st)).replay()
+                else:
+                    self._adj_segment(si, s0, s1, stream)
         self.reversed_state = (a.r[:n, :3].clone(), a.v[:n, :3].clone())
-        return a.gr[:n, :3].clone(), a.gv[:n, :3].clone(), a.ggm[:n].clone()
+        out = a.gr[:n, :3].clone(), a.gv[:n, :3].clone(), a.ggm[:n].clone()
+        if stream is not None:
+            stream.wait_stream(torch.cuda.current_stream(a.device))
+        return out
 
 
 class _RolloutFn(torch.autograd.Function):

@@ -256,3 +256,31 @@ def test_config4_shortened_against_fp64_adjoint(gpu, store_a):
         errs = {k: relerr(a, b) for k, a, b in zip(('r0', 'v0', 'm'), got, want)}
         for k, e in errs.items():
             assert e < tol[k], (name, errs)
+
+
+@pytest.mark.parametrize('graphs', [False, True])
+@pytest.mark.parametrize('sizes,adj_pairs', [([500], None), ([300, 200], None), ([500], True)])
+def test_rollout_on_another_stream(gpu, graphs, sizes, adj_pairs):
+    """forward and backward on a stream that lags behind the current one: the bits of the
+    current stream's run, read on the current stream, on first use and on a new state."""
+    n, steps = sum(sizes), 7
+    dev = torch.device('cuda')
+    ros = [Rollout(sizes, T, steps, 3, adj_pairs=adj_pairs, graphs=graphs) for _ in range(2)]
+    side = torch.cuda.Stream()
+    for seed in (1, 2):
+        r, v, m = compact(n, seed)
+        r, v, gm = (torch.tensor(x, device=dev) for x in (r, v, G_DEFAULT * m))
+        c = torch.tensor(np.random.default_rng(seed).normal(size=(n, 3)), device=dev)
+        torch.cuda.synchronize()
+        out = []
+        for ro, stream in zip(ros, (None, side)):
+            if stream is not None:
+                with torch.cuda.stream(stream):
+                    torch.cuda._sleep(20_000_000)   # ~10 ms
+            rK, vK = (x.clone() for x in ro.forward(r, v, gm, stream=stream))
+            out.append((rK, vK) + ro.backward(c, torch.zeros_like(c), stream=stream) + ro.reversed_state)
+        for x, y in zip(*out):
+            assert torch.equal(x, y)
+    for ro in ros:
+        ro.fwd.raise_on_device_error()
+        ro.adj.raise_on_device_error()
