@@ -116,6 +116,21 @@ def plan_part_bytes(sizes, tile, mode, comps=3):
     return int(L.grav_part_bytes(ctypes.byref(info))) * comps // 3
 
 
+def plan_fits(sizes, tile, mode, budget, comps=3):
+    """True when the unique-pair plan of `mode` with `tile` keeps its partial-sum slots within
+    `budget` bytes (None: no limit).  Its column slots, one per pair of row blocks, are
+    counted before it is planned: a plan with more slots than its tables can number does not
+    fit either."""
+    rows = tile.bpt * tile.threads
+    blocks = [-(-int(n) // rows) for n in sizes]
+    slots = sum(nb * (nb - 1) // 2 + nb for nb in blocks)   # at least; at most a grid's more
+    if slots + max(int(tile.grid), 1) > 2 ** 31 - 1:
+        return False
+    if budget is None:
+        return True
+    return slots * rows * 8 * comps <= budget and plan_part_bytes(sizes, tile, mode, comps) <= budget
+
+
 SLOT_BUDGET_FRACTION = 0.125
 SLOT_BUDGET_NO_GPU = 32 << 30
 
@@ -142,7 +157,7 @@ def fitting_tiles(sizes, mode, budget=None, comps=3, tiles=None):
         return tiles
     if budget is None:
         budget = slot_budget_bytes()
-    return [t for t in tiles if plan_part_bytes(sizes, t, mode, comps) <= budget]
+    return [t for t in tiles if plan_fits(sizes, t, mode, budget, comps)]
 
 
 def pair_plan_fits(sizes, budget=None, mode='fp32u', comps=3, tiles=None):
@@ -235,7 +250,9 @@ def default_tile(mode, sizes, device=None):
 
 def fp64_pair_tile(sizes, sm_count, budget=None):
     """Tile of the FP64 unique-pair kernel for this workload, or None where its slots do not
-    fit the slot budget (the ordered-pair kernel then serves).  The time is the FP64
+    fit the slot budget (the ordered-pair kernel, with a few MB of them, then serves; slots
+    take 24 bytes per body and row block before it: 0.7 GB at 60000 bodies, 34 GB at 600000;
+    a GB300's budget ends at ~630000).  The time is the FP64
     instructions of the busiest SM: ceil(units / SMs) units of 32 columns against a block of
     32, 64 or 128 rows, 20 per pair, and three per column slot and row in stage 2; small
     blocks win where units are few (a step at 300 bodies: 12.5 us with 32 rows, 31 with 128;
@@ -245,7 +262,7 @@ def fp64_pair_tile(sizes, sm_count, budget=None):
     best = None
     for rows in (32, 64, 128):
         t = _lib.Tile(1, rows, 32, sm_count)
-        if budget is not None and plan_part_bytes(sizes, t, _lib.GRAV_MODE_FP64U) > budget:
+        if not plan_fits(sizes, t, _lib.GRAV_MODE_FP64U, budget):
             continue
         info = make_plan(sizes, 1.0, t, _lib.GRAV_MODE_FP64U)[0]
         slots = sum(-(-n // rows) * n / 2 for n in sizes)

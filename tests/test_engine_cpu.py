@@ -4,8 +4,11 @@ taken, without a GPU."""
 import pytest
 import torch
 
+from gravitation_gb300 import _lib
 from gravitation_gb300 import build as gbuild
 from gravitation_gb300.adjoint import AdjointEngine
+from gravitation_gb300.engine import (fitting_tiles, fp64_pair_tile, pair_plan_fits, plan_fits,
+                                      plan_part_bytes, tile_list)
 
 
 @pytest.fixture(scope='module', autouse=True)
@@ -25,3 +28,26 @@ def test_adjoint_steps_hands_over_the_stored_rows(steps):
     a = torch.arange(steps * 12, dtype=torch.float64).reshape(steps, 3, 4)
     eng.steps(a, stream='s')
     assert seen == [('s', a[k].data_ptr()) for k in reversed(range(steps))]
+
+
+GB300_BUDGET = 284208 * 2 ** 20 // 8
+
+
+@pytest.mark.parametrize('sizes', [[1 << 21], [1 << 22], [3000000], [2000000] * 3, [1 << 24]])
+def test_workloads_too_large_for_unique_pairs(sizes):
+    """More slots than a plan can number: the FP64 engine takes ordered pairs, and no unique-pair
+    plan fits."""
+    assert fp64_pair_tile(sizes, 152, GB300_BUDGET) is None
+    if sizes[0] == 1 << 24:
+        assert pair_plan_fits(sizes, GB300_BUDGET, mode='fp32un') is False
+
+
+@pytest.mark.parametrize('mode', ['fp32un', _lib.GRAV_MODE_FP64U])
+@pytest.mark.parametrize('sizes', [[0], [1], [31], [32, 33, 0, 900], [5000], [70001]])
+def test_plan_fits_agrees_with_the_plan(mode, sizes):
+    for t in tile_list(mode):
+        t.grid = 608
+        need = plan_part_bytes(sizes, t, mode)
+        assert plan_fits(sizes, t, mode, need) and plan_fits(sizes, t, mode, None)
+        assert not need or not plan_fits(sizes, t, mode, need - 1)
+    assert len(fitting_tiles(sizes, 'fp32un', 1 << 40)) == len(tile_list('fp32un'))
