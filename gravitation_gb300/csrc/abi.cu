@@ -2,19 +2,41 @@
 //
 // Validation happens on the host before anything is queued on the GPU, so argument
 // errors never reach a kernel.  The library keeps no global mutable state apart from
-// the thread-local message of the last failure.
+// the thread-local message of the last failure and the kernels' shared-memory limits.
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
-#include <set>
 #include <string>
 #include <utility>
 #include <vector>
 
 #include "grav_types.h"
+
+namespace grav {
+
+// The limit belongs to the kernel and device, not to a launch: it is only ever raised, under a
+// lock, so that threads launching one kernel with different sizes cannot lower it between
+// another's call here and its launch.
+cudaError_t ensure_smem(const void* fn, int bytes)
+{
+	static std::mutex mu;
+	static std::map<std::pair<int, const void*>, int> limit;
+	int dev = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e != cudaSuccess) return e;
+	std::lock_guard<std::mutex> lock(mu);
+	const auto at = limit.find({dev, fn});
+	if (at != limit.end() && at->second >= bytes) return cudaSuccess;
+	e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+	if (e == cudaSuccess) limit[{dev, fn}] = bytes;
+	return e;
+}
+
+}  // namespace grav
 
 namespace {
 
@@ -60,21 +82,9 @@ const grav::Stage1Kernel* find_kernel(int mode, int bpt, int threads, int jtile)
 	return nullptr;
 }
 
-// Raise a kernel's dynamic shared-memory limit to what its launch asks for, once per
-// kernel and device: static plus dynamic shared memory above 48 KB (the near-pair
-// kernels' row buffers) needs the opt-in.  Called before occupancy queries and launches.
 cudaError_t ensure_smem(const grav::Stage1Kernel* k)
 {
-	static std::mutex mu;
-	static std::set<std::pair<int, const void*>> done;
-	int dev = 0;
-	cudaError_t e = cudaGetDevice(&dev);
-	if (e != cudaSuccess) return e;
-	std::lock_guard<std::mutex> lock(mu);
-	if (done.count({dev, k->fn})) return cudaSuccess;
-	e = cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k->smem_bytes);
-	if (e == cudaSuccess) done.insert({dev, k->fn});
-	return e;
+	return grav::ensure_smem(k->fn, k->smem_bytes);
 }
 
 bool valid_mode(int mode)

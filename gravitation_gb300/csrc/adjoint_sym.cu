@@ -24,10 +24,6 @@
 // as FP32, to the column slot of (I, J) (block J's last J slots).  Row
 // sums are compensated FP32 (TwoSum) and go out as FP32 (hi, lo) pairs.  Slot layout
 // [slot][NC][R]: a, h, g (NC = 7) or h, g (NC = 4).
-#include <mutex>
-#include <set>
-#include <utility>
-
 #include "grav_device.cuh"
 
 namespace grav {
@@ -372,27 +368,11 @@ const VjpSymKernel* find_vjp_sym(int bpt, int threads, int jtile, bool fa)
 // Launch the unique-pair backward pair kernel (programmatic dependent; it waits with
 // grid_dep_wait before it reads); fa: recompute the accelerations (7 slot components)
 // or not (4).  Returns cudaErrorInvalidValue for a shape that is not compiled.
-// Raise the kernel's dynamic shared-memory limit to its launch size (static plus dynamic
-// above 48 KB needs the opt-in: the 4-rows-per-thread shapes), once per kernel and device.
-static cudaError_t ensure_vjp_smem(const VjpSymKernel* k)
-{
-	static std::mutex mu;
-	static std::set<std::pair<int, const void*>> done;
-	int dev = 0;
-	cudaError_t e = cudaGetDevice(&dev);
-	if (e != cudaSuccess) return e;
-	std::lock_guard<std::mutex> lock(mu);
-	if (done.count({dev, k->fn})) return cudaSuccess;
-	e = cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k->smem);
-	if (e == cudaSuccess) done.insert({dev, k->fn});
-	return e;
-}
-
 cudaError_t launch_vjp_sym(const grav_batch& b, const float4* upos, bool fa, cudaStream_t st)
 {
 	const VjpSymKernel* k = find_vjp_sym(b.tile.bpt, b.tile.threads, b.tile.jtile, fa);
 	if (!k) return cudaErrorInvalidValue;
-	cudaError_t e = ensure_vjp_smem(k);
+	cudaError_t e = ensure_smem(k->fn, k->smem);
 	if (e != cudaSuccess) return e;
 	grav_batch copy = b;
 	void* args[] = {&copy, &upos};
@@ -407,7 +387,7 @@ int vjp_sym_occupancy(int bpt, int threads, int jtile, int* ctas_per_sm)
 		const VjpSymKernel* k = find_vjp_sym(bpt, threads, jtile, fa);
 		if (!k) return 0;
 		int occ = 0;
-		if (ensure_vjp_smem(k) != cudaSuccess ||
+		if (ensure_smem(k->fn, k->smem) != cudaSuccess ||
 			cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k->fn, k->threads, k->smem) !=
 				cudaSuccess)
 			return -1;

@@ -78,7 +78,7 @@ __device__ __forceinline__ unsigned cluster_ctas()
 inline cudaError_t launch_exchanging(const void* fn, unsigned grid, unsigned threads, int smem,
 	bool clustered, bool waits, cudaStream_t stream, void** args)
 {
-	cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+	cudaError_t e = ensure_smem(fn, smem);
 	if (e != cudaSuccess) return e;
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(grid);

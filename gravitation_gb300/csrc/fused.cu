@@ -351,8 +351,7 @@ cudaError_t launch_fused(const grav_batch& b, int flags, int threads, int rows, 
 {
 	const void* fn = find_fused(b.mode, threads);
 	const int64_t smem = fused_smem(b.mode, b.n_bodies, threads, rows);
-	cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		static_cast<int>(smem));
+	cudaError_t e = ensure_smem(fn, static_cast<int>(smem));
 	if (e != cudaSuccess) return e;
 	const unsigned grid = static_cast<unsigned>((b.n_bodies + rows - 1) / rows);
 	grav_batch copy = b;
@@ -400,8 +399,7 @@ int fused_occupancy(int mode, int64_t n, int threads, int rows, int* ctas_per_sm
 	const void* fn = find_fused(mode, threads);
 	if (!fn) return -1;
 	const int64_t smem = fused_smem(mode, n, threads, rows);
-	cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		static_cast<int>(smem));
+	cudaError_t e = ensure_smem(fn, static_cast<int>(smem));
 	if (e != cudaSuccess) return -2;
 	e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, fn, threads,
 		static_cast<size_t>(smem));

@@ -26,6 +26,11 @@ struct Stage1Kernel {
 	int cta_threads() const { return block ? block : threads; }
 };
 
+// Let launches of `fn` on the current device take `bytes` of dynamic shared memory (above 48 KB
+// of static plus dynamic the kernel's limit has to be raised).  Called before occupancy queries
+// and launches (abi.cu).
+cudaError_t ensure_smem(const void* fn, int bytes);
+
 // Stage-2 kernel (stage2.cu).  dependent = true launches it with programmatic stream
 // serialization (it reads only plan tables before its grid_dep_wait()); false launches
 // it the ordinary way, for callers whose previous kernel wrote those tables.

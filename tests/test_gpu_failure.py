@@ -46,3 +46,42 @@ def test_wait_check_rejects_bad_arguments(gpu):
     err = torch.zeros(1, dtype=torch.int32, device='cuda')
     assert L.grav_wait_check(err.data_ptr(), 0, None) == _lib.GRAV_E_ARG
     assert L.grav_wait_check(err.data_ptr(), 3_000_000_000, None) == _lib.GRAV_E_ARG
+
+
+@pytest.mark.parametrize('sizes,kw', [((64, 4096), {}), ((300, 2000, 9000), {}),
+                                      ((33, 500, 4000), {'fused': (1024, 1024)})])
+def test_threads_launch_one_kernel_with_different_sizes(gpu, sizes, kw):
+    """A kernel's shared-memory limit is not lowered by one thread under another's launch: threads
+    stepping universes of different sizes get the states of the steps taken alone."""
+    import threading
+    states, engines, failed = [], [], []
+    for n in sizes:
+        r, v, m = uniform_cube(n, seed=n)
+        pair = [Engine([n], 1e3, mode='fp32n', **kw) for _ in range(2)]
+        for e in pair:
+            e.set_state(r, v, G_DEFAULT * m)
+        engines.append(pair)
+    for alone, _ in engines:
+        for _ in range(200):
+            alone.step(2)
+    torch.cuda.synchronize()
+    start = threading.Barrier(len(sizes))
+
+    def work(eng, stream):
+        try:
+            start.wait()
+            for _ in range(200):
+                eng.step(2, stream=stream)
+            stream.synchronize()
+        except Exception as e:   # noqa: BLE001 -- reported by the main thread
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(pair[1], torch.cuda.Stream())) for pair in engines]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(60)
+    assert not failed and not any(t.is_alive() for t in threads), failed
+    for alone, threaded in engines:
+        threaded.raise_on_device_error()
+        assert torch.equal(alone.r, threaded.r) and torch.equal(alone.v, threaded.v)
