@@ -220,6 +220,7 @@ class Rollout:
         self.adj = AdjointEngine(self.sizes, self.T, device=device, pairs=adj_pairs)
         self.graphs = bool(graphs)
         self._fwd_graphs = {}
+        self._fwd_eps2 = None    # the eps2 that the forward's graphs hold
         self._adj_graphs = {}
         n = self.fwd.info.n_bodies
         nseg = -(-self.steps // self.every)
@@ -299,9 +300,17 @@ class Rollout:
         n = self.fwd.info.n_bodies
         self.fwd.set_state(r0, v0, gm, stream=stream)
         segs = self._segments()
+        # the captured launches hold the eps2 of their masses: masses that need another one are
+        # stepped launch by launch, and captured when they come again
+        eps2 = self.fwd.batch.eps2
+        graphs = self.graphs and self._fwd_eps2 in (None, eps2)
+        if self._fwd_graphs and not graphs:
+            torch.cuda.synchronize(self.fwd.device)
+            self._fwd_graphs.clear()
+        self._fwd_eps2 = eps2
         with self._on(stream):
             for si, (s0, s1) in enumerate(segs):
-                if self.graphs:
+                if graphs:
                     self._graph(self._fwd_graphs, si, self.fwd.device,
                                 lambda st, a=si, b=s0, c=s1: self._fwd_segment(a, b, c, st)).replay()
                 else:

@@ -574,7 +574,8 @@ class Engine:
 
     def capture_graph(self, steps=1):
         """CUDA graph of `steps` full steps (one launch, or stage 1 + stage 2: 2 launches
-        per step); returns a torch.cuda.CUDAGraph whose replay() runs them.
+        per step); returns a torch.cuda.CUDAGraph whose replay() runs them.  It holds the
+        eps2 of the masses loaded: capture again after set_state with other masses.
         The launches are recorded on a side stream that torch puts into capture mode."""
         side = torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream(self.device))

@@ -284,3 +284,25 @@ def test_rollout_on_another_stream(gpu, graphs, sizes, adj_pairs):
     for ro in ros:
         ro.fwd.raise_on_device_error()
         ro.adj.raise_on_device_error()
+
+
+@pytest.mark.parametrize('n', [200, 7300])
+def test_rollout_reused_with_other_masses(gpu, n):
+    """G m of 1e-1, 1e3, 1e-1 in turn: the smallest separation that the kernels resolve (eps2)
+    follows the masses of the pass, as in a Rollout made for it, captured or not."""
+    steps, dev = 6, torch.device('cuda')
+    r, v, m = compact(n, 4)
+    r[1] = r[0]             # coincident bodies meet at r2 = eps2
+    r[2] = 0.0              # and these between the two passes' eps2
+    r[3] = [1e-11, 0.0, 0.0]
+    r, v = (torch.tensor(x, device=dev) for x in (r, v))
+    ro = Rollout([n], 1e-9, steps, 3)
+    eps = []
+    for gm in (0.1, 1e3, 1e3, 0.1, 0.1):
+        g = torch.tensor(gm * m, device=dev)
+        got = [x.clone() for x in ro.forward(r, v, g)]
+        eps.append(ro.fwd.batch.eps2)
+        want = Rollout([n], 1e-9, steps, 3, graphs=False).forward(r, v, g)
+        assert all(torch.isfinite(x).all() for x in got)
+        assert all(torch.equal(x, y) for x, y in zip(got, want))
+    assert eps[1] > 10 * eps[0]
