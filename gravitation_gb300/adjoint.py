@@ -218,6 +218,9 @@ class Rollout:
         self.fwd = Engine(self.sizes, self.T, mode=mode, tile=fwd_tile, device=device,
                           tuner=tuner)
         self.adj = AdjointEngine(self.sizes, self.T, device=device, pairs=adj_pairs)
+        # one device error flag for both directions, read once per pass
+        self.adj.err = self.fwd.err
+        self.adj.batch.err = self.fwd.err.data_ptr()
         self.graphs = bool(graphs)
         self._fwd_graphs = {}
         self._fwd_eps2 = None    # the eps2 that the forward's graphs hold
@@ -365,7 +368,7 @@ class _RolloutFn(torch.autograd.Function):
         if g_vK is None:
             g_vK = torch.zeros_like(ro.final[1][:, :3])
         gr, gv, ggm = ro.backward(g_rK.to(torch.float64), g_vK.to(torch.float64))
-        ro.adj.raise_on_device_error()
+        ro.fwd.raise_on_device_error()
         return gr, gv, ctx.G * ggm, None, None
 
 

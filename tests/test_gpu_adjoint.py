@@ -306,3 +306,16 @@ def test_rollout_reused_with_other_masses(gpu, n):
         assert all(torch.isfinite(x).all() for x in got)
         assert all(torch.equal(x, y) for x, y in zip(got, want))
     assert eps[1] > 10 * eps[0]
+
+
+def test_rollout_reports_a_forward_timeout(gpu):
+    """A device error of the forward, set here from the host, is raised by the backward."""
+    from gravitation_gb300 import _lib
+    r, v, m = compact(100, 3)
+    r0, v0, mm = (torch.tensor(x, device='cuda', requires_grad=True) for x in (r, v, m))
+    ro = Rollout([100], T, 4, 2)
+    rK, _ = rollout(r0, v0, mm, G_DEFAULT, T, 4, ro=ro)
+    ro.fwd.err.fill_(_lib.GRAV_DEV_TIMEOUT)
+    with pytest.raises(_lib.GravError, match='bounded wait'):
+        rK.sum().backward()
+    assert ro.fwd.device_error() == _lib.GRAV_DEV_OK
