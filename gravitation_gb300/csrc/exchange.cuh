@@ -41,8 +41,11 @@ __device__ __forceinline__ float4 word_position(u128 v)
 		__uint_as_float(static_cast<uint32_t>(v >> 64)), 0.f);
 }
 
-// Poll one published position until its tag is `tag`; false when the bounded wait expired.
-__device__ __forceinline__ bool wait_word(const void* p, uint32_t tag, u128& v)
+// Poll one published position until its tag is `tag`; false when the bounded wait expired, or
+// that of another thread of the CTA did: *expired, one word of shared memory, zero at first,
+// keeps a CTA whose peers are gone from waiting anew for each of their words.
+__device__ __forceinline__ bool wait_word(const void* p, uint32_t tag, u128& v, int* expired,
+	uint64_t limit_ns = GRAV_WAIT_NS)
 {
 	if (word_tag(v) == tag) return true;
 	const uint64_t t0 = global_ns();
@@ -51,7 +54,11 @@ __device__ __forceinline__ bool wait_word(const void* p, uint32_t tag, u128& v)
 			v = load_word(p);
 			if (word_tag(v) == tag) return true;
 		}
-		if (global_ns() - t0 > GRAV_WAIT_NS) return false;
+		if (*const_cast<volatile int*>(expired)) return false;
+		if (global_ns() - t0 > limit_ns) {
+			*const_cast<volatile int*>(expired) = 1;
+			return false;
+		}
 	}
 }
 

@@ -23,8 +23,9 @@
 // only after it is done with step k's.  One CTA alone exchanges through its own shared
 // memory.  The CTAs wait on one another, so they are co-scheduled: up to 16 as one
 // thread-block cluster (launched as a programmatic dependent), more as a cooperative
-// launch.  Every wait is bounded (GRAV_WAIT_NS); when one expires the CTA records
-// GRAV_DEV_TIMEOUT and leaves without writing the state.
+// launch.  Every wait is bounded (GRAV_WAIT_NS), and once one has expired a CTA's others end
+// too: it records GRAV_DEV_TIMEOUT and leaves without writing its rows.  A CTA whose words
+// did arrive may have written its own, so the state is undefined then.
 //
 // Pair loop.  A CTA's rows come in groups of 4 and the columns in blocks of 64; a unit is one
 // group against one block and the CTA's units are dealt evenly to its warps in order, so a
@@ -58,7 +59,7 @@ constexpr int ST_CHUNK = 16;         // blocks per first-level FP32 sum
 constexpr int ST_SEG = 32;           // blocks between two passes over the near pairs met
 constexpr int ST_RPW = 10;           // rows whose state one warp holds (3 lanes each)
 constexpr int ST_MAX_ROWS = ST_RPW * ST_W;
-constexpr int ST_SMEM_MAX = 227 * 1024;
+constexpr int ST_SMEM_MAX = 227 * 1024 - 64;   // dynamic, less the kernel's own words
 
 // Shared memory of one CTA for n bodies and R rows per CTA (byte offsets, 16-byte units).
 struct StepsSmem {
@@ -115,6 +116,7 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 	constexpr bool DS = KIND == STEPS_DS;
 	constexpr bool NEAR = KIND == STEPS_NEAR;
 	extern __shared__ __align__(16) unsigned char steps_smem[];
+	__shared__ int expired;   // a wait of this CTA has run out (read after the first barrier)
 	const int tid = threadIdx.x;
 	const int lane = tid & 31;
 	const int warp = tid >> 5;
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 		w_hi = ((grow + 1) * NB * Wn + U - 1) / U - 1;
 	}
 
+	if (tid == 0) expired = 0;
 	// everything below belongs to the kernels before this one
 	grid_dep_wait();
 	const uint32_t tag0 = multi ? head->epoch + 1 : 0;   // tag of the positions step 0 makes
@@ -325,7 +328,7 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 							} else {
 								const float4* glo = xbuf + (((k - 1) & 1) * 2 + 1) * words + j;
 								u128 w = load_word(glo);
-								ok = wait_word(glo, tag0 + static_cast<uint32_t>(k) - 1, w) && ok;
+								ok = wait_word(glo, tag0 + static_cast<uint32_t>(k) - 1, w, &expired) && ok;
 								lj = word_position(w);
 							}
 							const float dx = cf[0] + rf[0], dy = cf[2] + rf[2], dz = cf[128] + rf[4];
@@ -467,12 +470,13 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 					l0 = load_word(src + words + j);
 					l1 = load_word(src + words + j1);
 				}
-				ok = ok && wait_word(src + j, want, w0) && wait_word(src + j1, want, w1);
+				ok = ok && wait_word(src + j, want, w0, &expired) && wait_word(src + j1, want, w1, &expired);
 				float4 c = word_position(w1);
 				if (j + 1 >= n) c = make_float4(FAR_PAD, FAR_PAD, FAR_PAD, 0.f);
 				set_pair(cols, p, word_position(w0), c);
 				if (lo_here) {
-					ok = ok && wait_word(src + words + j, want, l0) && wait_word(src + words + j1, want, l1);
+					ok = ok && wait_word(src + words + j, want, l0, &expired) &&
+						wait_word(src + words + j1, want, l1, &expired);
 					c = word_position(l1);
 					if (j + 1 >= n) c = make_float4(0.f, 0.f, 0.f, 0.f);
 					set_pair(colslo, p, word_position(l0), c);

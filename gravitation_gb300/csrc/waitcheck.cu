@@ -1,25 +1,35 @@
-// waitcheck.cu -- test hook for the bounded-wait failure path of the stage-1 kernels.
+// waitcheck.cu -- test hook for the bounded-wait failure path of the stage-1 and many-step
+// kernels.
 //
-// Every device-side wait of the library (an mbarrier phase completed by a bulk copy) is
-// bounded in time; when the bound expires the CTA records GRAV_DEV_TIMEOUT in the
+// Every device-side wait of the library (an mbarrier phase completed by a bulk copy, a word
+// that another CTA publishes) is bounded in time; when the bound expires the CTA records GRAV_DEV_TIMEOUT in the
 // caller's error flag and returns, so a lost copy never hangs the GPU and the context
 // stays usable.  This kernel exercises exactly that path without any fault: one CTA
 // initialises an mbarrier that nothing ever arrives on (no copy is issued), waits on it
-// with the same bounded wait and a caller-chosen limit, agrees on the outcome with
-// __syncthreads_or like the stage-1 kernels, records the error and returns.
-#include "grav_device.cuh"
+// with the same bounded wait and a caller-chosen limit, then on 64 words per thread that nothing
+// publishes (the first to expire ends them all), agrees on the outcome with __syncthreads_or
+// like the stage-1 kernels, records the error and returns.
+#include "exchange.cuh"
 
 namespace grav {
+
+__device__ uint4 g_unpublished;   // tag 0
 
 __global__ void __launch_bounds__(128) wait_timeout_kernel(int32_t* err, uint64_t limit_ns)
 {
 	__shared__ __align__(8) uint64_t bar;
+	__shared__ int expired;
 	if (threadIdx.x == 0) {
+		expired = 0;
 		mbar_init(&bar, 1);
 		fence_barrier_init();
 	}
 	__syncthreads();
-	const bool ok = mbar_wait_bounded(&bar, 0, limit_ns);
+	bool ok = mbar_wait_bounded(&bar, 0, limit_ns);
+	for (int i = 0; i < 64; ++i) {
+		u128 w = load_word(&g_unpublished);
+		ok = wait_word(&g_unpublished, 1, w, &expired, limit_ns) || ok;
+	}
 	if (__syncthreads_or(!ok)) {
 		if (threadIdx.x == 0) set_error(err, GRAV_DEV_TIMEOUT);
 		return;

@@ -293,8 +293,9 @@ int64_t grav_steps_scratch_bytes(int32_t n);
  * to a_out + k * a_stride (doubles); a_stride = 0 keeps the last step's only.  r, v and the
  * stage-1 positions are read at the start and written at the end of the launch.  At most one
  * CTA per SM; CTAs that wait on one another are one thread-block cluster or a cooperative
- * launch, and every wait is bounded: after 2 s it sets GRAV_DEV_TIMEOUT in b->err and the
- * state is left as it was.  b->part is not used.  Replaces the loop of a caller over
+ * launch, and every wait is bounded: after 2 s it sets GRAV_DEV_TIMEOUT in b->err.  r, v and
+ * the stage-1 positions are then undefined (some rows may have been stepped, others not) and
+ * have to be loaded again.  b->part is not used.  Replaces the loop of a caller over
  * universe_base.step's stage 1 and stage 2 calls (_base_.py:143-144).
  */
 int grav_steps(const grav_batch* b, int flags, int32_t steps, int64_t a_stride, void* scratch,
@@ -373,7 +374,8 @@ int64_t grav_adjoint_steps_scratch_bytes(int32_t n);
  * agree to FP32 rounding of the partial sums.  Positions and u (b->pos, a->upos) are read as
  * grav_adjoint_prepare or a step left them; the state and gradients are read at the start and
  * written at the end of the launch, b->pos and a->upos prepared for a further step.  Co-scheduled
- * and bounded like grav_steps: after 2 s of waiting it sets GRAV_DEV_TIMEOUT in b->err.
+ * and bounded like grav_steps: after 2 s of waiting it sets GRAV_DEV_TIMEOUT in b->err, and
+ * the state and gradients are undefined.
  */
 int grav_adjoint_steps(const grav_adjoint* a, int32_t steps, int64_t a_stride, void* scratch,
 	void* stream);
@@ -481,8 +483,8 @@ int grav_host_device_pointer(const void* host, void** dev);
 /* ---- failure path check -------------------------------------------------------------- */
 
 /* Test hook: one CTA waits, with the library's bounded wait and a limit of `limit_ns`
- * (<= 2e9), on an mbarrier that nothing completes, then writes GRAV_DEV_TIMEOUT to the
- * device int `err` and returns.  Shows that an expired wait is reported to the host and
+ * (<= 2e9), on an mbarrier that nothing completes and then on words that nothing publishes,
+ * writes GRAV_DEV_TIMEOUT to the device int `err` and returns.  Shows that an expired wait is reported to the host and
  * leaves the context usable.  No reference counterpart. */
 int grav_wait_check(int32_t* err, int64_t limit_ns, void* stream);
 

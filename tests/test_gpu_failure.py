@@ -85,3 +85,18 @@ def test_threads_launch_one_kernel_with_different_sizes(gpu, sizes, kw):
     for alone, threaded in engines:
         threaded.raise_on_device_error()
         assert torch.equal(alone.r, threaded.r) and torch.equal(alone.v, threaded.v)
+
+
+def test_expired_word_wait_ends_the_others(gpu):
+    """64 words per thread that nothing publishes, after one mbarrier: with a limit of 0.2 s the
+    CTA waits 0.4 s in all, not 13."""
+    L = _lib.load()
+    err = torch.zeros(1, dtype=torch.int32, device='cuda')
+    s = torch.cuda.current_stream()
+    e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    e0.record(s)
+    _lib.check(L.grav_wait_check(err.data_ptr(), 200_000_000, ctypes.c_void_p(s.cuda_stream)))
+    e1.record(s)
+    e1.synchronize()
+    assert int(err.item()) == _lib.GRAV_DEV_TIMEOUT
+    assert 390.0 < e0.elapsed_time(e1) < 1000.0
