@@ -35,7 +35,7 @@ constexpr int AT_CB = 64;            // columns per block
 constexpr int AT_CHUNK = 16;         // blocks per first-level FP32 sum
 constexpr int AT_RPW = 8;            // rows whose state one warp holds (4 lanes each)
 constexpr int AT_MAX_ROWS = AT_RPW * AT_W;
-constexpr int AT_SMEM_MAX = 227 * 1024 - 64;   // dynamic, less the kernel's own word
+constexpr int AT_SMEM_MAX = 227 * 1024;
 
 // Padding columns: no mass, no u, and at a distance whose powers stay finite.
 constexpr float AT_PAD = 1e9f;
@@ -84,7 +84,6 @@ __global__ void __launch_bounds__(AT_T, 1) adjoint_steps_kernel(const grav_batch
 	unsigned char* __restrict__ scratch)
 {
 	extern __shared__ __align__(16) unsigned char adjoint_smem[];
-	__shared__ int expired;   // a wait of this CTA has run out (read after the first barrier)
 	const int tid = threadIdx.x;
 	const int lane = tid & 31;
 	const int warp = tid >> 5;
@@ -125,7 +124,6 @@ __global__ void __launch_bounds__(AT_T, 1) adjoint_steps_kernel(const grav_batch
 	}
 	const bool lead = mine && c == 0;
 
-	if (tid == 0) expired = 0;
 	// everything below belongs to the kernels before this one
 	grid_dep_wait();
 	const uint32_t tag0 = head->epoch + 1;
@@ -329,8 +327,8 @@ __global__ void __launch_bounds__(AT_T, 1) adjoint_steps_kernel(const grav_batch
 				const int j = 2 * p, j1 = min(j + 1, n - 1);
 				u128 p0 = load_word(ps + j), p1 = load_word(ps + j1);
 				u128 q0 = load_word(us + j), q1 = load_word(us + j1);
-				ok = ok && wait_word(ps + j, want, p0, &expired) && wait_word(ps + j1, want, p1, &expired) &&
-					wait_word(us + j, want, q0, &expired) && wait_word(us + j1, want, q1, &expired);
+				ok = ok && wait_word(ps + j, want, p0) && wait_word(ps + j1, want, p1) &&
+					wait_word(us + j, want, q0) && wait_word(us + j1, want, q1);
 				float4 a1 = word_position(p1), d1 = word_position(q1);
 				if (j + 1 >= n) {
 					a1 = make_float4(AT_PAD, AT_PAD, AT_PAD, 0.f);

@@ -23,9 +23,9 @@
 // only after it is done with step k's.  One CTA alone exchanges through its own shared
 // memory.  The CTAs wait on one another, so they are co-scheduled: up to 16 as one
 // thread-block cluster (launched as a programmatic dependent), more as a cooperative
-// launch.  Every wait is bounded (GRAV_WAIT_NS), and once one has expired a CTA's others end
-// too: it records GRAV_DEV_TIMEOUT and leaves without writing its rows.  A CTA whose words
-// did arrive may have written its own, so the state is undefined then.
+// launch.  Every wait is bounded (GRAV_WAIT_NS) and a thread waits no more once one has expired:
+// the CTA records GRAV_DEV_TIMEOUT and leaves without writing its rows.  A CTA whose words did
+// arrive may have written its own, so the state is undefined then.
 //
 // Pair loop.  A CTA's rows come in groups of 4 and the columns in blocks of 64; a unit is one
 // group against one block and the CTA's units are dealt evenly to its warps in order, so a
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 	constexpr bool DS = KIND == STEPS_DS;
 	constexpr bool NEAR = KIND == STEPS_NEAR;
 	extern __shared__ __align__(16) unsigned char steps_smem[];
-	__shared__ int expired;   // a wait of this CTA has run out (read after the first barrier)
+	__shared__ int expired;   // a wait of the near pass has run out (read after the first barrier)
 	const int tid = threadIdx.x;
 	const int lane = tid & 31;
 	const int warp = tid >> 5;
@@ -470,13 +470,12 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 					l0 = load_word(src + words + j);
 					l1 = load_word(src + words + j1);
 				}
-				ok = ok && wait_word(src + j, want, w0, &expired) && wait_word(src + j1, want, w1, &expired);
+				ok = ok && wait_word(src + j, want, w0) && wait_word(src + j1, want, w1);
 				float4 c = word_position(w1);
 				if (j + 1 >= n) c = make_float4(FAR_PAD, FAR_PAD, FAR_PAD, 0.f);
 				set_pair(cols, p, word_position(w0), c);
 				if (lo_here) {
-					ok = ok && wait_word(src + words + j, want, l0, &expired) &&
-						wait_word(src + words + j1, want, l1, &expired);
+					ok = ok && wait_word(src + words + j, want, l0) && wait_word(src + words + j1, want, l1);
 					c = word_position(l1);
 					if (j + 1 >= n) c = make_float4(0.f, 0.f, 0.f, 0.f);
 					set_pair(colslo, p, word_position(l0), c);
