@@ -250,11 +250,12 @@ __device__ __forceinline__ float near_threshold(float max_abs_coord)
 // nearer the origin than the outermost by a factor of 8 (of 16 with few rows, which meet 8 by
 // chance).  With the radius of such a row, a body that escaped, the others would meet
 // near pairs everywhere (fp32un at 65536 bodies, one of them 1000 times farther out: 7.8 ms a
-// step against 1.3); it is left out and the warp tests every row against its own radius.
-template <int B>
+// step against 1.3); it is left out and the warp tests every row against its own radius.  Given
+// squares (radii squared), FACTOR is the factor's square.
+template <int B, int FACTOR = B <= 4 ? 16 : 8>
 __device__ __forceinline__ float common_scale(const float (&scale)[B], int real)
 {
-	constexpr float FAR = B <= 4 ? 16.f : 8.f;
+	constexpr float FAR = FACTOR;
 	float xmax = 3e38f;
 	for (int i = 0; i < B; ++i) {   // each round leaves one more row out
 		float top = 0.f;

@@ -50,7 +50,9 @@
 
 namespace grav {
 
-enum { STEPS_DS = 0, STEPS_NEAR = 1 };
+// Double-single separations everywhere; for near pairs, each row with a near radius of its own;
+// for near pairs, the rows of a group sharing theirs (common_scale).
+enum { STEPS_DS = 0, STEPS_NEAR = 1, STEPS_NEAR_SHARED = 2 };
 constexpr int ST_T = 512;            // threads per CTA
 constexpr int ST_W = ST_T / 32;
 constexpr int ST_RG = 4;             // rows per group
@@ -114,7 +116,8 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 	const int K, const int64_t a_stride, const int R, unsigned char* __restrict__ scratch)
 {
 	constexpr bool DS = KIND == STEPS_DS;
-	constexpr bool NEAR = KIND == STEPS_NEAR;
+	constexpr bool NEAR = KIND != STEPS_DS;
+	constexpr bool SHARED = KIND == STEPS_NEAR_SHARED;
 	extern __shared__ __align__(16) unsigned char steps_smem[];
 	__shared__ int expired;   // a wait of the near pass has run out (read after the first barrier)
 	const int tid = threadIdx.x;
@@ -220,6 +223,14 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 			const uint32_t eps_bits = __float_as_uint(eps2) + 1u;
 			uint32_t near_below[2];
 			float thr[2];
+			float common = 0.f;   // SHARED: the radius^2 that the group's rows share
+			if (SHARED) {
+				float own[ST_RG];
+#pragma unroll
+				for (int i = 0; i < ST_RG; ++i)
+					own[i] = reinterpret_cast<const float*>(rown + 2 * (g * ST_RG + i) + 1)[2];
+				common = common_scale<ST_RG, 256>(own, ST_RG);
+			}
 #pragma unroll
 			for (int r = 0; r < 2; ++r) {
 				const ulonglong2 xy = rp[2 * r], zt = rp[2 * r + 1];
@@ -235,6 +246,7 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 				if (NEAR) {
 					float unused;
 					unpack2(zt.y, thr[r], unused);
+					if (SHARED) thr[r] = fmaxf(thr[r], common);
 					const uint32_t t = __float_as_uint(thr[r]);
 					near_below[r] = t > eps_bits ? t - eps_bits : 0u;
 				}
@@ -530,19 +542,28 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 
 namespace {
 
-int steps_kind(int mode)
+// Rows share a near radius where the two-launch kernels' threads share one among their rows: 4
+// or 8 of them on unique pairs; on all pairs two from ~4100 to ~7000 bodies, one elsewhere.
+// Where they share, rows with radii of their own are less exact: rms force error at 6000
+// bodies, cube / Gaussian cloud, 2.0e-7 / 1.7e-7 alone, 1.3e-7 / 0.9e-7 shared, 1.4e-7 / 1.0e-7
+// with the unique-pair kernels, at 20.7 and 21.5 us a step (2500 bodies 6.9 and 7.4).  Where
+// they do not, rows alone are as exact as theirs (4096 bodies 2.1e-7 / 1.8e-7 against 2.2e-7 /
+// 1.9e-7, 9000 1.8e-7 / 1.5e-7 against 1.9e-7 / 1.5e-7) and 4 % faster.
+int steps_kind(int mode, int n)
 {
 	switch (mode) {
 	case GRAV_MODE_FP32C: case GRAV_MODE_FP32CU: return STEPS_DS;
-	case GRAV_MODE_FP32N: case GRAV_MODE_FP32UN: return STEPS_NEAR;
+	case GRAV_MODE_FP32N: return n > 4096 && n <= 7000 ? STEPS_NEAR_SHARED : STEPS_NEAR;
+	case GRAV_MODE_FP32UN: return STEPS_NEAR_SHARED;
 	default: return -1;
 	}
 }
 
 const void* steps_fn(int kind)
 {
-	return kind == STEPS_DS ? reinterpret_cast<const void*>(&steps_kernel<STEPS_DS>)
-	                        : reinterpret_cast<const void*>(&steps_kernel<STEPS_NEAR>);
+	return kind == STEPS_DS     ? reinterpret_cast<const void*>(&steps_kernel<STEPS_DS>)
+	       : kind == STEPS_NEAR ? reinterpret_cast<const void*>(&steps_kernel<STEPS_NEAR>)
+	                            : reinterpret_cast<const void*>(&steps_kernel<STEPS_NEAR_SHARED>);
 }
 
 }  // namespace
@@ -563,7 +584,7 @@ int steps_rows(int n, int sms, int steps)
 // CTA's rows fit its shared memory, and a CTA's rows its threads.
 bool steps_supported(int mode, int n, int sms)
 {
-	const int kind = steps_kind(mode);
+	const int kind = steps_kind(mode, n);
 	if (kind < 0 || n < 1 || sms < 1 || n > ST_MAX_ROWS * sms) return false;
 	const int R = steps_rows(n, sms, 1);
 	return R <= ST_MAX_ROWS && StepsSmem(kind, n, R).bytes <= ST_SMEM_MAX;
@@ -579,7 +600,7 @@ cudaError_t launch_steps(const grav_batch& b, int flags, int steps, int64_t a_st
 	int sms, cudaStream_t stream)
 {
 	const int n = static_cast<int>(b.n_bodies);
-	const int kind = steps_kind(b.mode);
+	const int kind = steps_kind(b.mode, n);
 	const void* fn = steps_fn(kind);
 	int R = steps_rows(n, sms, steps);
 	const int smem = StepsSmem(kind, n, R).bytes;

@@ -299,14 +299,17 @@ def default_fused(mode, sizes, dev_info=None):
 # (grav_steps), and up to which a single queued step does.  Measured on GB300, us per step of
 # 20 queued / accelerations alone / one step, in brackets the two-launch step:
 #   fp32n   64: 1.9 / 2.9 / 3.3 [8.5]   1000: 3.6 / 5.4 / 6.4 [9.1]   3000: 7.9 / 9.6 / 12.3 [13]
-#           4096: 11.8 / 13.8 / 16.9 [17.7]   6000: 20.4 / 23 / 28 [33]   12000: 74 / 74 / 84 [105]
+#           4096: 11.8 / 13.8 / 16.9 [17.7]   6000: 21.2 / 23 / 28 [33]   12000: 74 / 74 / 84 [105]
 #   fp32c   1000: 3.6 / 5.5 / 6.5 [11.1]   4096: 14.0 / 16.4 / 19.5 [19.3]   6000: 25 / 28 / 33 [37]
 # The unique-pair modes' own kernels pass it at 8000-9000 bodies (fp32un, default tile: 24 us
-# against 35 at 6500, 36 against 37 at 8192, 51 against 51 at 10000), but their partial sums
-# are shorter there (max force error 1.2e-6 against 3.5e-6 at 8192): they start at 6145.  The
-# plain modes, whose error is the rounding of the positions, keep their own kernels and their
-# sums bit for bit.  After a single step the last CTA moves the positions over, which from
-# ~2500 bodies on costs what the second launch does.
+# against 35 at 6500, 36 against 37 at 8192, 51 against 51 at 10000), but their worst body is
+# nearer there (force error of a cube / a Gaussian cloud at 8000 bodies, rows sharing their near
+# radius: rms 1.2e-7 / 0.8e-7 in both, max 2.2e-6 / 3.5e-6 against 1.5e-6 / 1.8e-6), so they
+# start at 6145.  fp32n has no such kernels: its ordered pairs in two launches are no nearer
+# (9000 bodies: rms 1.9e-7 / 1.5e-7, here 1.8e-7 / 1.5e-7).  The plain modes, whose error is the
+# rounding of the positions, keep their own kernels and their sums bit for bit.  After a single
+# step the last CTA moves the positions over, which from ~2500 bodies on costs what the second
+# launch does.
 STEPS_MAX_N = {'fp32n': 12288, 'fp32c': 6144, 'fp32un': 6144, 'fp32cu': 6144}
 STEPS_SINGLE_MAX_N = 2048
 

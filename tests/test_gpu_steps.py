@@ -169,3 +169,41 @@ def test_steps_clump(gpu, n):
         err = np.linalg.norm(acc[k, :, :3] - ref, axis=1)
         assert np.all(err <= TOL * magnitudes(r, gm)), (n, k)
         r, v = oracle.stage2_fp64(r, v, acc[k, :, :3], 1.0)
+
+
+@pytest.mark.parametrize('mode,n', [('fp32un', 300), ('fp32un', 2500), ('fp32un', 6000), ('fp32n', 4100),
+                                    ('fp32n', 5003)])
+def test_steps_shared_radius(gpu, mode, n):
+    """Where the pair kernels' rows share a near radius, a group of four consecutive rows does.
+    Heavy bodies at |x| ~ 100, each in a group whose others are at ~990, stand in pairs 6 apart:
+    beyond their own radius of 5, where rounding the positions to FP32 alone puts their forces
+    0.7-1.1e-6 off (rms, from the inputs in FP64), and within their group's 49, where the rounding
+    of an FP32 pair term is left: three products and the cube of a reciprocal square root good to
+    1.2e-7, at most 5e-7."""
+    r, v, m = uniform_cube(n, seed=n)
+    rng = np.random.default_rng(n + 1)
+    groups = np.arange(n // 4)[1:][::max(1, n // 256)][:64]
+    groups = groups[:len(groups) // 2 * 2]
+    for k in groups:
+        r[4 * k:4 * k + 4] = rng.choice([-1.0, 1.0], (4, 3)) * rng.uniform(980.0, 1000.0, (4, 3))
+    inner = 4 * groups + rng.integers(0, 4, len(groups))
+    for i, j in zip(inner[::2], inner[1::2]):
+        d = rng.normal(size=3)
+        mid = rng.choice([-1.0, 1.0], 3) * rng.uniform(98.0, 101.0, 3)
+        mid[rng.permutation(3)[:2]] *= rng.uniform(-0.3, 0.3, 2)
+        r[i], r[j] = mid + 3.0 * d / np.linalg.norm(d), mid - 3.0 * d / np.linalg.norm(d)
+    m[inner] = 1e5 * rng.uniform(1.0, 2.0, len(inner))
+    gm = G_DEFAULT * m
+    eng = Engine([n], 1.0, mode=mode)
+    assert eng.chained
+    eng.set_state(r, v, gm)
+    acc = torch.zeros((2, n, 4), dtype=torch.float64, device=eng.device)
+    eng.steps_to(acc)
+    torch.cuda.synchronize()
+    eng.raise_on_device_error()
+    acc = acc.cpu().numpy()
+    for k in range(2):
+        ref = oracle.accel_fp64(r, gm, 1.0, coincident=True)
+        err = np.linalg.norm(acc[k, inner, :3] - ref[inner], axis=1) / np.linalg.norm(ref[inner], axis=1)
+        assert np.sqrt((err ** 2).mean()) < 5e-7, (mode, n, k)
+        r, v = oracle.stage2_fp64(r, v, acc[k, :, :3], 1.0)
