@@ -26,7 +26,8 @@ import torch
 
 from . import _lib
 from ._lib import check
-from .engine import Engine, device_info, make_plan, _ctypes_to_device
+from .engine import (Engine, check_rows, device_info, make_plan, rows_contiguous,
+                     _ctypes_to_device)
 
 ADJ_TILE = (2, 128, 128)
 
@@ -163,7 +164,11 @@ class AdjointEngine:
     def steps(self, a_in, stream=None):
         """Backward steps over the forward's accelerations a_in (float64 [steps, n_bodies, 4],
         in forward order: the last is reversed first), in one launch where self.chained."""
-        if not self.chained or len(a_in) < 2 or not a_in.is_contiguous():
+        check_rows(a_in, sum(self.sizes), self.device, 'a_in')
+        if not rows_contiguous(a_in):
+            with torch.cuda.stream(stream):   # the copy lives and dies on the kernels' stream
+                a_in = a_in.contiguous()
+        if not self.chained or len(a_in) < 2:
             # by index: reversed(a_in) would be a flipped copy, made on the current stream
             for k in reversed(range(len(a_in))):
                 self.step(stream, a_in=a_in[k])

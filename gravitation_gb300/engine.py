@@ -176,6 +176,18 @@ def _ctypes_to_device(arr, nbytes, device):
     return dev
 
 
+def check_rows(a, n, device, what):
+    """ValueError unless a is float64 [steps, max(n, 1), 4] on `device`: the kernels that get
+    its address read or write all of it."""
+    if not (torch.is_tensor(a) and a.dtype == torch.float64 and a.device == device and a.dim() == 3
+            and tuple(a.shape[1:]) == (max(n, 1), 4)):
+        raise ValueError('%s must be a float64 tensor [steps, %d, 4] on %s' % (what, max(n, 1), device))
+
+
+def rows_contiguous(a):
+    return len(a) == 0 or a[0].is_contiguous()
+
+
 # SM time per pair of every compiled tile with three or more warps per scheduler (picoseconds;
 # an ordered pair of the all-pairs modes, an unordered one of the others), from stage 1 at
 # 65536 / 131072 bodies on GB300 (fp32un: the mean of a cube at rest and a Gaussian cloud).
@@ -560,7 +572,12 @@ class Engine:
 
     def steps_to(self, a, stream=None):
         """len(a) full steps, step k's accelerations written to a[k] (float64
-        [steps, n_bodies, 4], device)."""
+        [steps, n_bodies, 4], device; each a[k] contiguous, and apart from the others)."""
+        check_rows(a, self.info.n_bodies, self.device, 'a')
+        if not rows_contiguous(a) or len(a) > 1 and a.stride(0) < a[0].numel():
+            raise ValueError('the rows of each step must be contiguous and the steps apart')
+        if not len(a):
+            return
         flags = _lib.GRAV_S2_INTEGRATE | _lib.GRAV_S2_WRITE_A
         h = self._h(stream)
         keep = self.batch.a_out

@@ -1,14 +1,16 @@
 """CPU tests of the engines' host side: what is handed to the kernels, and which plans are
 taken, without a GPU."""
 
+import types
+
 import pytest
 import torch
 
 from gravitation_gb300 import _lib
 from gravitation_gb300 import build as gbuild
 from gravitation_gb300.adjoint import AdjointEngine
-from gravitation_gb300.engine import (fitting_tiles, fp64_pair_tile, pair_plan_fits, plan_fits,
-                                      plan_part_bytes, tile_list)
+from gravitation_gb300.engine import (Engine, fitting_tiles, fp64_pair_tile, pair_plan_fits,
+                                      plan_fits, plan_part_bytes, tile_list)
 
 
 @pytest.fixture(scope='module', autouse=True)
@@ -51,3 +53,41 @@ def test_plan_fits_agrees_with_the_plan(mode, sizes):
         assert plan_fits(sizes, t, mode, need) and plan_fits(sizes, t, mode, None)
         assert not need or not plan_fits(sizes, t, mode, need - 1)
     assert len(fitting_tiles(sizes, 'fp32un', 1 << 40)) == len(tile_list('fp32un'))
+
+
+def test_row_arguments_are_checked():
+    """Accelerations whose address goes to a kernel: shape, type, device, and for results the
+    layout, before anything is launched."""
+    good = torch.zeros((3, 5, 4), dtype=torch.float64)
+    bad = [good.to(torch.float32), good[:, :4], good[:, :, :3], good[0], good.tolist(),
+           torch.zeros((3, 5, 5), dtype=torch.float64), good.to('meta')]
+    adj = AdjointEngine.__new__(AdjointEngine)
+    adj.chained, adj.sizes, adj.device = False, [2, 3], torch.device('cpu')
+    eng = Engine.__new__(Engine)
+    eng.info, eng.device, eng.chained = types.SimpleNamespace(n_bodies=5), torch.device('cpu'), True
+    eng._steps = adj.step = None   # a launch would raise TypeError
+    for a in bad:
+        for call in (adj.steps, eng.steps_to):
+            with pytest.raises(ValueError):
+                call(a)
+    for a in (good.transpose(0, 1).contiguous().transpose(0, 1), good[:1].expand(3, 5, 4),
+              torch.zeros((3, 4, 5), dtype=torch.float64).transpose(1, 2)):
+        with pytest.raises(ValueError):
+            eng.steps_to(a)
+    eng.steps_to(good[:0])
+    adj.steps(good[:0])
+
+
+def test_adjoint_steps_of_strided_rows():
+    """Rows of a step that are not contiguous are copied; steps that are not are not."""
+    eng = AdjointEngine.__new__(AdjointEngine)
+    eng.chained, eng.sizes, eng.device = False, [3], torch.device('cpu')
+    seen = []
+    eng.step = lambda stream=None, a_in=None: seen.append(a_in.clone())
+    base = torch.arange(48, dtype=torch.float64)
+    for a in (base.reshape(4, 4, 3).transpose(1, 2), base.reshape(4, 3, 4)[::2],
+              base[:12].reshape(1, 3, 4).expand(4, 3, 4)):
+        del seen[:]
+        eng.steps(a)
+        assert all(x.is_contiguous() for x in seen)
+        assert torch.equal(torch.stack(seen), a.flip(0))

@@ -168,3 +168,20 @@ def test_adjoint_steps_unchained_on_another_stream(gpu, sizes, pairs):
     engines[1].raise_on_device_error()
     for x in ('r', 'v', 'gr', 'gv', 'ggm', 'pos', 'upos'):
         assert torch.equal(getattr(engines[0], x), getattr(engines[1], x)), x
+
+
+@pytest.mark.parametrize('sizes', [[70], [600], [300, 200]])
+def test_adjoint_steps_layouts(gpu, sizes):
+    """Steps apart by more than their rows, one step's rows repeated and strided rows: the bits of
+    the same accelerations packed."""
+    n = sum(sizes)
+    r, gm, gr, gv = state(n, 5)
+    a = torch.randn((8, n, 4), dtype=torch.float64, device='cuda')
+    for strided in (a[::2], a[:1].expand(3, n, 4), a.transpose(1, 2).contiguous().transpose(1, 2)):
+        engines = [AdjointEngine(sizes, 0.5) for _ in range(2)]
+        for e, x in zip(engines, (strided, strided.clone(memory_format=torch.contiguous_format))):
+            load(e, r, np.ones((n, 3)), gm, gr, gv)
+            e.steps(x)
+            e.raise_on_device_error()
+        for x in ('r', 'v', 'gr', 'gv', 'ggm'):
+            assert torch.equal(getattr(engines[0], x), getattr(engines[1], x)), x
