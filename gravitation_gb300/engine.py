@@ -473,19 +473,25 @@ class Engine:
     def _load(self, r, v, gm, stream):
         """set_state from tensors on the engine's device: two launches and one wait."""
         n = self.info.n_bodies
-        r, v, gm = (x.detach().reshape(shape).to(torch.float64).contiguous()
+        r, v, gm = (x.detach().reshape(shape).to(torch.float64)
                     for x, shape in ((r, (n, 3)), (v, (n, 3)), (gm, (n,))))
+        gm = gm.contiguous()
         span = torch.empty(2, dtype=torch.float64, device=self.r.device)
         check(self.lib.grav_gm_range(gm.data_ptr(), n, span.data_ptr(), self._h(None)))
         max_gm, bad = span.tolist()
         if bad:
             raise ValueError('G*m must be finite and >= 0')
         self.batch.eps2 = float(self.lib.grav_eps2(max_gm))
-        check(self.lib.grav_load_state(r.data_ptr(), v.data_ptr(), gm.data_ptr(), n,
-                                       self.r.data_ptr(), self.v.data_ptr(), self._h(stream)))
         if stream is not None:
             for x in (r, v, gm):
                 x.record_stream(stream)
+            # r and v may be `stream`'s own work: strided ones are packed there
+            with torch.cuda.stream(stream):
+                r, v = r.contiguous(), v.contiguous()
+        else:
+            r, v = r.contiguous(), v.contiguous()
+        check(self.lib.grav_load_state(r.data_ptr(), v.data_ptr(), gm.data_ptr(), n,
+                                       self.r.data_ptr(), self.v.data_ptr(), self._h(stream)))
         self.prepare(stream)
 
     def generate_state(self, scenarios, G, stream=None):

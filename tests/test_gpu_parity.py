@@ -495,3 +495,24 @@ def test_state_from_device_tensors(gpu, n):
             dev.set_state(wide[:, :3], wide[:, :3], wrong)
     torch.cuda.synchronize()
     assert torch.equal(before, dev.r)
+
+
+@pytest.mark.parametrize('n', [1, 200, 7000])
+def test_state_from_strided_tensors_of_another_stream(gpu, n):
+    """r and v written late on the stream that set_state is given, as the first three of four
+    columns (what an engine's own r and v are): the state they then hold is the one loaded."""
+    rng = np.random.default_rng(n)
+    r, v, gm = (torch.tensor(x, device='cuda') for x in (rng.normal(size=(n, 4)), rng.normal(size=(n, 4)),
+                                                         rng.uniform(1.0, 2.0, n)))
+    a, b = (Engine([n], 1e3, mode='fp32n') for _ in range(2))
+    a.set_state(r[:, :3].clone(), v[:, :3].clone(), gm)
+    late_r, late_v = torch.zeros_like(r), torch.zeros_like(v)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)   # ~10 ms
+        late_r.copy_(r)
+        late_v.copy_(v)
+    b.set_state(late_r[:, :3], late_v[:, :3], gm, stream=side)
+    torch.cuda.synchronize()
+    assert torch.equal(a.r, b.r) and torch.equal(a.v, b.v) and torch.equal(a.pos, b.pos)
