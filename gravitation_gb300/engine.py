@@ -440,6 +440,7 @@ class Engine:
             # grid-barrier counters of grav_step_fused (zero between calls)
             self.sync = torch.zeros(2, dtype=torch.int32, device=dev)
         self.scratch = None
+        self._owes_stage1 = False
         if self.chained:
             # exchange buffers of grav_steps (zeroed once, then its own)
             nbytes = int(self.lib.grav_steps_scratch_bytes(self.sizes[0]))
@@ -550,9 +551,14 @@ class Engine:
         check(self.lib.grav_prepare(self._bref, self._h(stream)))
 
     def stage1(self, stream=None):
+        self._owes_stage1 = False
         check(self.lib.grav_stage1(self._bref, self._h(stream)))
 
     def stage2(self, flags=_lib.GRAV_S2_INTEGRATE, stream=None):
+        """Stage 2 over the partial sums that stage 1, or forces(), left (queued steps in one
+        launch leave none)."""
+        if self._owes_stage1:
+            self.stage1(stream)
         check(self.lib.grav_stage2(self._bref, int(flags), self._h(stream)))
 
     def step(self, steps=1, stream=None, write_a=False):
@@ -560,7 +566,8 @@ class Engine:
         one launch) queued on the stream."""
         flags = _lib.GRAV_S2_INTEGRATE | (_lib.GRAV_S2_WRITE_A if write_a else 0)
         h = self._h(stream)
-        if self.chained and (int(steps) > 1 or self.sizes[0] <= STEPS_SINGLE_MAX_N):
+        self._owes_stage1 = False
+        if self.chained and (int(steps) > 1 or int(steps) == 1 and self.sizes[0] <= STEPS_SINGLE_MAX_N):
             self._steps(flags, int(steps), 0, h)
             return
         if self.fused:
@@ -615,6 +622,7 @@ class Engine:
         """Stage 1 only; returns the accelerations (float64 [n_bodies, 3], device)."""
         if self.chained:
             self._steps(_lib.GRAV_S2_WRITE_A, 1, 0, self._h(stream))
+            self._owes_stage1 = True   # should stage2 follow: this launch leaves no slots
             return self.a[:self.info.n_bodies, :3]
         self.stage1(stream)
         self.stage2(_lib.GRAV_S2_WRITE_A, stream)

@@ -91,3 +91,14 @@ def test_adjoint_steps_of_strided_rows():
         eng.steps(a)
         assert all(x.is_contiguous() for x in seen)
         assert torch.equal(torch.stack(seen), a.flip(0))
+
+
+@pytest.mark.parametrize('n', [100, 5000])
+def test_no_steps_launch_nothing(n):
+    """step(0), and a count below zero as range() takes it."""
+    eng = Engine.__new__(Engine)
+    eng.chained, eng.fused, eng.sizes = True, None, [n]
+    eng._h = lambda stream: None
+    eng._steps = None   # a launch would raise TypeError
+    for k in (0, -1):
+        eng.step(k)

@@ -207,3 +207,25 @@ def test_steps_shared_radius(gpu, mode, n):
         err = np.linalg.norm(acc[k, inner, :3] - ref[inner], axis=1) / np.linalg.norm(ref[inner], axis=1)
         assert np.sqrt((err ** 2).mean()) < 5e-7, (mode, n, k)
         r, v = oracle.stage2_fp64(r, v, acc[k, :, :3], 1.0)
+
+
+@pytest.mark.parametrize('mode,n', [('fp32n', 100), ('fp32n', 3000), ('fp32un', 5000)])
+def test_stage2_after_forces(gpu, mode, n):
+    """forces() and then stage2() is a step over the same partial sums as stage1() and stage2()."""
+    r, v, m = planted(n, 12)
+    a, b = (Engine([n], 1e3, mode=mode) for _ in range(2))
+    for e in (a, b):
+        assert e.chained
+        e.set_state(r, v, G_DEFAULT * m)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for _ in range(2):
+        a.forces(stream=side)
+        a.stage2(stream=side)
+        b.stage1()
+        b.stage2()
+    torch.cuda.synchronize()
+    for e in (a, b):
+        e.raise_on_device_error()
+    assert torch.equal(a.r, b.r) and torch.equal(a.v, b.v) and torch.equal(a.pos, b.pos)
+    assert not np.array_equal(a.r[:n, :3].cpu().numpy(), r)
