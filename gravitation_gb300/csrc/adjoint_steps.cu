@@ -20,7 +20,7 @@
 // pairs per lane as in steps.cu; 27 packed FMA-pipe instructions and two reciprocal square
 // roots per row and pair of columns (54 cycles), in the notation of adjoint.cu, per row
 //     P += inv3 u_j,  S += Gm_j inv3,  -Q += (Gm_j d.u_i - Gm_i d.u_j) inv2 inv3 d,
-//     g += inv3 d.u_j,      h = Gm_i P - u_i S - 3 Q, formed every 16 blocks.
+//     D += inv3 d.u_j,      h = Gm_i P - u_i S - 3 Q and g = D, formed every 16 blocks.
 // Zero separations are selected away (inv = 0).  Partials are FP32 over 16 blocks (32 terms
 // per lane and column parity), added into a second FP32 level; lanes and the warps' pieces of
 // a row are added by TwoSum in a fixed order: nothing depends on scheduling.
@@ -78,6 +78,8 @@ __device__ __forceinline__ void set_adjoint_pair(ulonglong2* cols, int p, const 
 	q[96].x = pack2(ua.z, uc.z);
 }
 
+// 512 threads leave 128 registers each: 132 bytes are spilled (with the chunk's g sums kept over
+// the whole piece 84, in the same time from 64 to 6900 bodies).
 __global__ void __launch_bounds__(AT_T, 1) adjoint_steps_kernel(const grav_batch b,
 	double* __restrict__ gr, double* __restrict__ gv, double* __restrict__ ggm, float4* upos,
 	const double* __restrict__ a_in, const int64_t a_stride, const int K, const int R,
@@ -201,9 +203,10 @@ __global__ void __launch_bounds__(AT_T, 1) adjoint_steps_kernel(const grav_batch
 			do {
 				const int m = min(AT_CHUNK, left);
 				const ulonglong2* __restrict__ cp = cols + cb * 128 + c16;
-				u64 S[2], Px[2], Py[2], Pz[2], Qx[2], Qy[2], Qz[2];
+				u64 S[2], Px[2], Py[2], Pz[2], Qx[2], Qy[2], Qz[2], D[2];
 #pragma unroll
-				for (int r = 0; r < 2; ++r) S[r] = Px[r] = Py[r] = Pz[r] = Qx[r] = Qy[r] = Qz[r] = 0ull;
+				for (int r = 0; r < 2; ++r)
+					S[r] = Px[r] = Py[r] = Pz[r] = Qx[r] = Qy[r] = Qz[r] = D[r] = 0ull;
 #pragma unroll 1
 				for (int q = 0; q < m; ++q, cp += 128) {
 #pragma unroll
@@ -224,7 +227,7 @@ __global__ void __launch_bounds__(AT_T, 1) adjoint_steps_kernel(const grav_batch
 							Pz[r] = fma2(cuz, inv3, Pz[r]);
 							const u64 duj = fma2(dz, cuz, fma2(dy, cu.y, mul2(dx, cu.x)));
 							const u64 dui = fma2(dz, uz[r], fma2(dy, uy[r], mul2(dx, ux[r])));
-							sg[r] = fma2(duj, inv3, sg[r]);
+							D[r] = fma2(duj, inv3, D[r]);
 							const u64 t = mul2(mul2(fma2(czg.y, dui, mul2(ng[r], duj)), inv2), inv3);
 							Qx[r] = fma2(t, dx, Qx[r]);
 							Qy[r] = fma2(t, dy, Qy[r]);
@@ -238,6 +241,7 @@ __global__ void __launch_bounds__(AT_T, 1) adjoint_steps_kernel(const grav_batch
 					sh[r][0] = add2(sh[r][0], fma2(ng[r], Px[r], fma2(ux[r], S[r], mul2(m3, Qx[r]))));
 					sh[r][1] = add2(sh[r][1], fma2(ng[r], Py[r], fma2(uy[r], S[r], mul2(m3, Qy[r]))));
 					sh[r][2] = add2(sh[r][2], fma2(ng[r], Pz[r], fma2(uz[r], S[r], mul2(m3, Qz[r]))));
+					sg[r] = add2(sg[r], D[r]);
 				}
 				left -= m;
 				cb += m;
