@@ -9,7 +9,8 @@ shape whose partial-sum slots fit the slot budget, at 1, 1/2 and 1/4 of the resi
 persistent grid, is timed as full steps replayed from a CUDA graph (CUDA events, at
 least ~2 ms of steps) on a seeded synthetic state of the sizes that asked, at their
 time step, and the fastest is cached as JSON (the four fastest of that pass timed
-again, longer, and the best of those kept).
+again, longer, and the best of those kept).  One universe of another size of the same bucket
+times the cached tile against the default once, and the faster serves that size.
 
 Cache robustness: an unreadable or malformed cache file is ignored (and rewritten),
 entries from another library build (different source hash) or naming a tile that is
@@ -107,7 +108,11 @@ class Tuner:
 
     def lookup(self, mode, sizes, dev_info):
         """Cached tile for the key, or None (missing, stale or invalid entry)."""
-        ent = self.load().get(self.key(mode, sizes, dev_info))
+        return self._tile(mode, self.load().get(self.key(mode, sizes, dev_info)))
+
+    @staticmethod
+    def _tile(mode, ent):
+        """The tile of a cache entry, or None."""
         if not isinstance(ent, dict):
             return None
         try:
@@ -125,48 +130,83 @@ class Tuner:
 
     def store(self, mode, sizes, dev_info, tile, ms):
         with self._lock:
-            self.load()[self.key(mode, sizes, dev_info)] = {
-                'bpt': tile.bpt, 'threads': tile.threads, 'jtile': tile.jtile,
-                'grid': tile.grid, 'ms': ms}
+            self.load()[self.key(mode, sizes, dev_info)] = self._entry(tile, ms)
+            self._keep_size(mode, sizes, dev_info, tile, ms)
             self.save()
+
+    @staticmethod
+    def _entry(tile, ms):
+        return {'bpt': tile.bpt, 'threads': tile.threads, 'jtile': tile.jtile,
+                'grid': tile.grid, 'ms': ms}
+
+    # ---- one universe: the choice for its very size ---------------------------------
+    MAX_SIZES = 64   # kept per bucket; beyond that the one kept longest goes
+
+    def _sizes(self, mode, sizes, dev_info):
+        """Of a bucket's entry, the tiles timed for one universe's very size, by size."""
+        ent = self.load()[self.key(mode, sizes, dev_info)]
+        if not isinstance(ent.get('sizes'), dict):
+            ent['sizes'] = {}
+        return ent['sizes']
+
+    def _keep_size(self, mode, sizes, dev_info, tile, ms):
+        if len(sizes) != 1:
+            return
+        own = self._sizes(mode, sizes, dev_info)
+        age = {k: e['stamp'] if isinstance(e, dict) and isinstance(e.get('stamp'), int) else 0
+               for k, e in own.items()}
+        own[str(int(sizes[0]))] = dict(self._entry(tile, ms), stamp=1 + max(age.values(), default=0))
+        if len(own) > self.MAX_SIZES:
+            del own[min(age, key=age.get)]
+
+    def _for_size(self, mode, sizes, dev_info, cached, T):
+        """The tile for one universe whose bucket has a tuned one: what was timed for this
+        size, else the faster of the cached tile and the default, timed now."""
+        from .engine import default_tile, make_plan
+        t = self._tile(mode, self._sizes(mode, sizes, dev_info).get(str(int(sizes[0]))))
+        if t is not None:
+            return t
+        tiles = [cached, default_tile(mode, sizes, dev_info.index)]
+        plans = {x.key() + (make_plan(sizes, 1.0, x, mode)[0].grid,) for x in tiles}
+        ms, t = 0.0, cached
+        if len(plans) > 1:
+            time_tile = self._timer(mode, sizes, dev_info, 5, T)
+            times = [min(time_tile(x, 4.0), time_tile(x, 4.0)) for x in tiles]
+            ms, t = min(zip(times, tiles), key=lambda p: p[0])
+        with self._lock:
+            self._keep_size(mode, sizes, dev_info, t, ms)
+            self.save()
+        return t
 
     # ---- tuning ---------------------------------------------------------------------
     def choose(self, mode, sizes, dev_info, tune_if_missing=None, T=None):
         """Tile for the workload: cached, else tuned (if enabled, with time step T), else
         the default.  The entry is tuned at the sizes that asked first and serves their
-        whole bucket.  Single universes are bucketed by quarter octave (fine_class): with
-        octave classes, the fp32un entry of the 4097-8192 class was tuned at ~5000
-        bodies and ran a 8192-body step in 55 us against 39 us for the tile tuned at 8192
-        (the stream-K work units quantise differently); tuning every entry at its
-        class's upper edge instead cost sizes far below the edge up to 10 % (fp32n at
-        5000 bodies: 53 against 48 us) and the per-universe loop of the batched
-        workload 13 %."""
+        whole bucket, one universe of another size only where it is faster there than the
+        default (timed once per size, if tuning is enabled): the work units quantise
+        differently at each size, and an fp32un entry tuned at 7200 bodies runs a step of
+        8192 in 45 us against the default's 37, one tuned at 14500 a step of 16384 in 114
+        against 107.  Tuning every entry at its class's upper edge instead cost sizes far
+        below the edge up to 10 % (fp32n at 5000 bodies: 53 against 48 us) and the
+        per-universe loop of the batched workload 13 %."""
         from .engine import default_tile
+        if tune_if_missing is None:
+            tune_if_missing = os.environ.get('GRAV_AUTOTUNE', '1') != '0'
         t = self.lookup(mode, sizes, dev_info)
         if t is not None:
+            if tune_if_missing and len(sizes) == 1 and int(sizes[0]) > 0:
+                return self._for_size(mode, sizes, dev_info, t, T)
             return t
         if sum(int(n) for n in sizes) == 0:
             return default_tile(mode, sizes, dev_info.index)   # nothing to time
-        if tune_if_missing is None:
-            tune_if_missing = os.environ.get('GRAV_AUTOTUNE', '1') != '0'
         if tune_if_missing:
             return self.tune(mode, sizes, dev_info, T=T)
         return default_tile(mode, sizes, dev_info.index)
 
-    def tune(self, mode, sizes, dev_info, reps=5, grid_factors=(1, 0.5, 0.25), T=None):
-        """Time every compiled tile shape, with the persistent grid at each of
-        `grid_factors` x (SMs x resident CTAs), on a seeded state and cache the fastest.
-        What is timed is the full step (stage 1 + stage 2) replayed from a CUDA graph: a
-        smaller grid gives each CTA more work units but leaves fewer partial-sum slots
-        per row for stage 2, which at a few thousand bodies is worth as much.  Above
-        2^38 interactions per step a replay holds one step instead of `reps`.  The steps
-        use the workload's time step T (one per universe or one for all; default the
-        reference's 1e3): the near-pair kernels' cost follows the state, and a uniform
-        cube streaming for a few steps at T = 1e3 takes the shape of its velocity
-        distribution, where more pairs are near than in the cube (at T = 1 nothing
-        moves, and the tiles with 8 rows per thread timed 12 % faster than they run)."""
+    def _timer(self, mode, sizes, dev_info, reps, T):
+        """time_tile(tile, min_ms) for a seeded state of these sizes."""
         import torch
-        from .engine import Engine, fitting_tiles, make_plan, occupancy, tile_list
+        from .engine import Engine
         from .scenarios import uniform_cube
         sizes = [int(s) for s in sizes]
         rs, vs, ms = [], [], []
@@ -178,13 +218,12 @@ class Tuner:
         r = np.concatenate(rs) if rs else np.zeros((0, 3))
         v = np.concatenate(vs) if vs else np.zeros((0, 3))
         gm = np.concatenate(ms) if ms else np.zeros(0)
-        best = None
-        seen = set()
         step_T = 1e3 if T is None else T
         if sum(n * n for n in sizes) >= 1 << 38:
             # steps of 0.1 s and more (above ~500k bodies): one step per replay is
             # already far above the timing noise, and keeps tuning to about a minute
             reps = 1
+
         def time_tile(t, min_ms):
             """ms per step of tile t: full steps replayed from a CUDA graph, enough
             replays for about `min_ms` of steps (short steps time noisily)."""
@@ -210,6 +249,25 @@ class Tuner:
             del g, eng
             return out
 
+        return time_tile
+
+    def tune(self, mode, sizes, dev_info, reps=5, grid_factors=(1, 0.5, 0.25), T=None):
+        """Time every compiled tile shape, with the persistent grid at each of
+        `grid_factors` x (SMs x resident CTAs), on a seeded state and cache the fastest.
+        What is timed is the full step (stage 1 + stage 2) replayed from a CUDA graph: a
+        smaller grid gives each CTA more work units but leaves fewer partial-sum slots
+        per row for stage 2, which at a few thousand bodies is worth as much.  Above
+        2^38 interactions per step a replay holds one step instead of `reps`.  The steps
+        use the workload's time step T (one per universe or one for all; default the
+        reference's 1e3): the near-pair kernels' cost follows the state, and a uniform
+        cube streaming for a few steps at T = 1e3 takes the shape of its velocity
+        distribution, where more pairs are near than in the cube (at T = 1 nothing
+        moves, and the tiles with 8 rows per thread timed 12 % faster than they run)."""
+        from .engine import fitting_tiles, make_plan, occupancy, tile_list
+        sizes = [int(s) for s in sizes]
+        best = None
+        seen = set()
+        time_tile = self._timer(mode, sizes, dev_info, reps, T)
         timed = []
         # unique-pair shapes whose partial-sum slots exceed the slot budget at these
         # sizes are not candidates (rows per block set the slots' N^2 / R growth)

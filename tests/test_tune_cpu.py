@@ -83,3 +83,45 @@ def test_quarter_octave_classes():
         c = fine_class(n)
         assert n <= c < 1.26 * n + 1, n
         assert fine_class(c) == c
+
+
+def test_another_size_of_the_bucket(tmp_path, monkeypatch):
+    """An entry tuned at 7200 bodies serves 8192 only where it is the faster there: timed against
+    the default once, remembered in the file, never at the size it was tuned for, and not when
+    tuning is off; at most MAX_SIZES sizes are remembered."""
+    cached, default = _lib.Tile(4, 128, 128, 456), _lib.Tile(8, 128, 128, 304)
+    timed = []
+    slow = {}
+
+    def timer(self, mode, sizes, dev, reps, T):
+        def time_tile(t, min_ms):
+            timed.append((sizes[0], t.key()))
+            return slow.get((sizes[0], t.key()), 1.0)
+        return time_tile
+
+    monkeypatch.setattr(Tuner, '_timer', timer)
+    monkeypatch.setattr('gravitation_gb300.engine.default_tile',
+                        lambda mode, sizes, device=None: _lib.Tile(*default.key(), default.grid))
+    path = str(tmp_path / 'c.json')
+    t = Tuner(path, build_hash='h')
+    t.store('fp32un', [7200], DEV, cached, 0.03)
+    choose = lambda n, t=t: t.choose('fp32un', [n], DEV, tune_if_missing=True).key()  # noqa: E731
+    assert choose(7200) == cached.key() and not timed
+    slow[8192, cached.key()] = 1.2
+    slow[8000, default.key()] = 1.2
+    assert t.choose('fp32un', [8192], DEV, tune_if_missing=False).key() == cached.key() and not timed
+    assert choose(8192) == default.key() and {k for _, k in timed} == {cached.key(), default.key()}
+    assert choose(8000) == cached.key()
+    del timed[:]
+    again = Tuner(path, build_hash='h')
+    assert choose(8192, again) == default.key() and choose(8000, again) == cached.key()
+    assert choose(7200, again) == cached.key() and not timed
+    for n in range(7300, 7300 + Tuner.MAX_SIZES):
+        choose(n)
+    entry = json.loads(open(path).read())['entries'][t.key('fp32un', [8192], DEV)]
+    assert len(entry['sizes']) == Tuner.MAX_SIZES and '7200' not in entry['sizes']
+    entry['sizes'] = {'8192': 'garbage', '8000': 3}
+    t.load()[t.key('fp32un', [8192], DEV)] = entry
+    assert choose(8192) == default.key()
+    entry['sizes'] = 'garbage'
+    assert choose(8192) == default.key()
