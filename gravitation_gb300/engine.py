@@ -214,8 +214,8 @@ def tile_time(mode, tile, info, sm_count, resident):
     two), plus the slots' traffic in stage 2 (24 bytes per entry, written and read, at ~8
     TB/s).  Over the unique-pair modes at 300-131072 bodies (56 measured sets of tiles) the
     tile it picks ran within 0.2 % of the fastest on average, at worst 7 % (fp32cu at 6500
-    bodies), over the all-pairs modes within 0.4 %; the rule before it, which did not count the CTAs that share an SM, was 5-30 %
-    off above 8192 bodies."""
+    bodies, fp32un at 9000), over the all-pairs modes within 0.4 %; the rule before it, which
+    did not count the CTAs that share an SM, was 5-30 % off above 8192 bodies."""
     grid = min(info.grid, info.n_units)
     on_sm = min(-(-grid // sm_count), resident)
     warps = on_sm * tile.threads / 128.0
@@ -232,6 +232,10 @@ def tile_time(mode, tile, info, sm_count, resident):
 # 1.5 / 7.5, 8/128/128 1.7 / 7.0, 8/64/128 1.7 / 8.0, 8/128/256 1.9 / 7.4.
 DEFAULT_JTILE_MAX = {'fp32u': 64, 'fp32un': 64}
 DEFAULT_ALSO = {'fp32un': [(8, 128, 128)]}
+# And shapes it may pick where no CTA has more than one unit.  fp32un from 6145 to ~7300 bodies:
+# 4/128/128 28.8-30.0 us a step (rms force error 1.4e-7 - 1.3e-7), 8/128/128 34.1-35.9 (1.3e-7 -
+# 1.2e-7), 8/64/64 31.9-37.7, 4/64/64 29.0-37.9.
+DEFAULT_ONE_WAVE = {'fp32un': [(4, 128, 128)]}
 
 
 def default_tile(mode, sizes, device=None):
@@ -242,7 +246,8 @@ def default_tile(mode, sizes, device=None):
     cands = fitting_tiles(sizes, mode) or tile_list(mode)
     longest = DEFAULT_JTILE_MAX.get(mode, 128)
     also = DEFAULT_ALSO.get(mode, ())
-    cands = [t for t in cands if t.jtile <= longest or t.key() in also] or cands
+    one_wave = DEFAULT_ONE_WAVE.get(mode, ())
+    cands = [t for t in cands if t.jtile <= longest or t.key() in also or t.key() in one_wave] or cands
     best = None
     for t in cands:
         occ = occupancy(mode, t, device)
@@ -250,6 +255,8 @@ def default_tile(mode, sizes, device=None):
             continue
         t.grid = info.sm_count * occ
         pinfo, _, _ = make_plan(sizes, 1.0, t, mode)
+        if t.key() in one_wave and pinfo.n_units > t.grid:
+            continue
         # no pairs at all (only empty universes): stage 1 launches nothing, any compiled
         # shape serves
         score = tile_time(mode, t, pinfo, info.sm_count, occ) if pinfo.n_units else float('inf')

@@ -160,3 +160,18 @@ def test_near_mode_in_dense_clusters(gpu):
         assert np.array_equal(a, eng.forces().cpu().numpy())
         err = np.linalg.norm(a - ref, axis=1) / scale
         assert err.max() < TOL, (t.key(), int(err.argmax()), err.max())
+
+
+@pytest.mark.parametrize('n,one_wave', [(6145, True), (7168, True), (7297, True), (7700, False)])
+def test_default_tile_of_one_wave(gpu, n, one_wave):
+    """fp32un from 6145 bodies to where a CTA would get a second unit: rows of 4 in blocks of 512;
+    its forces like those of any shape."""
+    r, v, m = planted_cube(n, 512, n)
+    eng = Engine([n], 1.0, mode='fp32un')
+    assert (eng.tile.key() == (4, 128, 128)) == one_wave
+    assert not one_wave or eng.info.n_units <= eng.info.grid
+    eng.set_state(r, v, G_DEFAULT * m)
+    a = eng.forces().cpu().numpy()
+    eng.raise_on_device_error()
+    ref = oracle.accel_fp64(r, G_DEFAULT * m, 1.0, coincident=True)
+    assert np.all(np.linalg.norm(a - ref, axis=1) <= TOL * magnitudes(r, G_DEFAULT * m))
