@@ -1,5 +1,6 @@
 // exchange.cuh -- tagged 128-bit words between the CTAs of one launch (steps.cu,
-// adjoint_steps.cu) and the launch that puts those CTAs on the GPU together.
+// adjoint_steps.cu), and the launch that puts CTAs which wait on one another on the GPU
+// together (those, and fused.cu).
 #pragma once
 #include "grav_device.cuh"
 
@@ -63,6 +64,8 @@ __device__ __forceinline__ bool wait_word(const void* p, uint32_t tag, u128& v, 
 	}
 }
 
+// Hardware cluster barrier, split: every thread of every CTA of the cluster arrives
+// (release: its earlier loads and stores are ordered before) and later waits (acquire).
 __device__ __forceinline__ void cluster_arrive()
 {
 	asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -73,6 +76,7 @@ __device__ __forceinline__ void cluster_wait()
 	asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// CTAs in this CTA's thread-block cluster (1 when launched without clusters)
 __device__ __forceinline__ unsigned cluster_ctas()
 {
 	unsigned v;

@@ -24,13 +24,11 @@
 // every 32 columns the FP32 partials are folded into compensated (TwoSum) sums.  The
 // splits' (hi, lo) sums go through shared memory and are combined in a fixed pairwise
 // tree: the result does not depend on scheduling.
-#include "grav_device.cuh"
+#include "exchange.cuh"
 
 namespace grav {
 
 enum { FUSED_PLAIN = 0, FUSED_DS = 1, FUSED_NEAR = 2 };
-constexpr unsigned FUSED_CLUSTER_PORTABLE = 8;   // portable thread-block cluster size
-constexpr unsigned FUSED_CLUSTER_MAX = 16;       // largest, where the GPU schedules it
 
 struct __align__(32) frow4 {
 	double x, y, z, w;
@@ -47,26 +45,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
 __device__ __forceinline__ void cp_async_wait_all()
 {
 	asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-// CTAs in this CTA's thread-block cluster (1 when launched without clusters)
-__device__ __forceinline__ unsigned cluster_ctas()
-{
-	unsigned v;
-	asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(v));
-	return v;
-}
-
-// Hardware cluster barrier, split: every thread of every CTA of the cluster arrives
-// (release: its earlier loads and stores are ordered before) and later waits (acquire).
-__device__ __forceinline__ void cluster_arrive()
-{
-	asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void cluster_wait()
-{
-	asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Bytes of dynamic shared memory: positions (and low parts) of n bodies padded to a
@@ -351,47 +329,12 @@ cudaError_t launch_fused(const grav_batch& b, int flags, int threads, int rows, 
 {
 	const void* fn = find_fused(b.mode, threads);
 	const int64_t smem = fused_smem(b.mode, b.n_bodies, threads, rows);
-	cudaError_t e = ensure_smem(fn, static_cast<int>(smem));
-	if (e != cudaSuccess) return e;
 	const unsigned grid = static_cast<unsigned>((b.n_bodies + rows - 1) / rows);
 	grav_batch copy = b;
 	int f = flags, R = rows;
 	int32_t* s = sync;
 	void* args[] = {&copy, &f, &R, &s};
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3(grid);
-	cfg.blockDim = dim3(threads);
-	cfg.dynamicSmemBytes = static_cast<size_t>(smem);
-	cfg.stream = stream;
-	cudaLaunchAttribute attr[2];
-	cfg.attrs = attr;
-	cfg.numAttrs = grid > 1 ? 1 : 0;
-	bool cluster = grid > 1 && grid <= FUSED_CLUSTER_MAX;
-	if (cluster) {
-		attr[0].id = cudaLaunchAttributeClusterDimension;
-		attr[0].val.clusterDim.x = grid;
-		attr[0].val.clusterDim.y = 1;
-		attr[0].val.clusterDim.z = 1;
-		if (grid > FUSED_CLUSTER_PORTABLE) {
-			int fits = 0;
-			e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-			if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fits, fn, &cfg);
-			if (e != cudaSuccess) {
-				cudaGetLastError();  // a refused query is not sticky: fall back
-				fits = 0;
-			}
-			cluster = fits > 0;
-		}
-	}
-	if (grid > 1 && !cluster) {
-		attr[0].id = cudaLaunchAttributeCooperative;
-		attr[0].val.cooperative = 1;
-	} else {
-		attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-		attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
-		++cfg.numAttrs;
-	}
-	return cudaLaunchKernelExC(&cfg, fn, args);
+	return launch_exchanging(fn, grid, threads, static_cast<int>(smem), grid > 1, grid > 1, stream, args);
 }
 
 int fused_occupancy(int mode, int64_t n, int threads, int rows, int* ctas_per_sm)
