@@ -303,6 +303,15 @@ __global__ void __launch_bounds__(ST_T, 1) steps_kernel(const grav_batch b, cons
 						sz[r] = add2(sz[r], fz[r]);
 					}
 				}
+				if (SHARED && __reduce_add_sync(0xffffffffu, __popc(nmask)) > 2u * m) {
+					// near pairs in more than one of 16 lanes' blocks: the rows' own radii from here on
+#pragma unroll
+					for (int r = 0; r < 2; ++r) {
+						thr[r] = reinterpret_cast<const float*>(rp + 2 * r + 1)[2];
+						const uint32_t t = __float_as_uint(thr[r]);
+						near_below[r] = t > eps_bits ? t - eps_bits : 0u;
+					}
+				}
 				if (NEAR) {
 					// cold path: each lane goes through the blocks where it met a pair within the near
 					// radius, one such pair at a time, all lanes side by side
@@ -548,7 +557,11 @@ namespace {
 // bodies, cube / Gaussian cloud, 2.0e-7 / 1.7e-7 alone, 1.3e-7 / 0.9e-7 shared, 1.4e-7 / 1.0e-7
 // with the unique-pair kernels, at 20.7 and 21.5 us a step (2500 bodies 6.9 and 7.4).  Where
 // they do not, rows alone are as exact as theirs (4096 bodies 2.1e-7 / 1.8e-7 against 2.2e-7 /
-// 1.9e-7, 9000 1.8e-7 / 1.5e-7 against 1.9e-7 / 1.5e-7) and 4 % faster.
+// 1.9e-7, 9000 1.8e-7 / 1.5e-7 against 1.9e-7 / 1.5e-7) and 4 % faster.  A piece that meets
+// near pairs in more than one of 16 lanes' blocks (of 8 pairs) goes on with the rows' own
+// radii: two Plummer spheres of 6100 bodies take 58 us a step (own radii alone 55, shared to
+// the end 146), bodies spread over four decades 32 (23, 120), in the error of which the pairs
+// between the two radii show (norm 2.3e-7; 3.2e-7 own, 1.6e-7 shared).
 int steps_kind(int mode, int n)
 {
 	switch (mode) {

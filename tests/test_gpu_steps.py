@@ -17,7 +17,7 @@ import torch
 
 import oracle
 from gravitation_gb300.engine import Engine, STEPS_SINGLE_MAX_N
-from gravitation_gb300.scenarios import G_DEFAULT, uniform_cube
+from gravitation_gb300.scenarios import G_DEFAULT, plummer_pair, uniform_cube
 
 pytestmark = pytest.mark.gpu
 
@@ -171,28 +171,35 @@ def test_steps_clump(gpu, n):
         r, v = oracle.stage2_fp64(r, v, acc[k, :, :3], 1.0)
 
 
-@pytest.mark.parametrize('mode,n', [('fp32un', 300), ('fp32un', 2500), ('fp32un', 6000), ('fp32n', 4100),
-                                    ('fp32n', 5003)])
-def test_steps_shared_radius(gpu, mode, n):
-    """Where the pair kernels' rows share a near radius, a group of four consecutive rows does.
-    Heavy bodies at |x| ~ 100, each in a group whose others are at ~990, stand in pairs 6 apart:
-    beyond their own radius of 5, where rounding the positions to FP32 alone puts their forces
-    0.7-1.1e-6 off (rms, from the inputs in FP64), and within their group's 49, where the rounding
-    of an FP32 pair term is left: three products and the cube of a reciprocal square root good to
-    1.2e-7, at most 5e-7."""
+def spread_groups(n):
+    """A cube whose every few groups of four rows hold three bodies on its faces and a heavy one
+    at |x| ~ 100, these in pairs 6 apart: (r, v, m, heavy rows)."""
     r, v, m = uniform_cube(n, seed=n)
     rng = np.random.default_rng(n + 1)
-    groups = np.arange(n // 4)[1:][::max(1, n // 256)][:64]
-    groups = groups[:len(groups) // 2 * 2]
+    count = min(64, n // 32 * 2)
+    groups = np.arange(1, n // 4)[::max(1, (n // 4 - 1) // count)][:count]
     for k in groups:
-        r[4 * k:4 * k + 4] = rng.choice([-1.0, 1.0], (4, 3)) * rng.uniform(980.0, 1000.0, (4, 3))
-    inner = 4 * groups + rng.integers(0, 4, len(groups))
-    for i, j in zip(inner[::2], inner[1::2]):
+        r[4 * k:4 * k + 4] = rng.uniform(-1000.0, 1000.0, (4, 3))
+        r[4 * k + np.arange(4), rng.integers(0, 3, 4)] = rng.choice([-1.0, 1.0], 4) * rng.uniform(980.0, 1000.0, 4)
+    heavy = 4 * groups + rng.integers(0, 4, len(groups))
+    for i, j in zip(heavy[::2], heavy[1::2]):
         d = rng.normal(size=3)
         mid = rng.choice([-1.0, 1.0], 3) * rng.uniform(98.0, 101.0, 3)
         mid[rng.permutation(3)[:2]] *= rng.uniform(-0.3, 0.3, 2)
         r[i], r[j] = mid + 3.0 * d / np.linalg.norm(d), mid - 3.0 * d / np.linalg.norm(d)
-    m[inner] = 1e5 * rng.uniform(1.0, 2.0, len(inner))
+    m[heavy] = 1e5 * rng.uniform(1.0, 2.0, len(heavy))
+    return r, v, m, heavy
+
+
+@pytest.mark.parametrize('mode,n', [('fp32un', 300), ('fp32un', 2500), ('fp32un', 6000), ('fp32n', 4100),
+                                    ('fp32n', 5003)])
+def test_steps_shared_radius(gpu, mode, n):
+    """Where the pair kernels' rows share a near radius, a group of four consecutive rows does.
+    The heavy pairs stand beyond their own radius of 5, where rounding the positions to FP32 alone
+    puts their forces 0.6-1.0e-6 off (rms, from the inputs in FP64), and within their group's 49,
+    where the rounding of an FP32 pair term is left: three products and the cube of a reciprocal
+    square root good to 1.2e-7, at most 5e-7."""
+    r, v, m, heavy = spread_groups(n)
     gm = G_DEFAULT * m
     eng = Engine([n], 1.0, mode=mode)
     assert eng.chained
@@ -204,9 +211,44 @@ def test_steps_shared_radius(gpu, mode, n):
     acc = acc.cpu().numpy()
     for k in range(2):
         ref = oracle.accel_fp64(r, gm, 1.0, coincident=True)
-        err = np.linalg.norm(acc[k, inner, :3] - ref[inner], axis=1) / np.linalg.norm(ref[inner], axis=1)
+        err = np.linalg.norm(acc[k, heavy, :3] - ref[heavy], axis=1) / np.linalg.norm(ref[heavy], axis=1)
         assert np.sqrt((err ** 2).mean()) < 5e-7, (mode, n, k)
         r, v = oracle.stage2_fp64(r, v, acc[k, :, :3], 1.0)
+
+
+@pytest.mark.parametrize('mode,n', [('fp32un', 40), ('fp32un', 500), ('fp32un', 3000), ('fp32un', 6144),
+                                    ('fp32n', 5003)])
+@pytest.mark.parametrize('shape', ['pair', 'steep'])
+def test_steps_dense(gpu, shape, mode, n):
+    """Two dense spheres, and bodies spread over four decades of distance: near pairs everywhere
+    within the radius that a group shares, so that its rows go on with their own."""
+    if shape == 'pair':
+        r, v, m = plummer_pair(n, seed=n)
+    else:
+        rng = np.random.default_rng(n)
+        u = rng.normal(size=(n, 3))
+        r = 10.0 ** rng.uniform(0.0, 4.0, (n, 1)) * u / np.linalg.norm(u, axis=1, keepdims=True)
+        v, m = rng.normal(size=(n, 3)), rng.uniform(1.0, 100.0, n)
+    gm = G_DEFAULT * m
+    one, two = (Engine([n], 1e-3, mode=mode) for _ in range(2))
+    for e in (one, two):
+        assert e.chained
+        e.set_state(r, v, gm)
+    acc = torch.zeros((3, n, 4), dtype=torch.float64, device=one.device)
+    one.steps_to(acc)
+    for _ in range(3):
+        two.step(1)
+    torch.cuda.synchronize()
+    for e in (one, two):
+        e.raise_on_device_error()
+    if n <= STEPS_SINGLE_MAX_N:
+        assert torch.equal(one.r, two.r) and torch.equal(one.v, two.v)
+    acc = acc.cpu().numpy()
+    for k in range(3):
+        ref = oracle.accel_fp64(r, gm, 1.0, coincident=True)
+        err = np.linalg.norm(acc[k, :, :3] - ref, axis=1)
+        assert np.all(err <= TOL * magnitudes(r, gm)), (shape, n, k)
+        r, v = oracle.stage2_fp64(r, v, acc[k, :, :3], 1e-3)
 
 
 @pytest.mark.parametrize('mode,n', [('fp32n', 100), ('fp32n', 3000), ('fp32un', 5000)])
