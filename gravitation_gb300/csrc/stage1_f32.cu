@@ -16,8 +16,8 @@
 // through double-buffered shared memory with 1-D bulk copies (cp.async.bulk,
 // completion on an mbarrier), sums each j-tile's contribution in FP32 and folds
 // that partial into a compensated FP32 sum (TwoSum hi + lo, ~48 bits, no FP64 in the
-// loop).  The CTA's piece of the segment goes as FP64 to its own slot of b.part;
-// stage 2 adds the slots in FP64 in a fixed order, so results do not depend on
+// loop).  The CTA's piece of the segment goes as that pair to its own slot of b.part;
+// stage 2 adds the slots by TwoSum in a fixed order, so results do not depend on
 // scheduling.
 //
 // GRAV_MODE_FP32C reads a second FP32 array with the low parts of the positions

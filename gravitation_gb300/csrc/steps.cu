@@ -5,12 +5,12 @@
 // dependent launches per step (the persistent stage-1 grid, then stage 2 over its slots)
 // spend most of it on launch, drain and memory latency: 8.8 us per step at 64 bodies, 9.2 us
 // at 1000, 17.7 us at 4096 (fp32n, graph-replayed).  Here one grid of at most one CTA per SM
-// stays for all K steps: 1.9, 3.6 and 11.6 us per step of 20.  Each CTA keeps the FP64 state
+// stays for all K steps: 1.9, 3.6 and 11.8 us per step of 20.  Each CTA keeps the FP64 state
 // of its R rows in registers and every body's FP32 position in shared memory; per step it
 // completes its rows' accelerations over all columns, integrates the rows and exchanges the
 // new positions with the other CTAs.  At 1000 bodies a step is ~1 us of pair work and ~0.5 us
-// of the slowest warp's near pairs, ~0.8 us of FP64 update (a chain of eleven FP64
-// instructions of 67 cycles each) and ~1.4 us of exchange; at 4096 the pair loop takes 7.8 us,
+// of the slowest warp's near pairs, ~0.8 us of FP64 update (a chain of eight FP64
+// instructions of 67 cycles each to the new position, three more to its low part) and ~1.4 us of exchange; at 4096 the pair loop takes 7.8 us,
 // 70 % of what its FMA-pipe instructions need.
 //
 // Exchange.  There is no grid barrier between steps.  A row's new position is published as
@@ -39,13 +39,13 @@
 // a row are added by TwoSum (48 bits) in warp order: nothing depends on scheduling.
 //
 // Near pairs.  The loop keeps one bit per block and lane that met a pair within the near
-// radius; after every 32 blocks each lane goes through its own blocks' near pairs, all lanes
-// side by side.  The CTAs run in step, so the warp with the most near pairs sets everyone's
-// pace: with the warp going through the union of its lanes' blocks after every 16, a step took
-// 4.5 us at 1000 bodies (2.9 without the near pairs) and 14.0 at 4096; so 3.8 and 11.6.  The
-// low parts are not kept in shared memory (unless one CTA holds every row): the few that near
-// pairs need come from the exchange buffer, and the exchange moves half the bytes (14.0 to
-// 12.6 us at 4096).
+// radius (each row's own, or one that the group shares: steps_kind); after every 32 blocks each
+// lane goes through its own blocks' near pairs, all lanes side by side.  The CTAs run in step,
+// so the warp with the most near pairs sets everyone's pace: with the warp going through the
+// union of its lanes' blocks after every 16, a step took 4.5 us at 1000 bodies (2.9 without the
+// near pairs) and 14.0 at 4096; so 3.8 and 11.8.  The low parts are not kept in shared memory
+// (unless one CTA holds every row): the few that near pairs need come from the exchange buffer,
+// and the exchange moves half the bytes (14.0 to 12.6 us at 4096).
 #include "exchange.cuh"
 
 namespace grav {

@@ -67,9 +67,13 @@ _DTYPE_MODE = {'float32': 'fp32n', 'float64': 'fp64'}
 UNIQUE_PAIRS_FROM_N = 4608
 
 
-# Above this fraction of near pairs the near-corrected kernels spend more time on their
-# correction path than double-single separations for every pair cost (fp32c / fp32cu,
-# ~1.4x the plain loop): the near path then runs on most steps of the loop.
+# Above this fraction of near pairs the near-corrected kernels take longer than double-single
+# separations for every pair (fp32c / fp32cu).  fp32un against fp32cu on GB300, us a step at
+# 6144 / 16384 / 65536 bodies: cube (near fraction 1e-4) 23.6 / 105 / 1330 against 28.7 / 117 /
+# 1570; a Gaussian cloud 3 widths off the origin (0.9-1.3e-3) 25.4 / 121 / 1517, 5 widths (3e-3)
+# 29.5 / 135 / 1764; the reference's galaxy (3.3e-3) 35.9 / 158 / 2240; two Plummer spheres
+# (1.9e-2) 58 / 167 / 2072.  fp32n and fp32c meet at the same fraction: galaxy of 1024 / 4096
+# bodies 5.1 / 18.0 against 3.9 / 14.4, the cloud at 3 widths 4.3 / 12.7.
 NEAR_DS_FRACTION = 1e-3
 
 
@@ -78,7 +82,8 @@ def near_pair_fraction(r, samples=1 << 16, seed=0, rows=8):
     the near-corrected kernels treat as near: |r_j - r_i| below m / GRAV_NEAR_KAPPA,
     where m is the largest |coordinate| among the `rows` bodies a thread holds (i and
     rows - 1 others drawn at random, as the kernels' rows are spread over the body
-    order).  About 5e-5 for the uniform cube of the benchmark; dense clusters far from
+    order; the kernels leave rows far outside most of their thread's out of m, this
+    estimate does not).  About 5e-5 for the uniform cube of the benchmark; dense clusters far from
     the origin, and discs whose outer bodies set the radius for the inner ones, reach
     1e-3 and more."""
     r = np.asarray(r, dtype=np.float64)[:, :3]
