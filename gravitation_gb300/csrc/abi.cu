@@ -489,7 +489,8 @@ int grav_steps(const grav_batch* b, int flags, int32_t steps, int64_t a_stride, 
 	if (rc) return rc;
 	if (b->n_univ != 1) return fail(GRAV_E_ARG, "grav_steps takes one universe (n_univ = %d)", b->n_univ);
 	if (steps < 0) return fail(GRAV_E_ARG, "steps < 0");
-	if (!scratch) return fail(GRAV_E_ARG, "scratch is NULL");
+	if (!scratch || reinterpret_cast<uintptr_t>(scratch) % 16)
+		return fail(GRAV_E_ARG, "scratch is NULL or not 16-byte aligned");
 	if (!b->err) return fail(GRAV_E_ARG, "NULL err pointer");
 	if (flags & ~(GRAV_S2_INTEGRATE | GRAV_S2_WRITE_A))
 		return fail(GRAV_E_ARG, "grav_steps takes GRAV_S2_INTEGRATE and GRAV_S2_WRITE_A only");

@@ -574,7 +574,8 @@ extern "C" int grav_adjoint_steps(const grav_adjoint* a, int32_t steps, int64_t 
 	const grav_batch& b = *a->b;
 	if (b.n_univ != 1) return grav::record_error(GRAV_E_ARG, "grav_adjoint_steps takes one universe");
 	if (steps < 0) return grav::record_error(GRAV_E_ARG, "steps < 0");
-	if (!scratch) return grav::record_error(GRAV_E_ARG, "scratch is NULL");
+	if (!scratch || reinterpret_cast<uintptr_t>(scratch) % 16)
+		return grav::record_error(GRAV_E_ARG, "scratch is NULL or not 16-byte aligned");
 	if (!a->a_in) return grav::record_error(GRAV_E_ARG, "grav_adjoint_steps needs the accelerations (a_in)");
 	if (b.n_bodies == 0 || steps == 0) return GRAV_OK;
 	// one step alone overwrites the positions it reads, which only two launches keep apart

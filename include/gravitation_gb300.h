@@ -280,8 +280,8 @@ int grav_step_fused(const grav_batch* b, int flags, int32_t threads, int32_t row
  * with double-single separations for every pair). */
 int grav_steps_supported(int mode, int32_t n, int32_t sm_count);
 
-/* Bytes of device scratch grav_steps needs for n bodies: zeroed once by the caller, then
- * left alone between calls (it numbers the exchanged positions). */
+/* Bytes of device scratch grav_steps needs for n bodies, 16-byte aligned: zeroed once by the
+ * caller, then left alone between calls (it numbers the exchanged positions). */
 int64_t grav_steps_scratch_bytes(int32_t n);
 
 /*
@@ -362,8 +362,8 @@ int grav_adjoint_step(const grav_adjoint* a, void* stream);
  * every CTA holds all positions and u in shared memory (up to ~7k bodies). */
 int grav_adjoint_steps_supported(int32_t n, int32_t sm_count);
 
-/* Bytes of device scratch grav_adjoint_steps needs for n bodies: zeroed once by the caller,
- * then left alone between calls (it numbers the exchanged words). */
+/* Bytes of device scratch grav_adjoint_steps needs for n bodies, 16-byte aligned: zeroed once
+ * by the caller, then left alone between calls (it numbers the exchanged words). */
 int64_t grav_adjoint_steps_scratch_bytes(int32_t n);
 
 /*

@@ -1,6 +1,7 @@
 """CPU tests of the engines' host side: what is handed to the kernels, and which plans are
 taken, without a GPU."""
 
+import ctypes
 import types
 
 import pytest
@@ -102,3 +103,26 @@ def test_no_steps_launch_nothing(n):
     eng._steps = None   # a launch would raise TypeError
     for k in (0, -1):
         eng.step(k)
+
+
+def test_scratch_of_the_many_step_launches_is_aligned():
+    """Their exchange uses 128-bit accesses: scratch off a 16-byte boundary is refused."""
+    L = _lib.load()
+    b = _lib.Batch()
+    b.mode = _lib.GRAV_MODE_FP32N
+    b.tile = _lib.Tile(1, 128, 128, 1)
+    b.n_seg, b.n_pad_total, b.n_bodies, b.n_univ = 1, 128, 100, 1
+    b.univ = b.seg = b.pos = b.r = b.v = b.err = 16
+    b.eps2 = 1e-25
+    a = _lib.Adjoint()
+    flat = _lib.Batch.from_buffer_copy(b)
+    flat.mode = _lib.GRAV_MODE_FP32
+    a.b = ctypes.pointer(flat)
+    a.gr = a.gv = a.ggm = a.upos = a.part7 = a.a_in = 16
+    for off in (8, 24, 4):
+        scratch = ctypes.c_void_p(off)   # never dereferenced: validation fails first
+        assert L.grav_steps(ctypes.byref(b), 1, 0, 0, scratch, None) == _lib.GRAV_E_ARG
+        assert L.grav_adjoint_steps(ctypes.byref(a), 0, 0, scratch, None) == _lib.GRAV_E_ARG
+    scratch = ctypes.c_void_p(32)
+    assert L.grav_steps(ctypes.byref(b), 1, 0, 0, scratch, None) == _lib.GRAV_OK           # no steps
+    assert L.grav_adjoint_steps(ctypes.byref(a), 0, 0, scratch, None) == _lib.GRAV_OK
